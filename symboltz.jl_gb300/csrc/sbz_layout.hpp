@@ -7,11 +7,13 @@
 //   ψ_{j,0..Lh} for j = 0..nx-1 (massive ν momentum bins)
 // The equations are those of src/models/{gravity,generic_species,photons,neutrinos}.jl and the
 // couplings of src/models/cosmologies.jl:85-98.  Every row is written as
-//   (J x)_i = cv[sp]·(A x[ip] + C x[inx]) + (cv[dg] + cv[tr])·x[i] + Σ_e cv[e]·x[ecol]
+//   (J x)_i = cv[sp]·(A x[ip] + C x[inx]) + cv[dg]·x[i] + Σ_e cv[e]·x[ecol]
 //             + cv[dx]·(x[dxa] - (3k/4) x[dxb]) + cv[phid]·Φ̇(x) + cv[psid]·Ψ(x)
 // where cv[] are τ-dependent coefficients and Φ̇(x), Ψ(x) the two metric functionals
 // (src/models/gravity.jl:38-39).  The "dx" term keeps the Thomson drag in difference form
-// (θ_b - θ_γ), as the reference writes it, so the residual is free of cancellation.
+// (θ_b - θ_γ), as the reference writes it, so the residual is free of cancellation.  A row's whole
+// diagonal is one slot (the last photon rows' κ̇ - (l+1)/τ included), so a product spends one FP64
+// instruction less per row.
 #pragma once
 #include <cstdint>
 
@@ -30,7 +32,7 @@ constexpr int kNodePow = 16;
 
 // coefficient slots
 enum : int {
-  CV_ZERO = 0, CV_ONE, CV_K, CV_KD, CV_TRG, CV_TRN, CV_TRH, CV_THREE, CV_FOUR, CV_K2, CV_4K3, CV_M1,
+  CV_ZERO = 0, CV_ONE, CV_K, CV_KD, CV_TRN, CV_TRH, CV_THREE, CV_FOUR, CV_K2, CV_4K3, CV_M1,
   CV_MH,       // -ℋ
   CV_M3HCS,    // -3ℋ c_s²
   CV_KDR,      // κ̇ R, R = 4ργ/(3ρb)
@@ -40,13 +42,15 @@ enum : int {
   CV_KD10,     // -κ̇/10
   CV_KD2,      // -κ̇/2
   CV_PB,       // -k²/(3ℋ)
-  CV_MASSIVE = 21  // + 3j: k q_j, -dlnf_j, -(k/3) dlnf_j / q_j
+  CV_MASSIVE = 20,  // + 3j: k q_j, -dlnf_j, -(k/3) dlnf_j / q_j
+  CV_KDTRG = CV_MASSIVE + 3 * kMaxNx  // κ̇ - (l_γ + 1)/τ: diagonal of the last photon rows
 };
+static_assert(CV_KDTRG < kNCV, "coefficient slots");
 
 struct CompDesc {
   double A, C;
   int16_t ip, inx, e0c, e1c, e2c, dxa, dxb, pad;
-  uint8_t sp, dg, tr, e0, e1, e2, phid, psid, dx, pad2[7];
+  uint8_t sp, dg, e0, e1, e2, phid, psid, dx, pad2[8];
 };
 
 // base scalars per τ (value and d/dτ), combined by CoefExpr into cv[] and functional weights
@@ -58,6 +62,7 @@ enum : int {
   B_IE = 13 + 24,    // + j: 1/E_j
   B_COUNT = 13 + 32
 };
+constexpr int kBaseConst = B_IK2 + 1;  // base scalars below this one depend on the mode only, not on τ
 
 // value = K1·B[b[0]]·B[b[1]]·B[b[2]] + K2·B[b[3]]·B[b[4]]·B[b[5]]
 struct CoefExpr {
@@ -73,7 +78,7 @@ struct ModelDesc {
   int16_t psiComp[kMaxFun], rhoComp[kMaxFun];
   int nchain;
   int16_t chFirst[kMaxChains], chLast[kMaxChains], chAttach[kMaxChains];  // attach: head row or -1
-  int nexpr;
+  int nexpr, nexpr_t;  // all expressions; the first nexpr_t depend on τ, the others only on the mode
 };
 
 // per-cosmology constants for the kernels

@@ -283,94 +283,99 @@ __device__ __forceinline__ void table_cubic(const CosmoDesc* __restrict__ cd, co
 // reciprocals 1/a, 1/ℋ, 1/τ as rsqrt(v²) (v > 0), with dr/dτ = -u r³, u = (1/2) dw/dτ for the
 // derivative sets.  The expressions are then spread over the group.  The caller guarantees that no
 // thread still reads the target sets; the call ends with a group barrier.
+// Base scalars of one time on 16 lanes (c = 0..15, every lane of the warp calls; live: the time
+// exists, dq: with derivatives) into Bq/dBq; source: e^{-κ}, κ̈, κ⃛ into src.
+__device__ __forceinline__ void coef_base(int lane, bool live, bool dq, bool source, double tq, const CosmoDesc* cd,
+                                          const double* __restrict__ tab, int nx, const ModeK& mk, double* Bq, double* dBq, double* src) {
+  const int c = lane & 15;
+  double v = 0, d = 0;
+  if (live && c < 7) table_cubic(cd, tab, tq, c, dq, v, d);
+  const int base = lane & ~15;
+  const double a = __shfl_sync(FULL, v, base), da = __shfl_sync(FULL, d, base);
+  const double hc = __shfl_sync(FULL, v, base + 1), dhc = __shfl_sync(FULL, d, base + 1);
+  const int j = c - 8;
+  const bool bin = j >= 0 && j < nx;
+  const double xj = bin ? cd->xq[j] : 0.0, ixj = bin ? cd->ixq[j] : 0.0;
+  const double x = bin ? xj : c == 5 ? a : c == 6 ? hc : c == 7 ? tq : 1.0;
+  const double dx = bin ? 0.0 : c == 5 ? da : c == 6 ? dhc : 1.0;
+  const double ys = bin ? cd->y0 : 0.0;
+  const double ya = ys * a;
+  const double w = fma(x, x, ya * ya);
+  const double r = rsqrt(w);
+  const double E = w * r;
+  const double p2 = (bin ? xj : r) * r;                     // bins: x_j / E; lane 5: 1/a²
+  const double p3 = (bin ? E : cd->R0) * (bin ? ixj : r);  // bins: E / x_j; lane 5: R0 / a
+  double ur = 0, dr = 0, dp2 = 0, dp3 = 0;
+  if (dq) {
+    const double u = fma(x, dx, ya * (ys * da));
+    ur = u * r;                                   // bins: dE/dτ
+    dr = -ur * (r * r);
+    dp2 = (bin ? xj : r) * dr;                    // bins: d(x_j/E)/dτ; lane 5: half of d(1/a²)/dτ
+    dp3 = (bin ? ur : cd->R0) * (bin ? ixj : dr);
+  }
+  if (live) {
+    if (bin) {
+      Bq[B_Q + j] = p2; Bq[B_IQ + j] = p3; Bq[B_E + j] = E; Bq[B_IE + j] = r;
+      if (dq) { dBq[B_Q + j] = dp2; dBq[B_IQ + j] = dp3; dBq[B_E + j] = ur; dBq[B_IE + j] = dr; }
+    } else if (c == 5) {
+      Bq[B_IA] = r; Bq[B_IA2] = p2; Bq[B_R] = p3;
+      if (dq) { dBq[B_IA] = dr; dBq[B_IA2] = 2.0 * dp2; dBq[B_R] = dp3; }
+    } else if (c == 6) {
+      Bq[B_IH] = r;
+      if (dq) dBq[B_IH] = dr;
+    } else if (c == 7) {
+      Bq[B_ITAU] = r; Bq[B_ONE] = 1; Bq[B_K] = mk.k; Bq[B_K2] = mk.k2; Bq[B_IK] = mk.ik; Bq[B_IK2] = mk.ik2;
+      if (dq) { dBq[B_ITAU] = dr; dBq[B_ONE] = 0; dBq[B_K] = 0; dBq[B_K2] = 0; dBq[B_IK] = 0; dBq[B_IK2] = 0; }
+    }
+    if (c == 1) {  // ℋ
+      Bq[B_H] = v;
+      if (dq) dBq[B_H] = d;
+    } else if (c == 2) {  // κ̇ (for the sources, dκ̇/dτ is κ̈ from lane c = 5)
+      Bq[B_KD] = v;
+      if (dq && !source) dBq[B_KD] = d;
+    } else if (c == 3) {  // c_s²
+      Bq[B_CS2] = v;
+      if (dq) dBq[B_CS2] = d;
+    } else if (c >= 4 && c < 7 && source) {  // e^{-κ}, κ̈, κ⃛
+      src[c - 4] = v;
+      if (c == 5) dBq[B_KD] = v;
+    }
+  }
+}
+
+// One coefficient expression K1 p0 p1 p2 + K2 q0 q1 q2 (with its τ-derivative when deriv) into set C.
+__device__ __forceinline__ void coef_expr(const CoefExpr& X, const double* Bq, const double* dBq, bool deriv, CSet& C) {
+  const double p0 = Bq[X.b[0]], p1 = Bq[X.b[1]], p2 = Bq[X.b[2]];
+  const double q0 = Bq[X.b[3]], q1 = Bq[X.b[4]], q2 = Bq[X.b[5]];
+  const double p12 = p1 * p2, q12 = q1 * q2;
+  const double val = fma(X.K1, p0 * p12, X.K2 * (q0 * q12));
+  double dval = 0;
+  if (deriv) {
+    const double dp0 = dBq[X.b[0]], dp1 = dBq[X.b[1]], dp2 = dBq[X.b[2]];
+    const double dq0 = dBq[X.b[3]], dq1 = dBq[X.b[4]], dq2 = dBq[X.b[5]];
+    const double dP = fma(dp0, p12, p0 * fma(dp1, p2, p1 * dp2));
+    const double dQ = fma(dq0, q12, q0 * fma(dq1, q2, q1 * dq2));
+    dval = fma(X.K1, dP, X.K2 * dQ);
+  }
+  const int d = X.dest;
+  if (d < kNCV) { C.cv[d] = val; C.cvd[d] = dval; }
+  else { C.w[d - kNCV] = val; C.wd[d - kNCV] = dval; }
+}
+
 template <int NW, int NSL, typename ST>
 __device__ __forceinline__ void coef_eval(const Grp<NW>& g, ModeMem<NW, NSL, ST>& W, const int* set, const double* taus, int nt,
                           unsigned dmask, bool source, const CosmoDesc* cd, const double* __restrict__ tab,
                           int nexpr, int nx, const ModeK& mk) {
   // times 2p, 2p+1 in pass p: warp p of the group, or every pass on the one warp when NW = 1
   for (int pass = NW == 1 ? 0 : g.wq; 2 * pass < nt; pass += NW) {
-    const int lane = g.lane, q = 2 * pass + (lane >> 4), c = lane & 15;
+    const int q = 2 * pass + (g.lane >> 4);
     const bool live = q < nt;
-    const bool dq = live && ((dmask >> q) & 1u);
-    double v = 0, d = 0;
-    if (live && c < 7) table_cubic(cd, tab, taus[q], c, dq, v, d);
-    const int base = lane & ~15;
-    const double a = __shfl_sync(FULL, v, base), da = __shfl_sync(FULL, d, base);
-    const double hc = __shfl_sync(FULL, v, base + 1), dhc = __shfl_sync(FULL, d, base + 1);
-    const double tq = live ? taus[q] : 1.0;
-    double* Bq = W.B[live ? q : 0]; double* dBq = W.dB[live ? q : 0];
-    const int j = c - 8;
-    const bool bin = j >= 0 && j < nx;
-    const double xj = bin ? cd->xq[j] : 0.0, ixj = bin ? cd->ixq[j] : 0.0;
-    const double x = bin ? xj : c == 5 ? a : c == 6 ? hc : c == 7 ? tq : 1.0;
-    const double dx = bin ? 0.0 : c == 5 ? da : c == 6 ? dhc : 1.0;
-    const double ys = bin ? cd->y0 : 0.0;
-    const double ya = ys * a;
-    const double w = fma(x, x, ya * ya);
-    const double r = rsqrt(w);
-    const double E = w * r;
-    const double p2 = (bin ? xj : r) * r;                     // bins: x_j / E; lane 5: 1/a²
-    const double p3 = (bin ? E : cd->R0) * (bin ? ixj : r);  // bins: E / x_j; lane 5: R0 / a
-    double ur = 0, dr = 0, dp2 = 0, dp3 = 0;
-    if (dq) {
-      const double u = fma(x, dx, ya * (ys * da));
-      ur = u * r;                                   // bins: dE/dτ
-      dr = -ur * (r * r);
-      dp2 = (bin ? xj : r) * dr;                    // bins: d(x_j/E)/dτ; lane 5: half of d(1/a²)/dτ
-      dp3 = (bin ? ur : cd->R0) * (bin ? ixj : dr);
-    }
-    if (live) {
-      if (bin) {
-        Bq[B_Q + j] = p2; Bq[B_IQ + j] = p3; Bq[B_E + j] = E; Bq[B_IE + j] = r;
-        if (dq) { dBq[B_Q + j] = dp2; dBq[B_IQ + j] = dp3; dBq[B_E + j] = ur; dBq[B_IE + j] = dr; }
-      } else if (c == 5) {
-        Bq[B_IA] = r; Bq[B_IA2] = p2; Bq[B_R] = p3;
-        if (dq) { dBq[B_IA] = dr; dBq[B_IA2] = 2.0 * dp2; dBq[B_R] = dp3; }
-      } else if (c == 6) {
-        Bq[B_IH] = r;
-        if (dq) dBq[B_IH] = dr;
-      } else if (c == 7) {
-        Bq[B_ITAU] = r; Bq[B_ONE] = 1; Bq[B_K] = mk.k; Bq[B_K2] = mk.k2; Bq[B_IK] = mk.ik; Bq[B_IK2] = mk.ik2;
-        if (dq) { dBq[B_ITAU] = dr; dBq[B_ONE] = 0; dBq[B_K] = 0; dBq[B_K2] = 0; dBq[B_IK] = 0; dBq[B_IK2] = 0; }
-      }
-      if (c == 1) {  // ℋ
-        Bq[B_H] = v;
-        if (dq) dBq[B_H] = d;
-      } else if (c == 2) {  // κ̇ (for the sources, dκ̇/dτ is κ̈ from lane c = 5)
-        Bq[B_KD] = v;
-        if (dq && !source) dBq[B_KD] = d;
-      } else if (c == 3) {  // c_s²
-        Bq[B_CS2] = v;
-        if (dq) dBq[B_CS2] = d;
-      } else if (c >= 4 && c < 7 && source) {  // e^{-κ}, κ̈, κ⃛
-        W.src[c - 4] = v;
-        if (c == 5) dBq[B_KD] = v;
-      }
-    }
+    coef_base(g.lane, live, live && ((dmask >> q) & 1u), source, live ? taus[q] : 1.0, cd, tab, nx, mk, W.B[live ? q : 0],
+              W.dB[live ? q : 0], W.src);
   }
   g.sync();
-  // expression e at time q (with its τ-derivative when deriv): K1 p0 p1 p2 + K2 q0 q1 q2
-  auto expr = [&](int q, int e, bool deriv) {
-    const CoefExpr& X = cd->expr[e];
-    const double* Bq = W.B[q];
-    const double p0 = Bq[X.b[0]], p1 = Bq[X.b[1]], p2 = Bq[X.b[2]];
-    const double q0 = Bq[X.b[3]], q1 = Bq[X.b[4]], q2 = Bq[X.b[5]];
-    const double p12 = p1 * p2, q12 = q1 * q2;
-    const double val = fma(X.K1, p0 * p12, X.K2 * (q0 * q12));
-    double dval = 0;
-    if (deriv) {
-      const double* dBq = W.dB[q];
-      const double dp0 = dBq[X.b[0]], dp1 = dBq[X.b[1]], dp2 = dBq[X.b[2]];
-      const double dq0 = dBq[X.b[3]], dq1 = dBq[X.b[4]], dq2 = dBq[X.b[5]];
-      const double dP = fma(dp0, p12, p0 * fma(dp1, p2, p1 * dp2));
-      const double dQ = fma(dq0, q12, q0 * fma(dq1, q2, q1 * dq2));
-      dval = fma(X.K1, dP, X.K2 * dQ);
-    }
-    CSet& C = W.cs[set[q]];
-    const int d = X.dest;
-    if (d < kNCV) { C.cv[d] = val; C.cvd[d] = dval; }
-    else { C.w[d - kNCV] = val; C.wd[d - kNCV] = dval; }
-  };
+  // expression e at time q
+  auto expr = [&](int q, int e, bool deriv) { coef_expr(cd->expr[e], W.B[q], W.dB[q], deriv, W.cs[set[q]]); };
   // the qi-th time with (deriv) or without derivatives
   auto time_of = [&](int qi, bool deriv) {
     int q = 0;
@@ -397,6 +402,19 @@ __device__ __forceinline__ void coef_eval(const Grp<NW>& g, ModeMem<NW, NSL, ST>
     }
   }
   g.sync();
+}
+
+// The τ-independent coefficients of a mode (functions of k and the cosmology), into every set once
+// per mode; coef_eval then forms only the first M.nexpr_t expressions (40 of 53 at nx = 5).
+__device__ __forceinline__ void coef_mode(int tid, int nthr, CSet* cs, const CosmoDesc* cd, const ModelDesc& M, const ModeK& mk) {
+  const int nc = M.nexpr - M.nexpr_t;
+  auto base = [&](int b) { return b == B_ONE ? 1.0 : b == B_K ? mk.k : b == B_K2 ? mk.k2 : b == B_IK ? mk.ik : mk.ik2; };
+  for (int p = tid; p < nc * kNSets; p += nthr) {
+    const CoefExpr& X = cd->expr[M.nexpr_t + p % nc];
+    const double val = fma(X.K1, base(X.b[0]) * (base(X.b[1]) * base(X.b[2])), X.K2 * (base(X.b[3]) * (base(X.b[4]) * base(X.b[5]))));
+    CSet& C = cs[p / nc];
+    if (X.dest < kNCV) C.cv[X.dest] = val; else C.w[X.dest - kNCV] = val;
+  }
 }
 
 // Metric functionals of a shared-memory vector v (every warp computes them): Ψ(v) and the δρ
@@ -439,7 +457,7 @@ __device__ __forceinline__ void matvec(const Grp<NW>& g, const double* x, const 
     double o = 0;
     if (i < M.n) {
       const CompDesc& D = comps[i];
-      o = cv[D.sp] * (D.A * x[D.ip] + D.C * x[D.inx]) + (cv[D.dg] + cv[D.tr]) * x[i];
+      o = cv[D.sp] * (D.A * x[D.ip] + D.C * x[D.inx]) + cv[D.dg] * x[i];
       if (s == 0 && gt < 32) o += cv[D.e0] * x[D.e0c] + cv[D.e1] * x[D.e1c] + cv[D.e2] * x[D.e2c] + cv[D.dx] * (x[D.dxa] - k34 * x[D.dxb]);
       if ((g.pp >> s) & 1u) o += cv[D.phid] * phd + cv[D.psid] * psi;
     }
@@ -469,7 +487,7 @@ __device__ __forceinline__ void matvec_dtau(const Grp<NW>& g, const double* x, c
     double o = 0;
     if (i < M.n) {
       const CompDesc& D = comps[i];
-      o = cvd[D.sp] * (D.A * x[D.ip] + D.C * x[D.inx]) + (cvd[D.dg] + cvd[D.tr]) * x[i];
+      o = cvd[D.sp] * (D.A * x[D.ip] + D.C * x[D.inx]) + cvd[D.dg] * x[i];
       if ((g.pp >> s) & 1u) o += cvd[D.phid] * phd + cv[D.phid] * dphd + cvd[D.psid] * psi + cv[D.psid] * dpsi;
       if (s == 0 && gt < 32) o += cvd[D.e0] * x[D.e0c] + cvd[D.e1] * x[D.e1c] + cvd[D.e2] * x[D.e2c] + cvd[D.dx] * (x[D.dxa] - k34 * x[D.dxb]);
     }
@@ -500,8 +518,8 @@ __device__ __forceinline__ void matvec_jd(const Grp<NW>& g, const double* x, con
     if (i < M.n) {
       const CompDesc& D = comps[i];
       const double ax = D.A * x[D.ip] + D.C * x[D.inx], xi = x[i];
-      o = cv[D.sp] * ax + (cv[D.dg] + cv[D.tr]) * xi;
-      d = cvd[D.sp] * ax + (cvd[D.dg] + cvd[D.tr]) * xi;
+      o = cv[D.sp] * ax + cv[D.dg] * xi;
+      d = cvd[D.sp] * ax + cvd[D.dg] * xi;
       if (s == 0 && gt < 32) {
         const double x0 = x[D.e0c], x1 = x[D.e1c], x2 = x[D.e2c], xd = x[D.dxa] - k34 * x[D.dxb];
         o += cv[D.e0] * x0 + cv[D.e1] * x1 + cv[D.e2] * x2 + cv[D.dx] * xd;
@@ -711,7 +729,7 @@ __device__ __forceinline__ void factorize(const Grp<NW>& g, ModeMem<NW, NSL, ST>
                                           double s, double gam, bool scan) {
   const int gt = g.gt, lane = g.lane;
   const double* cv = C.cv;
-  // per-row inputs, all threads: diagonal s - (dg + tr), the two chain couplings, the rank-2
+  // per-row inputs, all threads: diagonal s - dg, the two chain couplings, the rank-2
   // columns; the functional weights in solve precision
 #pragma unroll
   for (int sl = 0; sl < NSL; ++sl) {
@@ -719,7 +737,7 @@ __device__ __forceinline__ void factorize(const Grp<NW>& g, ModeMem<NW, NSL, ST>
     if (i < M.n) {
       const CompDesc& D = comps[i];
       const double spv = cv[D.sp];
-      W.dd[i] = to_st<ST>(s - (cv[D.dg] + cv[D.tr]));
+      W.dd[i] = to_st<ST>(s - cv[D.dg]);
       W.sup[i] = to_st<ST>(-spv * D.C);
       W.sub[i] = to_st<ST>(-spv * D.A);
       W.Z1[i] = to_st<ST>(cv[D.phid]);
@@ -754,7 +772,7 @@ __device__ __forceinline__ void factorize(const Grp<NW>& g, ModeMem<NW, NSL, ST>
     double row[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) row[c] = 0;
-    row[j] += s - (cv[D.dg] + cv[D.tr]);
+    row[j] += s - cv[D.dg];
     const double spv = cv[D.sp];
     int c;
     if ((c = head_local(D.ip)) >= 0) row[c] -= spv * D.A;
@@ -932,6 +950,104 @@ __device__ __forceinline__ void stage_solve(const Grp<NW>& g, ModeMem<NW, NSL, S
   }
 }
 
+// Adiabatic initial conditions (src/models/cosmologies.jl:74-77 and species ieqs): mode scalars (every
+// lane of a warp calls), then the value of unknown i except Φ.
+struct IcScal { double Psi, kt, F1, F2, G2, N2, kdv; };
+__device__ __forceinline__ IcScal ic_scalars(int lane, const ModelDesc& M, const CosmoDesc* cd, const double* B, double k, double t) {
+  IcScal s;
+  s.kdv = B[B_KD];
+  double Ir = 0;
+  if (lane < M.nx) Ir = cd->Wq[lane] * B[B_E + lane];
+  Ir = warp_sum(Ir);
+  const double rg = cd->Og0, rn = cd->On0 + cd->wh * Ir;  // × a⁻⁴
+  const double fnu = rn / (rg + rn);
+  s.Psi = 10.0 / (15.0 + 4.0 * fnu);
+  s.kt = k * t;
+  s.F1 = 2.0 / 3.0 * s.kt * s.Psi;
+  s.F2 = -8.0 / 15.0 * k / s.kdv * s.F1;
+  s.G2 = s.F2 / 16.0;
+  s.N2 = 2.0 / 15.0 * s.kt * s.kt * s.Psi;
+  return s;
+}
+__device__ __forceinline__ double ic_value(int i, const ModelDesc& M, const CosmoDesc* cd, const double* B, const IcScal& s, double k) {
+  double v = 0;
+  if (i == 1 || i == 3) v = -1.5 * s.Psi;
+  else if (i == 2 || i == 4) v = 0.5 * k * s.kt * s.Psi;
+  else if (i == 5) v = -2 * s.Psi;
+  else if (i == 6) v = s.F1;
+  else if (i == 7) v = s.F2;
+  else if (i == 8) v = 5.0 / 16.0 * s.F2;
+  else if (i == 9) v = -1.0 / 16.0 * k / s.kdv * s.F2;
+  else if (i == 10) v = s.G2;
+  else if (i == M.oFt) v = -3.0 / 7.0 * k / s.kdv * s.F2;
+  else if (i == M.oGt) v = -3.0 / 7.0 * k / s.kdv * s.G2;
+  else if (i == M.oN) v = -2 * s.Psi;
+  else if (i == M.oN + 1) v = 2.0 / 3.0 * s.kt * s.Psi;
+  else if (i == M.oN + 2) v = s.N2;
+  else if (i == M.oN + 3) v = 3.0 / 7.0 * s.kt * s.N2;
+  else if (i >= M.oH) {
+    const int jb = (i - M.oH) / (M.Lh + 1), l = (i - M.oH) - jb * (M.Lh + 1);
+    const double dl = cd->dlnf[jb];
+    if (l == 0) v = 0.5 * s.Psi * dl;
+    else if (l == 1) v = -1.0 / 3.0 * B[B_IQ + jb] * (0.5 * s.kt * s.Psi) * dl;
+    else if (l == 2) v = -0.5 * (1.0 / 15.0 * s.kt * s.kt * s.Psi) * dl;
+  }
+  return v;
+}
+
+// Δ_m(τ0) = Σ ρ_s Δ_s / Σ ρ_s over c, b, massive ν (src/observables/fourier.jl:39-52) from the final
+// state x and the base scalars B at τ0; one warp, valid on lane 0.
+__device__ __forceinline__ double delta_m(int lane, const ModelDesc& M, const CosmoDesc* cd, const double* B, const double* x, const ModeK& mk) {
+  double I0 = 0, I1 = 0, Ir = 0;
+  if (lane < M.nx) {
+    const int base = M.oH + lane * (M.Lh + 1);
+    I0 = cd->Wq[lane] * B[B_E + lane] * x[base];
+    I1 = cd->Wq[lane] * cd->xq[lane] * x[base + 1];
+    Ir = cd->Wq[lane] * B[B_E + lane];
+  }
+  I0 = warp_sum(I0); I1 = warp_sum(I1); Ir = warp_sum(Ir);
+  const double ia = B[B_IA], Hc = B[B_H];
+  double num = cd->Oc0 * (x[1] + 3 * Hc * x[2] * mk.ik2) + cd->Ob0 * (x[3] + 3 * Hc * x[4] * mk.ik2);
+  double den = cd->Oc0 + cd->Ob0;
+  num += cd->wh * ia * (I0 + 3 * Hc * I1 * mk.ik);
+  den += cd->wh * ia * Ir;
+  return num / den;
+}
+
+// Line-of-sight quantities at one saved time (src/models/cosmologies.jl:99-105) from the state x, its
+// derivative f, the metric functionals and Π'' (one thread).
+__device__ __forceinline__ void write_output(const PtArgs& A, const CosmoDesc* cd, const ModeK& mk, double tau, const double* x, const double* f,
+                                             const double* src, double kd, double psi, double phid, double psid, double Pidd, int item, int j) {
+  const double k = mk.k;
+  const double ek = src[0], kdd = src[1], kddd = src[2];
+  const double v = -kd * ek, vd = (kd * kd - kdd) * ek, vdd = (-kd * kd * kd + 3 * kd * kdd - kddd) * ek;
+  const double Pi = x[7] + x[8] + x[10];
+  const double Pid = f[7] + f[8] + f[10];
+  const double sSW = v * (x[5] * 0.25 + psi + Pi / 16), sISW = ek * (psid + phid);
+  const double sDop = (vd * x[4] + v * f[4]) * mk.ik2;
+  const double sPol = 3.0 / 16.0 * mk.ik2 * (vdd * Pi + 2 * vd * Pid + v * Pidd);
+  const double chi = cd->tau0 - tau;
+  const double SE = 3.0 / 16.0 * v * Pi / ((k * chi) * (k * chi));
+  if (A.output == SBZ_OUT_FACTORS) {
+    double* o = A.out + ((size_t)item * A.ntau + j) * 7;
+    o[0] = x[5] * 0.25 + psi + Pi / 16; o[1] = psid + phid; o[2] = x[4]; o[3] = f[4];
+    o[4] = Pi; o[5] = Pid; o[6] = Pidd;
+  } else if (A.output == SBZ_OUT_SOURCES4) {
+    double* o = A.out + ((size_t)item * A.ntau + j) * 4;
+    o[0] = k * (sSW + sISW); o[1] = k * sDop; o[2] = k * sPol; o[3] = k * k * SE;
+  } else {
+    const double Spsi = (tau >= cd->taurec) ? -(psi + x[0]) * (tau - cd->taurec) / (cd->tau0 - cd->taurec) / chi : 0.0;
+    double* o = A.out + ((size_t)item * A.ntau + j) * 3;
+    o[0] = k * (sSW + sISW + sDop + sPol); o[1] = k * k * SE; o[2] = Spsi;
+  }
+}
+
+// Zero output of a saved time before the mode starts or after it failed.
+__device__ __forceinline__ void zero_output(const PtArgs& A, int gt, int nthr, int n, int item, int j) {
+  const int w = A.output == SBZ_OUT_SOURCES ? 3 : A.output == SBZ_OUT_SOURCES4 ? 4 : A.output == SBZ_OUT_FACTORS ? 7 : A.output == SBZ_OUT_STATE ? n : 0;
+  for (int i = gt; i < w; i += nthr) A.out[((size_t)item * A.ntau + j) * w + i] = 0;
+}
+
 // ------------------------------------------------------------------------------------------
 // outputs at one saved time τ for state y (coefficient set kNSets-1 is used as scratch)
 template <int NW, int NSL, typename ST>
@@ -949,7 +1065,7 @@ __device__ void emit_output(const Grp<NW>& g, ModeMem<NW, NSL, ST>& W, const PtA
   // line-of-sight sources (src/models/cosmologies.jl:99-105)
   const int so = kNSets - 1;
   const double k = mk.k;
-  coef_eval(g, W, &so, &tau, 1, 1u, true, cd, tab, M.nexpr, M.nx, mk);
+  coef_eval(g, W, &so, &tau, 1, 1u, true, cd, tab, M.nexpr_t, M.nx, mk);
   const CSet& CS = W.cs[so];
 #pragma unroll
   for (int sl = 0; sl < NSL; ++sl) { const int i = comp_of<NW>(gt, sl); if (i < M.n) W.x[i] = y[sl]; }
@@ -966,31 +1082,8 @@ __device__ void emit_output(const Grp<NW>& g, ModeMem<NW, NSL, ST>& W, const PtA
     double gv = 0;
     if (gt == 7 || gt == 8 || gt == 10) gv = dJy[0] + Jf[0];
     const double Pidd = warp_sum(gv);
-    if (gt == 0) {
-      const double ek = W.src[0], kdd = W.src[1], kddd = W.src[2];
-      const double kd = W.B[0][B_KD];
-      const double v = -kd * ek, vd = (kd * kd - kdd) * ek, vdd = (-kd * kd * kd + 3 * kd * kdd - kddd) * ek;
-      const double Pi = W.x[7] + W.x[8] + W.x[10];
-      const double Pid = W.f[7] + W.f[8] + W.f[10];
-      const double psid = dpsi_w + psi_f;  // Ψ' = (∂Ψ/∂τ) y + Ψ(f)
-      const double sSW = v * (W.x[5] * 0.25 + psi + Pi / 16), sISW = ek * (psid + phid);
-      const double sDop = (vd * W.x[4] + v * W.f[4]) * mk.ik2;
-      const double sPol = 3.0 / 16.0 * mk.ik2 * (vdd * Pi + 2 * vd * Pid + v * Pidd);
-      const double chi = cd->tau0 - tau;
-      const double SE = 3.0 / 16.0 * v * Pi / ((k * chi) * (k * chi));
-      if (A.output == SBZ_OUT_FACTORS) {
-        double* o = A.out + ((size_t)item * A.ntau + j) * 7;
-        o[0] = W.x[5] * 0.25 + psi + Pi / 16; o[1] = psid + phid; o[2] = W.x[4]; o[3] = W.f[4];
-        o[4] = Pi; o[5] = Pid; o[6] = Pidd;
-      } else if (A.output == SBZ_OUT_SOURCES4) {
-        double* o = A.out + ((size_t)item * A.ntau + j) * 4;
-        o[0] = k * (sSW + sISW); o[1] = k * sDop; o[2] = k * sPol; o[3] = k * k * SE;
-      } else {
-        const double Spsi = (tau >= cd->taurec) ? -(psi + W.x[0]) * (tau - cd->taurec) / (cd->tau0 - cd->taurec) / chi : 0.0;
-        double* o = A.out + ((size_t)item * A.ntau + j) * 3;
-        o[0] = k * (sSW + sISW + sDop + sPol); o[1] = k * k * SE; o[2] = Spsi;
-      }
-    }
+    if (gt == 0)  // Ψ' = (∂Ψ/∂τ) y + Ψ(f)
+      write_output(A, cd, mk, tau, W.x, W.f, W.src, W.B[0][B_KD], psi, phid, dpsi_w + psi_f, Pidd, item, j);
   }
   g.sync();
 }
@@ -1053,47 +1146,15 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
     const int sIC = kNSets - 1;
 
     // ---- adiabatic initial conditions (src/models/cosmologies.jl:74-77 and species ieqs) ----
-    coef_eval(g, W, &sIC, &t, 1, 0u, false, cd, tab, M.nexpr, M.nx, mk);
+    coef_mode(gt, NT, W.cs, cd, M, mk);
+    g.sync();
+    coef_eval(g, W, &sIC, &t, 1, 0u, false, cd, tab, M.nexpr_t, M.nx, mk);
     {
-      const double kdv = W.B[0][B_KD];
-      double Ir = 0;
-      if (g.lane < M.nx) Ir = cd->Wq[g.lane] * W.B[0][B_E + g.lane];
-      Ir = warp_sum(Ir);
-      const double rg = cd->Og0, rn = cd->On0 + cd->wh * Ir;  // × a⁻⁴
-      const double fnu = rn / (rg + rn);
-      const double Psi = 10.0 / (15.0 + 4.0 * fnu);
-      const double kt = k * t;
-      const double F1 = 2.0 / 3.0 * kt * Psi;
-      const double F2 = -8.0 / 15.0 * k / kdv * F1;
-      const double G2 = F2 / 16.0;
-      const double N2 = 2.0 / 15.0 * kt * kt * Psi;
+      const IcScal ic = ic_scalars(g.lane, M, cd, W.B[0], k, t);
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) {
         const int i = comp_of<NW>(gt, sl);
-        double v = 0;
-        if (i < n) {
-          if (i == 1 || i == 3) v = -1.5 * Psi;
-          else if (i == 2 || i == 4) v = 0.5 * k * kt * Psi;
-          else if (i == 5) v = -2 * Psi;
-          else if (i == 6) v = F1;
-          else if (i == 7) v = F2;
-          else if (i == 8) v = 5.0 / 16.0 * F2;
-          else if (i == 9) v = -1.0 / 16.0 * k / kdv * F2;
-          else if (i == 10) v = G2;
-          else if (i == M.oFt) v = -3.0 / 7.0 * k / kdv * F2;
-          else if (i == M.oGt) v = -3.0 / 7.0 * k / kdv * G2;
-          else if (i == M.oN) v = -2 * Psi;
-          else if (i == M.oN + 1) v = 2.0 / 3.0 * kt * Psi;
-          else if (i == M.oN + 2) v = N2;
-          else if (i == M.oN + 3) v = 3.0 / 7.0 * kt * N2;
-          else if (i >= M.oH) {
-            const int jb = (i - M.oH) / (M.Lh + 1), l = (i - M.oH) - jb * (M.Lh + 1);
-            const double dl = cd->dlnf[jb];
-            if (l == 0) v = 0.5 * Psi * dl;
-            else if (l == 1) v = -1.0 / 3.0 * W.B[0][B_IQ + jb] * (0.5 * kt * Psi) * dl;
-            else if (l == 2) v = -0.5 * (1.0 / 15.0 * kt * kt * Psi) * dl;
-          }
-        }
+        const double v = i < n ? ic_value(i, M, cd, W.B[0], ic, k) : 0.0;
         y[sl] = v;
         if (i < n) W.x[i] = v;
       }
@@ -1102,7 +1163,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
       double psi0, rho0;
       functionals(g.fc, W.x, W.cs[sIC].w, psi0, rho0);  // Φ slot still 0
       g.sync();
-      if (gt == 0) { y[0] = Psi - psi0; W.x[0] = y[0]; }
+      if (gt == 0) { y[0] = ic.Psi - psi0; W.x[0] = y[0]; }
       g.sync();
     }
     // outputs at or before the initial time
@@ -1110,13 +1171,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
     if (taus) {
       while (jout < A.ntau && taus[jout] <= t) {
         if (taus[jout] < t) {  // before the mode starts: zero
-          if (A.output == SBZ_OUT_SOURCES && gt < 3) A.out[((size_t)item * A.ntau + jout) * 3 + gt] = 0;
-        if (A.output == SBZ_OUT_SOURCES4 && gt < 4) A.out[((size_t)item * A.ntau + jout) * 4 + gt] = 0;
-        if (A.output == SBZ_OUT_FACTORS && gt < 7) A.out[((size_t)item * A.ntau + jout) * 7 + gt] = 0;
-          if (A.output == SBZ_OUT_SOURCES4 && gt < 4) A.out[((size_t)item * A.ntau + jout) * 4 + gt] = 0;
-        if (A.output == SBZ_OUT_FACTORS && gt < 7) A.out[((size_t)item * A.ntau + jout) * 7 + gt] = 0;
-          if (A.output == SBZ_OUT_FACTORS && gt < 7) A.out[((size_t)item * A.ntau + jout) * 7 + gt] = 0;
-          if (A.output == SBZ_OUT_STATE) for (int i = gt; i < n; i += NT) A.out[((size_t)item * A.ntau + jout) * n + i] = 0;
+          zero_output(A, gt, NT, n, item, jout);
         } else {
           emit_output(g, W, A, cd, tab, comps, M, mk, t, y, item, jout);
         }
@@ -1126,7 +1181,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
 
     // ---- integration ----
     if (t < tend) {
-      coef_eval(g, W, &sJ, &t, 1, 1u, false, cd, tab, M.nexpr, M.nx, mk);
+      coef_eval(g, W, &sJ, &t, 1, 1u, false, cd, tab, M.nexpr_t, M.nx, mk);
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) { const int i = comp_of<NW>(gt, sl); if (i < n) W.x[i] = y[sl]; }
       g.sync();
@@ -1146,7 +1201,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
 #pragma unroll
         for (int sl = 0; sl < NSL; ++sl) { const int i = comp_of<NW>(gt, sl); if (i < n) W.x[i] = y[sl] + h0 * f0[sl]; }
         const double th = t + h0;
-        coef_eval(g, W, &sE, &th, 1, 0u, false, cd, tab, M.nexpr, M.nx, mk);
+        coef_eval(g, W, &sE, &th, 1, 0u, false, cd, tab, M.nexpr_t, M.nx, mk);
         double f1[NSL];
         matvec<NW, NSL>(g, W.x, W.cs[sE], comps, M, k, f1);
         double d2 = 0;
@@ -1207,7 +1262,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
         tset[TB::NTIME] = sE;
         // coefficients at the later stage times (the last one, t + h, with τ-derivatives: it is the
         // next step's Jacobian set), and the factorisation for this h
-        coef_eval(g, W, tset + 1, W.ctl + 4, TB::NTIME, 1u << (TB::NTIME - 1), false, cd, tab, M.nexpr, M.nx, mk);
+        coef_eval(g, W, tset + 1, W.ctl + 4, TB::NTIME, 1u << (TB::NTIME - 1), false, cd, tab, M.nexpr_t, M.nx, mk);
         factorize(g, W, F, CJ, comps, M, k, h, s, TB::gam, scan);
         double b[NSL], Fv[NSL], Y[NSL], Ul[NSL];  // Ul: the last stage computed
         double U[kRolledStages<NW, ST> ? 1 : TB::S][NSL];  // the stages (unrolled loop)
@@ -1388,12 +1443,7 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
     }
     // saved times never reached (failed mode): zero
     if (taus) {
-      for (; jout < A.ntau; ++jout) {
-        if (A.output == SBZ_OUT_SOURCES && gt < 3) A.out[((size_t)item * A.ntau + jout) * 3 + gt] = 0;
-        if (A.output == SBZ_OUT_SOURCES4 && gt < 4) A.out[((size_t)item * A.ntau + jout) * 4 + gt] = 0;
-        if (A.output == SBZ_OUT_FACTORS && gt < 7) A.out[((size_t)item * A.ntau + jout) * 7 + gt] = 0;
-        if (A.output == SBZ_OUT_STATE) for (int i = gt; i < n; i += NT) A.out[((size_t)item * A.ntau + jout) * n + i] = 0;
-      }
+      for (; jout < A.ntau; ++jout) zero_output(A, gt, NT, n, item, jout);
     }
     bool finite = true;
 #pragma unroll
@@ -1404,27 +1454,13 @@ __device__ void pt_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __r
       // Δ_m(τ0) = Σ ρ_s Δ_s / Σ ρ_s over c, b, massive ν   (src/observables/fourier.jl:39-52)
       const int so = kNSets - 1;
       g.sync();
-      coef_eval(g, W, &so, &tend, 1, 0u, false, cd, tab, M.nexpr, M.nx, mk);
+      coef_eval(g, W, &so, &tend, 1, 0u, false, cd, tab, M.nexpr_t, M.nx, mk);
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) { const int i = comp_of<NW>(gt, sl); if (i < n) W.x[i] = y[sl]; }
       g.sync();
       if (g.wq == 0) {
-        double I0 = 0, I1 = 0, Ir = 0;
-        if (g.lane < M.nx) {
-          const int base = M.oH + g.lane * (M.Lh + 1);
-          I0 = cd->Wq[g.lane] * W.B[0][B_E + g.lane] * W.x[base];
-          I1 = cd->Wq[g.lane] * cd->xq[g.lane] * W.x[base + 1];
-          Ir = cd->Wq[g.lane] * W.B[0][B_E + g.lane];
-        }
-        I0 = warp_sum(I0); I1 = warp_sum(I1); Ir = warp_sum(Ir);
-        if (gt == 0) {
-          const double ia = W.B[0][B_IA], Hc = W.B[0][B_H];
-          double num = cd->Oc0 * (W.x[1] + 3 * Hc * W.x[2] * mk.ik2) + cd->Ob0 * (W.x[3] + 3 * Hc * W.x[4] * mk.ik2);
-          double den = cd->Oc0 + cd->Ob0;
-          num += cd->wh * ia * (I0 + 3 * Hc * I1 * mk.ik);
-          den += cd->wh * ia * Ir;
-          A.out[item] = num / den;
-        }
+        const double d = delta_m(g.lane, M, cd, W.B[0], W.x, mk);
+        if (gt == 0) A.out[item] = d;
       }
     }
     if (gt == 0) {
@@ -1509,7 +1545,9 @@ __global__ void __launch_bounds__(32) rhs_kernel(PtArgs A, const double* __restr
   mk.k = A.item_k[item]; mk.k2 = mk.k * mk.k; mk.ik = 1.0 / mk.k; mk.ik2 = mk.ik * mk.ik;
   const double tau = tau_in[item];
   const int so = 0;
-  coef_eval(g, W, &so, &tau, 1, 1u, false, cd, tab, M.nexpr, M.nx, mk);
+  coef_mode(g.gt, 32, W.cs, cd, M, mk);
+  __syncwarp();
+  coef_eval(g, W, &so, &tau, 1, 1u, false, cd, tab, M.nexpr_t, M.nx, mk);
   for (int i = g.gt; i < n; i += 32) W.x[i] = y_in[(size_t)item * n + i];
   __syncwarp();
   double f[NSL], ft[NSL];

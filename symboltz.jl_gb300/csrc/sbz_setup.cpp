@@ -29,17 +29,17 @@ int build_model(const sbz_model& m, ModelDesc& M, std::vector<CompDesc>& comps) 
   comps.assign(n, CompDesc{});
   for (auto& c : comps) {
     c.A = c.C = 0; c.ip = c.inx = c.e0c = c.e1c = c.e2c = c.dxa = c.dxb = (int16_t)Z;
-    c.sp = c.dg = c.tr = c.e0 = c.e1 = c.e2 = c.phid = c.psid = c.dx = CV_ZERO;
+    c.sp = c.dg = c.e0 = c.e1 = c.e2 = c.phid = c.psid = c.dx = CV_ZERO;
   }
   auto chain = [&](int i, int ip, int inx, double A, double C, int sp) {
     CompDesc& c = comps[i]; c.ip = (int16_t)ip; c.inx = (int16_t)inx; c.A = A; c.C = C; c.sp = (uint8_t)sp;
   };
-  auto hier = [&](auto idx, int L, int sp, int dg, int tr) {  // generic free-streaming hierarchy 0..L
+  auto hier = [&](auto idx, int L, int sp, int dg, int dgl) {  // free-streaming hierarchy 0..L, diagonals dg and (l = L) dgl
     for (int l = 0; l <= L; ++l) {
       const int i = idx(l);
       if (l < L) chain(i, l > 0 ? idx(l - 1) : Z, idx(l + 1), double(l) / (2 * l + 1), -double(l + 1) / (2 * l + 1), sp);
-      else { chain(i, idx(l - 1), Z, 1.0, 0.0, sp); comps[i].tr = (uint8_t)tr; }
-      comps[i].dg = (uint8_t)dg;
+      else chain(i, idx(l - 1), Z, 1.0, 0.0, sp);
+      comps[i].dg = (uint8_t)(l < L ? dg : dgl);
     }
   };
   // metric and matter
@@ -50,8 +50,8 @@ int build_model(const sbz_model& m, ModelDesc& M, std::vector<CompDesc>& comps) 
   comps[4].e0 = CV_MH; comps[4].e0c = 4; comps[4].e1 = CV_CSK2; comps[4].e1c = 3; comps[4].psid = CV_K2;
   comps[4].dx = CV_KDR; comps[4].dxa = 4; comps[4].dxb = (int16_t)Fi(M, 1);
   // photons
-  hier([&](int l) { return Fi(M, l); }, M.Lg, CV_K, CV_KD, CV_TRG);
-  hier([&](int l) { return Gi(M, l); }, M.Lg, CV_K, CV_KD, CV_TRG);
+  hier([&](int l) { return Fi(M, l); }, M.Lg, CV_K, CV_KD, CV_KDTRG);
+  hier([&](int l) { return Gi(M, l); }, M.Lg, CV_K, CV_KD, CV_KDTRG);
   comps[Fi(M, 0)].dg = CV_ZERO; comps[Fi(M, 0)].phid = CV_FOUR;
   comps[Fi(M, 1)].dg = CV_ZERO; comps[Fi(M, 1)].psid = CV_4K3;
   comps[Fi(M, 1)].dx = CV_DRAG_F1; comps[Fi(M, 1)].dxa = 4; comps[Fi(M, 1)].dxb = (int16_t)Fi(M, 1);
@@ -85,6 +85,7 @@ int build_model(const sbz_model& m, ModelDesc& M, std::vector<CompDesc>& comps) 
   addch(Ni(M, 0), Ni(M, M.Ln), -1);
   for (int j = 0; j < M.nx; ++j) addch(Hi(M, j, 0), Hi(M, j, M.Lh), -1);
   M.nexpr = 27 + 5 * M.nx;  // coefficient expressions emitted by build_cosmo
+  M.nexpr_t = 19 + 4 * M.nx;
   return SBZ_OK;
 }
 
@@ -97,16 +98,17 @@ int build_cosmo(const Background& B, const ModelDesc& M, const sbz_model& m, Cos
   D.Oc0 = P.Oc0; D.Ob0 = P.Ob0; D.Og0 = P.Og0; D.On0 = P.On0; D.wh = P.wh; D.y0 = P.y0;
   D.R0 = 4.0 / 3.0 * P.Og0 / P.Ob0; D.As = P.As; D.ns = P.ns; D.kpivot = P.kpivot;
   for (int j = 0; j < M.nx; ++j) { D.xq[j] = P.xq[j]; D.Wq[j] = P.Wq[j]; D.dlnf[j] = P.dlnf[j]; D.ixq[j] = 1.0 / P.xq[j]; }
-  int ne = 0;
+  int ne = 0, nc = 0;  // τ-dependent expressions from the front, the others from nexpr_t
   auto E = [&](int dest, double K1, int a0, int a1 = B_ONE, int a2 = B_ONE, double K2 = 0, int b0 = B_ONE, int b1 = B_ONE, int b2 = B_ONE) {
-    CoefExpr& e = D.expr[ne++];
+    const bool tdep = a0 >= kBaseConst || a1 >= kBaseConst || a2 >= kBaseConst || b0 >= kBaseConst || b1 >= kBaseConst || b2 >= kBaseConst;
+    CoefExpr& e = D.expr[tdep ? ne++ : M.nexpr_t + nc++];
     e.K1 = K1; e.K2 = K2; e.dest = (int16_t)dest;
     e.b[0] = (uint8_t)a0; e.b[1] = (uint8_t)a1; e.b[2] = (uint8_t)a2; e.b[3] = (uint8_t)b0; e.b[4] = (uint8_t)b1; e.b[5] = (uint8_t)b2;
   };
   E(CV_ONE, 1.0, B_ONE);
   E(CV_K, 1.0, B_K);
   E(CV_KD, 1.0, B_KD);
-  E(CV_TRG, -(M.Lg + 1.0), B_ITAU);
+  E(CV_KDTRG, 1.0, B_KD, B_ONE, B_ONE, -(M.Lg + 1.0), B_ITAU);
   E(CV_TRN, -(M.Ln + 1.0), B_ITAU);
   E(CV_TRH, -(M.Lh + 1.0), B_ITAU);
   E(CV_THREE, 3.0, B_ONE);
@@ -141,7 +143,7 @@ int build_cosmo(const Background& B, const ModelDesc& M, const sbz_model& m, Cos
   E(R0 + 3, P.On0, B_IA2);
   for (int j = 0; j < M.nx; ++j) E(R0 + 4 + j, P.wh * P.Wq[j], B_IA2, B_E + j);
   (void)m;
-  return ne == M.nexpr ? SBZ_OK : SBZ_ERR_STATE;
+  return ne == M.nexpr_t && ne + nc == M.nexpr ? SBZ_OK : SBZ_ERR_STATE;
 }
 
 }  // namespace sbz
