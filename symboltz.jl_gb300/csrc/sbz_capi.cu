@@ -381,15 +381,22 @@ int sbz_bg_coefficients(const sbz_problem* pb, int cosmo, int n, const double* t
   return SBZ_OK;
 }
 
-static int pt_run(sbz_problem* pb, int nk, const int* d_cosmo, const double* d_ks, const double* d_ti, const int* d_order,
-                  int ntau, const double* d_taus, int output, double* d_out, int* d_status, int64_t* d_steps) {
-  sbz::PtArgs A{};
+// model part of the kernel arguments
+static void pt_model_args(const sbz_problem* pb, sbz::PtArgs& A) {
   A.model = pb->d_model.as<sbz::ModelDesc>();
   A.comps = pb->d_comps.as<sbz::CompDesc>();
   A.model_n = pb->M.n;
+  A.nchain = pb->M.nchain;
+  for (int c = 0; c < pb->M.nchain; ++c) A.chain_rows = std::max(A.chain_rows, pb->M.chLast[c] - pb->M.chFirst[c] + 1);
   A.cosmos = pb->d_cosmos.as<sbz::CosmoDesc>();
   A.tables = pb->d_tables.as<double>();
   A.table_stride = pb->table_stride;
+}
+
+static int pt_run(sbz_problem* pb, int nk, const int* d_cosmo, const double* d_ks, const double* d_ti, const int* d_order,
+                  int ntau, const double* d_taus, int output, double* d_out, int* d_status, int64_t* d_steps) {
+  sbz::PtArgs A{};
+  pt_model_args(pb, A);
   A.item_cosmo = d_cosmo; A.item_k = d_ks; A.item_tau_ini = d_ti; A.order = d_order; A.nitems = nk;
   A.taus = ntau > 0 ? d_taus : nullptr; A.ntau = ntau;
   A.output = output; A.out = d_out; A.status = d_status; A.steps = d_steps;
@@ -432,8 +439,7 @@ int sbz_pt_rhs(sbz_problem* pb, int nk, const int* cosmo, const double* ks, cons
   SBZ_CUDA(cudaMemcpy(d_c, cos.data(), sizeof(int) * nk, cudaMemcpyHostToDevice));
   SBZ_CUDA(cudaMemcpy(d_y, y, ny, cudaMemcpyHostToDevice));
   sbz::PtArgs A{};
-  A.model = pb->d_model.as<sbz::ModelDesc>(); A.comps = pb->d_comps.as<sbz::CompDesc>(); A.model_n = n;
-  A.cosmos = pb->d_cosmos.as<sbz::CosmoDesc>(); A.tables = pb->d_tables.as<double>(); A.table_stride = pb->table_stride;
+  pt_model_args(pb, A);
   A.item_cosmo = d_c; A.item_k = d_k; A.nitems = nk;
   r = sbz::rhs_launch(A, d_y, d_t, d_f, d_ft, pb->stream);
   if (r == SBZ_OK) {
@@ -702,8 +708,7 @@ static int spectrum_cmb_impl(sbz_problem* pb, int cosmo, const sbz_bessel* jl, i
     SBZ_CUDA(cudaMemsetAsync(pb->d_status.p, 0, sizeof(int) * nc, st));
   } else {
     sbz::PtArgs A{};
-    A.model = pb->d_model.as<sbz::ModelDesc>(); A.comps = pb->d_comps.as<sbz::CompDesc>(); A.model_n = pb->M.n;
-    A.cosmos = pb->d_cosmos.as<sbz::CosmoDesc>(); A.tables = pb->d_tables.as<double>(); A.table_stride = pb->table_stride;
+    pt_model_args(pb, A);
     A.item_cosmo = pb->d_cosmo.as<int>(); A.item_k = pb->d_k.as<double>(); A.item_tau_ini = pb->d_ti.as<double>();
     A.order = pb->d_order.as<int>(); A.nitems = nc;
     A.taus = pb->d_taus.as<double>(); A.ntau = ntau; A.output = SBZ_OUT_SOURCES;

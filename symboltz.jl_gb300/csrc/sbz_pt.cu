@@ -7,6 +7,8 @@ int pt_launch_f32_w1(const PtArgs& A, int nw, int warps_per_block, int blocks_pe
 int pt_launch_f32_w2_w4(const PtArgs& A, int nw, int warps_per_block, int blocks_per_sm, int num_sms, cudaStream_t stream);
 int pt_launch_f64_w1(const PtArgs& A, int nw, int warps_per_block, int blocks_per_sm, int num_sms, cudaStream_t stream);
 int pt_launch_f64_w2_w4(const PtArgs& A, int nw, int warps_per_block, int blocks_per_sm, int num_sms, cudaStream_t stream);
+int pt_launch_lat_f32(const PtArgs& A, int num_sms, cudaStream_t stream);
+int pt_launch_lat_f64(const PtArgs& A, int num_sms, cudaStream_t stream);
 
 // Warps per mode when the caller leaves it open: a spectrum's run time is set by its slowest
 // (highest-k) modes, so while the modes fit on the GPU a few at a time, each gets the four
@@ -24,6 +26,9 @@ int pt_launch(const PtArgs& A, int precision, int warps_per_block, int warps_per
   // groups per SM, so a slow mode shares its SM with at most one other
   if (blocks_per_sm <= 0 && nw == 4) blocks_per_sm = A.nitems <= 8 * num_sms ? 1 : 2;
   if (nw == 8) blocks_per_sm = 1;  // eight-warp groups: one mode per SM
+  // one mode per SM: the latency kernel, while its four solver warps hold every chain (nx <= 5) and a
+  // chain fits a warp
+  const bool lat = nw == 4 && blocks_per_sm == 1 && A.nchain <= 8 && A.chain_rows <= 32;
   if (precision == SBZ_MIXED) {
     // lazy refinement left open: the later stages skip their FP64 refinement when stage 1's first
     // correction is below 1e-5 error weights (Rodas5P's stage right-hand sides carry coefficients up
@@ -34,9 +39,11 @@ int pt_launch(const PtArgs& A, int precision, int warps_per_block, int warps_per
     // away from the oracle on the reference's ΛCDM(lmax = 5) model.
     PtArgs B = A;
     if (B.refine_skip < 0) B.refine_skip = nw >= 4 ? 1e-5f : 0.0f;
+    if (lat) return pt_launch_lat_f32(B, num_sms, stream);
     return nw == 1 ? pt_launch_f32_w1(B, nw, warps_per_block, blocks_per_sm, num_sms, stream)
                    : pt_launch_f32_w2_w4(B, nw, warps_per_block, blocks_per_sm, num_sms, stream);
   }
+  if (lat) return pt_launch_lat_f64(A, num_sms, stream);
   return nw == 1 ? pt_launch_f64_w1(A, nw, warps_per_block, blocks_per_sm, num_sms, stream) : pt_launch_f64_w2_w4(A, nw, warps_per_block, blocks_per_sm, num_sms, stream);
 }
 

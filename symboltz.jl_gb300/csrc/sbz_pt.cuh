@@ -11,6 +11,7 @@ struct PtArgs {
   const ModelDesc* model;     // device
   const CompDesc* comps;      // device, model_n entries
   int model_n;
+  int nchain, chain_rows;     // free-streaming chains of the model and the rows of the longest
   const CosmoDesc* cosmos;    // device, one per cosmology
   const double* tables;       // device, cosmology c at tables + c * table_stride
   int64_t table_stride;
