@@ -22,9 +22,10 @@
 //     FP64 work, and reach the others through shared memory (each FP64 warp instruction holds a
 //     sub-partition for 64 cycles: 8 of warp 0's 23 instructions per product leave it);
 //   * scans and sums stop at the level that the longest chain or sum of the model needs.
-// Every sum keeps the order and the fusion of the generic kernel, so both give the same bits in FP64
-// and in mixed precision (the stage sums use explicit fma: a product left unfused by the compiler in one
-// of the two kernels changes an FP32 rounding somewhere and then every later step).
+// Every sum keeps the order and the fusion of the generic kernel, so both give the same bits in mixed
+// precision (the stage sums use explicit fma: a product left unfused by the compiler in one
+// of the two kernels changes an FP32 rounding somewhere and then every later step).  In all-FP64
+// solves the pivots' reciprocals differ from the generic kernel's by a unit in the last place.
 #include "sbz_pt_impl.cuh"
 
 namespace sbz {
@@ -36,15 +37,18 @@ enum : int {
   LB_MAIN = 1,  // solver warps
   LB_COMP,      // companion warps
   LB_STEP,      // the step's last stage and y1 are in shared memory (both sides)
-  LB_CTL,       // step control published (companions arrive, solvers wait)
-  LB_COEF,      // coefficients of the later stage times ready (companions arrive, solvers wait)
+  LB_CTL,       // step size and decision published (control warp arrives, solvers wait)
+  LB_COEF,      // coefficients of the later stage times ready (coefficient warps arrive, solvers wait)
   LB_RHS,       // a stage's right-hand side is in shared memory; companions may add the previous stage (both)
   LB_SUM,       // next stage's sums ready (companions arrive, solvers wait)
-  LB_LU,        // chain pivots ready (solvers and the head warp)
-  LB_HEAD,      // head inverse ready (head warp arrives, solvers wait)
+  LB_DD,        // factorisation diagonals ready (solvers arrive, control warp waits)
+  LB_LU,        // chain pivots ready (control warp arrives, solvers wait)
+  LB_HROW,      // head rows ready (solver warp 3 arrives, control warp waits)
+  LB_HEAD,      // head inverse ready (control warp arrives, solvers wait)
   LB_FUN,       // metric functionals ready (functional warp arrives, the others wait)
-  LB_REJ,       // a rejected step's speculative f(t1, y1) is done with the step-end set (both)
-  LB_CO3        // the three coefficient warps
+  LB_REJ,       // a rejected step: the solvers have left the step-end set (both)
+  LB_CO3,       // the three coefficient warps
+  LB_ERR        // error-norm parts (companion warps 0..2 arrive, the control warp waits)
 };
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
@@ -72,6 +76,8 @@ struct LatMem {
   float redf[2][4];
   double ctl[4 + kMaxT];
   int ctlf, accept;
+  double tA[TB::S], tC[TB::S], td[TB::S];  // tableau: last A and C of each stage, d
+  int tq[TB::S], tinc[TB::S];              // stage time set, incremental input
   CosmoDesc cdesc;
   int item;
 };
@@ -228,13 +234,34 @@ __device__ __forceinline__ Fun lat_matvec(const LGrp& g, LatMem<NSL, ST>& W, con
   return F;
 }
 
+// Reciprocal of a pivot.  FP32: the hardware approximation (pivots are far from the subnormals that the
+// non-ftz form would handle).  FP64: its 20-bit seed and two Newton steps r += r (1 - v r), each squaring
+// the error: about one unit in the last place for a fifth of a division's FP64 instructions.
+template <typename ST>
+__device__ __forceinline__ ST lat_rcp(ST v);
+template <>
+__device__ __forceinline__ float lat_rcp<float>(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+template <>
+__device__ __forceinline__ double lat_rcp<double>(double v) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(v));
+  r = fma(r, fma(-v, r, 1.0), r);
+  return fma(r, fma(-v, r, 1.0), r);
+}
+// Magnitudes in order as integers (an FP64 comparison holds the FP64 pipe like a product).
+__device__ __forceinline__ unsigned mag_key(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long mag_key(double v) { return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull; }
+
 // ---- structured solve with the step's factorisation in registers -----------------------------------
 // Warp p eliminates chains 2p and 2p + 1 (lane j: row last - j), as in sbz_pt_impl.cuh.
 template <typename ST>
 struct LatScan {
   int i0, i1, j0, j1, n0, n1;  // rows, rows clamped into the arrays, chain lengths
-  bool on0, on1, pair;
-  int nlev;                    // levels that the longer chain needs (the others have zero multipliers)
+  bool on0, on1, pair, more;   // more: a chain has more than eight rows (levels 3 and 4 have nonzero multipliers)
   ST f0[5], f1[5], b0[5], b1[5], d0, d1;
 };
 template <typename ST>
@@ -247,44 +274,31 @@ struct LatFactor {
 template <int NV, int NSL, typename ST>
 __device__ __forceinline__ void lat_solve_M(const LGrp& g, const LatScan<ST>& S, const LatFactor<ST>& F, ST* v0, ST* v1) {
   const int lane = g.lane;
+  if (g.wq == 3) {  // Φ and CDM ([[s, 1], [0, s+ℋ]]), on every lane of the warp with fewest rows
+    const ST a2 = v0[2] * F.ihc, a1 = (v0[1] - a2) * F.is, a0 = v0[0] * F.is;
+    ST c0 = 0, c1 = 0, c2 = 0;
+    if (NV > 1) { c2 = v1[2] * F.ihc; c1 = (v1[1] - c2) * F.is; c0 = v1[0] * F.is; }
+    __syncwarp();
+    if (lane == 0) {
+      v0[0] = a0; v0[1] = a1; v0[2] = a2;
+      if (NV > 1) { v1[0] = c0; v1[1] = c1; v1[2] = c2; }
+    }
+  }
   if (S.pair) {
     const ST r0 = v0[S.j0], r1 = v0[S.j1];
     ST x0 = S.on0 ? r0 : ST(0), x1 = S.on1 ? r1 : ST(0);
     ST y0 = ST(0), y1 = ST(0);
     if (NV > 1) { const ST s0 = v1[S.j0], s1 = v1[S.j1]; y0 = S.on0 ? s0 : ST(0); y1 = S.on1 ? s1 : ST(0); }
-    ST hb0 = ST(0), hb1 = ST(0);
-    if (g.wq == 0 && lane < 8) { hb0 = v0[3 + lane]; if (NV > 1) hb1 = v1[3 + lane]; }
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      if (q >= S.nlev) break;
+    ST hb0 = v0[3 + (lane & 7)], hb1 = NV > 1 ? v1[3 + (lane & 7)] : ST(0);
+    // levels 0..2 always, the others where a chain of the warp has more than eight rows: one branch per
+    // direction (a branch per level cost as much as the level it skipped)
+    auto fwd = [&](int q) {
       const int d = 1 << q;
       const ST px0 = shfl_up_(x0, d), px1 = shfl_up_(x1, d);
       x0 += S.f0[q] * px0; x1 += S.f1[q] * px1;
       if (NV > 1) { const ST py0 = shfl_up_(y0, d), py1 = shfl_up_(y1, d); y0 += S.f0[q] * py0; y1 += S.f1[q] * py1; }
-    }
-    if (g.wq == 0) {
-      // head: chain 0 (photon T tail) ends at F2 (lane 4), chain 1 (P tail) at G2 (lane 7)
-      const ST c0 = __shfl_sync(FULL, x0, S.n0 - 1), c1 = __shfl_sync(FULL, x1, S.n1 - 1);
-      const ST cf = lane == 4 ? c0 : c1;
-      if (lane == 4 || lane == 7) hb0 -= F.hm * cf;
-      ST o0 = 0, o1 = 0;
-      if (NV > 1) {
-        const ST e0 = __shfl_sync(FULL, y0, S.n0 - 1), e1 = __shfl_sync(FULL, y1, S.n1 - 1);
-        const ST ce = lane == 4 ? e0 : e1;
-        if (lane == 4 || lane == 7) hb1 -= F.hm * ce;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        o0 += F.hv[q] * __shfl_sync(FULL, hb0, q);
-        if (NV > 1) o1 += F.hv[q] * __shfl_sync(FULL, hb1, q);
-      }
-      if (lane < 8) { v0[3 + lane] = o0; if (NV > 1) v1[3 + lane] = o1; }
-    }
-    x0 *= S.d0; x1 *= S.d1;
-    if (NV > 1) { y0 *= S.d0; y1 *= S.d1; }
-#pragma unroll
-    for (int q = 0; q < 5; ++q) {
-      if (q >= S.nlev) break;
+    };
+    auto bwd = [&](int q) {
       const int d = 1 << q;
       const ST px0 = __shfl_down_sync(FULL, x0, d), px1 = __shfl_down_sync(FULL, x1, d);
       x0 += S.b0[q] * px0; x1 += S.b1[q] * px1;
@@ -292,21 +306,45 @@ __device__ __forceinline__ void lat_solve_M(const LGrp& g, const LatScan<ST>& S,
         const ST py0 = __shfl_down_sync(FULL, y0, d), py1 = __shfl_down_sync(FULL, y1, d);
         y0 += S.b0[q] * py0; y1 += S.b1[q] * py1;
       }
-    }
-    if (S.on0) { v0[S.i0] = x0; if (NV > 1) v1[S.i0] = y0; }
-    if (S.on1) { v0[S.i1] = x1; if (NV > 1) v1[S.i1] = y1; }
-  }
-  if (g.wq == 3) {
-    if (lane == 16 || lane == 17) {  // CDM: [[s, 1], [0, s+ℋ]]
-      ST* v = lane == 16 ? v0 : v1;
-      if (lane == 16 || NV > 1) {
-        const ST zt = v[2] * F.ihc;
-        v[2] = zt;
-        v[1] = (v[1] - zt) * F.is;
+    };
+    auto back = [&]() {
+      x0 *= S.d0; x1 *= S.d1;
+      if (NV > 1) { y0 *= S.d0; y1 *= S.d1; }
+      bwd(0); bwd(1); bwd(2);
+      if (S.more) { bwd(3); bwd(4); }
+      if (S.on0) { v0[S.i0] = x0; if (NV > 1) v1[S.i0] = y0; }
+      if (S.on1) { v0[S.i1] = x1; if (NV > 1) v1[S.i1] = y1; }
+    };
+    fwd(0); fwd(1); fwd(2);
+    if (S.more) { fwd(3); fwd(4); }
+    if (g.wq == 0) {
+      // head: chain 0 (photon T tail) ends at F2 (lane 4), chain 1 (P tail) at G2 (lane 7); hm is zero on
+      // the other lanes.  Its shuffles and the back substitution's are one straight run of code.
+      const ST c0 = __shfl_sync(FULL, x0, S.n0 - 1), c1 = __shfl_sync(FULL, x1, S.n1 - 1);
+      hb0 -= F.hm * (lane == 4 ? c0 : c1);
+      if (NV > 1) {
+        const ST e0 = __shfl_sync(FULL, y0, S.n0 - 1), e1 = __shfl_sync(FULL, y1, S.n1 - 1);
+        hb1 -= F.hm * (lane == 4 ? e0 : e1);
       }
-    } else if (lane == 18) {
-      v0[0] *= F.is;
-      if (NV > 1) v1[0] *= F.is;
+      ST q0[8], q1[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) { q0[q] = __shfl_sync(FULL, hb0, q); q1[q] = NV > 1 ? __shfl_sync(FULL, hb1, q) : ST(0); }
+      x0 *= S.d0; x1 *= S.d1;
+      if (NV > 1) { y0 *= S.d0; y1 *= S.d1; }
+      ST o0 = 0, o1 = 0;
+      bwd(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { o0 += F.hv[q] * q0[q]; if (NV > 1) o1 += F.hv[q] * q1[q]; }
+      bwd(1);
+#pragma unroll
+      for (int q = 4; q < 8; ++q) { o0 += F.hv[q] * q0[q]; if (NV > 1) o1 += F.hv[q] * q1[q]; }
+      bwd(2);
+      if (lane < 8) { v0[3 + lane] = o0; if (NV > 1) v1[3 + lane] = o1; }
+      if (S.more) { bwd(3); bwd(4); }
+      if (S.on0) { v0[S.i0] = x0; if (NV > 1) v1[S.i0] = y0; }
+      if (S.on1) { v0[S.i1] = x1; if (NV > 1) v1[S.i1] = y1; }
+    } else {
+      back();
     }
   }
   bar_sync(LB_MAIN, kSolvers);
@@ -344,101 +382,108 @@ __device__ __forceinline__ void lat_factor_inputs(const LGrp& g, LatMem<NSL, ST>
   F.fS[0] = to_st<ST>(cv[CV_PA]); F.fS[1] = to_st<ST>(cv[CV_PB]); F.fS[2] = to_st<ST>(cv[CV_MH]);
 }
 
-// Factorisation for the step size s = 1/(hγ); ends with the rank-2 columns z1, z2 and the head-value
-// factors P of the thread's rows in registers.
+// Chain LU from the truncation ends, one chain per lane of the control warp (precision ST); four rows are
+// read ahead of the serial pivot recurrence.  Then the photon tails' couplings to the head.
 template <int NSL, typename ST>
-__device__ __forceinline__ void lat_factorize(const LGrp& g, LatMem<NSL, ST>& W, LatFactor<ST>& F, LatScan<ST>& S, const Rows<NSL>& R, const CSet& C,
-                                              const CompDesc* __restrict__ comps, const ModelDesc& M, double k, double h, double s,
-                                              const double (&dg)[NSL], const int (&at)[NSL], ST (&z1)[NSL], ST (&z2)[NSL], ST (&P)[NSL]) {
+__device__ __forceinline__ void lat_chain_lu(int lane, LatMem<NSL, ST>& W, const ModelDesc& M) {
+  if (lane >= M.nchain) return;
+  const int first = M.chFirst[lane], last = M.chLast[lane];
+  ST dn = lat_rcp<ST>(W.dd[last]);
+  W.dinv[last] = dn; W.mfw[last] = 0;
+  for (int i = last - 1; i >= first; i -= 4) {
+    ST sp[4], sb[4], d[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = i - q > first ? i - q : first;
+      sp[q] = W.sup[r]; sb[q] = W.sub[r + 1]; d[q] = W.dd[r];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (i - q >= first) {
+        const ST di = lat_rcp<ST>(d[q] - sp[q] * sb[q] * dn);
+        W.dinv[i - q] = di; W.mfw[i - q] = sp[q] * dn;
+        dn = di;
+      }
+  }
+  if (lane < 2) {  // coupling of x[first] into the head row (F2, G2)
+    const ST hs = W.sup[M.chAttach[lane]];
+    const ST hm = hs * dn;
+    W.hmul[lane] = hm;
+    W.hcorr[lane] = hm * W.sub[first];
+  }
+}
+
+// Factorisation for the step size s = 1/(hγ), first part: diagonals to the control warp, which runs the
+// chain LU and inverts the head, and the head rows (solver warp 3).
+template <int NSL, typename ST>
+__device__ __forceinline__ void lat_factor_start(const LGrp& g, LatMem<NSL, ST>& W, LatFactor<ST>& F, const Rows<NSL>& R, const CSet& C,
+                                                 const CompDesc* __restrict__ comps, int n, double k, double h, double s, const double (&dg)[NSL]) {
   const int lane = g.lane;
   const double* cv = C.cv;
 #pragma unroll
-  for (int sl = 0; sl < NSL; ++sl) { const int i = R.i[sl]; if (i < M.n) W.dd[i] = to_st<ST>(s - dg[sl]); }
-  bar_sync(LB_MAIN, kSolvers);
-  if (g.wq == 0 && lane < M.nchain) {  // chain LU from the truncation end; the next row is read ahead of the recurrence
-    const int ch = lane, first = M.chFirst[ch], last = M.chLast[ch];
-    ST dn = rcp<ST>(W.dd[last]);
-    W.dinv[last] = dn; W.mfw[last] = 0;
-    int i = last - 1;
-    ST sp = W.sup[i], sb = W.sub[i + 1], d = W.dd[i];  // a one-row chain reads the row before it and uses nothing
-    while (i >= first) {
-      const int ni = i > first ? i - 1 : i;
-      const ST nsp = W.sup[ni], nsb = W.sub[ni + 1], nd = W.dd[ni];
-      const ST di = rcp<ST>(d - sp * sb * dn);
-      W.dinv[i] = di; W.mfw[i] = sp * dn;
-      dn = di; sp = nsp; sb = nsb; d = nd;
-      --i;
-    }
-    if (ch < 2) {  // coupling of x[first] into the head row (F2, G2)
-      const ST hs = W.sup[M.chAttach[ch]];
-      const ST hm = hs * dn;
-      W.hmul[ch] = hm;
-      W.hcorr[ch] = hm * W.sub[first];
-    }
-  }
-  if (g.wq == 3 && lane >= 16 && lane < 24) {  // assemble head row 3 + j
-    const int j = lane - 16, r = 3 + j;
-    const double k34 = 0.75 * k;
-    const CompDesc& D = comps[r];
-    double row[8];
+  for (int sl = 0; sl < NSL; ++sl) { const int i = R.i[sl]; if (i < n) W.dd[i] = to_st<ST>(s - dg[sl]); }
+  bar_arrive(LB_DD, kSolvers + 32);
+  if (g.wq == 3) {
+    if (lane >= 16 && lane < 24) {  // assemble head row 3 + j
+      const int j = lane - 16, r = 3 + j;
+      const double k34 = 0.75 * k;
+      const CompDesc& D = comps[r];
+      double row[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) row[c] = 0;
-    row[j] += s - cv[D.dg];
-    const double spv = cv[D.sp];
-    int c;
-    if ((c = head_local(D.ip)) >= 0) row[c] -= spv * D.A;
-    if ((c = head_local(D.inx)) >= 0) row[c] -= spv * D.C;
-    if ((c = head_local(D.e0c)) >= 0) row[c] -= cv[D.e0];
-    if ((c = head_local(D.e1c)) >= 0) row[c] -= cv[D.e1];
-    if ((c = head_local(D.e2c)) >= 0) row[c] -= cv[D.e2];
-    if ((c = head_local(D.dxa)) >= 0) row[c] -= cv[D.dx];
-    if ((c = head_local(D.dxb)) >= 0) row[c] += k34 * cv[D.dx];
+      for (int c = 0; c < 8; ++c) row[c] = 0;
+      row[j] += s - cv[D.dg];
+      const double spv = cv[D.sp];
+      int c;
+      if ((c = head_local(D.ip)) >= 0) row[c] -= spv * D.A;
+      if ((c = head_local(D.inx)) >= 0) row[c] -= spv * D.C;
+      if ((c = head_local(D.e0c)) >= 0) row[c] -= cv[D.e0];
+      if ((c = head_local(D.e1c)) >= 0) row[c] -= cv[D.e1];
+      if ((c = head_local(D.e2c)) >= 0) row[c] -= cv[D.e2];
+      if ((c = head_local(D.dxa)) >= 0) row[c] -= cv[D.dx];
+      if ((c = head_local(D.dxb)) >= 0) row[c] += k34 * cv[D.dx];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) W.H[j * 8 + q] = to_st<ST>(row[q]);
+      for (int q = 0; q < 8; ++q) W.H[j * 8 + q] = to_st<ST>(row[q]);
+    }
+    __syncwarp();
+    bar_arrive(LB_HROW, 64);
   }
   F.is = to_st<ST>(h * TB::gam);
-  F.ihc = rcp<ST>(to_st<ST>(s - cv[CV_MH]));
+  F.ihc = lat_rcp<ST>(to_st<ST>(s - cv[CV_MH]));
+}
+
+// Second part, from the chain pivots: ends with the rank-2 columns z1, z2 and the head-value factors P of
+// the thread's rows in registers.
+template <int NSL, typename ST>
+__device__ __forceinline__ void lat_factor_finish(const LGrp& g, LatMem<NSL, ST>& W, LatFactor<ST>& F, LatScan<ST>& S, const Rows<NSL>& R,
+                                                  const ModelDesc& M, const int (&at)[NSL], ST (&z1)[NSL], ST (&z2)[NSL], ST (&P)[NSL]) {
+  const int lane = g.lane;
   bar_sync(LB_LU, kSolvers + 32);
-  if (S.pair) {  // Kogge-Stone multipliers of both recurrences of the warp's two chains
-#pragma unroll
-    for (int hc = 0; hc < 2; ++hc) {
-      const int j = hc ? S.j1 : S.j0, L = hc ? S.n1 : S.n0;
-      const bool on = hc ? S.on1 : S.on0;
-      const ST di = W.dinv[j];
-      ST a = (on && lane > 0) ? -W.mfw[j] : ST(0);
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const int d = 1 << q;
-        ST m = ST(0);
-        if (q < S.nlev) {
-          const ST ap = shfl_up_(a, d);
-          m = (on && lane >= d) ? a : ST(0);
-          if (lane >= d) a *= ap;
-        }
-        if (hc) S.f1[q] = m; else S.f0[q] = m;
-      }
-      a = on ? -di * W.sub[j] : ST(0);
-#pragma unroll
-      for (int q = 0; q < 5; ++q) {
-        const int d = 1 << q;
-        ST m = ST(0);
-        if (q < S.nlev) {
-          const ST ap = __shfl_down_sync(FULL, a, d);
-          const bool in = lane + d < L;
-          m = (on && in) ? a : ST(0);
-          if (in) a *= ap;
-        }
-        if (hc) S.b1[q] = m; else S.b0[q] = m;
-      }
-      if (hc) S.d1 = on ? di : ST(0); else S.d0 = on ? di : ST(0);
-      if (on) W.bP[j] = a;  // ∂z_i/∂h
-    }
+  if (S.pair) {  // Kogge-Stone multipliers of both recurrences of the warp's two chains, side by side
+    const ST e0 = W.dinv[S.j0], e1 = W.dinv[S.j1], m0 = W.mfw[S.j0], m1 = W.mfw[S.j1], u0 = W.sub[S.j0], u1 = W.sub[S.j1];
+    ST a0 = (S.on0 && lane > 0) ? -m0 : ST(0), a1 = (S.on1 && lane > 0) ? -m1 : ST(0);
+    ST c0 = S.on0 ? -e0 * u0 : ST(0), c1 = S.on1 ? -e1 * u1 : ST(0);
+    auto level = [&](int q) {
+      const int d = 1 << q;
+      const ST p0 = shfl_up_(a0, d), p1 = shfl_up_(a1, d);
+      const ST q0 = __shfl_down_sync(FULL, c0, d), q1 = __shfl_down_sync(FULL, c1, d);
+      const bool up = lane >= d, in0 = lane + d < S.n0, in1 = lane + d < S.n1;
+      S.f0[q] = (S.on0 && up) ? a0 : ST(0); S.f1[q] = (S.on1 && up) ? a1 : ST(0);
+      S.b0[q] = (S.on0 && in0) ? c0 : ST(0); S.b1[q] = (S.on1 && in1) ? c1 : ST(0);
+      if (up) { a0 *= p0; a1 *= p1; }
+      if (in0) c0 *= q0;
+      if (in1) c1 *= q1;
+    };
+    level(0); level(1); level(2);
+    if (S.more) { level(3); level(4); }
+    S.d0 = S.on0 ? e0 : ST(0); S.d1 = S.on1 ? e1 : ST(0);
+    if (S.on0) W.bP[S.j0] = c0;  // ∂z_i/∂h
+    if (S.on1) W.bP[S.j1] = c1;
   }
   bar_sync(LB_HEAD, kSolvers + 32);
   if (g.wq == 0) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) F.hv[q] = W.Hinv[(lane & 7) * 8 + q];
-    F.hm = lane == 4 ? W.hmul[0] : W.hmul[1];
+    F.hm = lane == 4 ? W.hmul[0] : lane == 7 ? W.hmul[1] : ST(0);
   }
   // rank-2 correction: Z1 = M⁻¹ c_Φ̇, Z2 = M⁻¹ c_Ψ
   lat_solve_M<2, NSL, ST>(g, S, F, W.Z1, W.Z2);
@@ -454,7 +499,7 @@ __device__ __forceinline__ void lat_factorize(const LGrp& g, LatMem<NSL, ST>& W,
   lat_functionals_st(g, F, W.Z1, psi1, p1);
   lat_functionals_st(g, F, W.Z2, psi2, p2);
   const ST a = 1 - p1, b = -p2, c = -psi1, d = 1 - psi2;
-  const ST idet = ST(1) / (a * d - b * c);
+  const ST idet = sizeof(ST) == 8 ? lat_rcp<ST>(a * d - b * c) : ST(1) / (a * d - b * c);
   F.S00 = d * idet; F.S01 = -b * idet; F.S10 = -c * idet; F.S11 = a * idet;
 }
 
@@ -490,14 +535,25 @@ __device__ void lat_emit(const LGrp& g, LatMem<NSL, ST>& W, const Rows<NSL>& R, 
   bar_sync(LB_MAIN, kSolvers);
 }
 
-// Step control as ptk::pt_body publishes it, the divisions and stage times one per lane.
+// Step control as ptk::pt_body publishes it, in two parts: flags, h, 1/h and 1/(hγ) (what the solver warps
+// wait for; the divisions one per lane), then the step end and the stage times.  Returns the step end.
 template <int NSL, typename ST>
-__device__ __forceinline__ void lat_publish(int lane, LatMem<NSL, ST>& W, double hp, double tc, double tend) {
+__device__ __forceinline__ double lat_publish(int lane, LatMem<NSL, ST>& W, double& hp, double tc, double tend) {
+  // the divisions start before the clamp to the end point, which is rare, is decided
+  double inv = 1.0 / (lane == 1 ? hp * TB::gam : hp);
   const bool done = !(tc < tend);
-  if (tc + 1.01 * hp >= tend) hp = tend - tc;
-  const double te = (hp == tend - tc) ? tend : tc + hp;
+  const double left = tend - tc;
+  if (tc + 1.01 * hp >= tend) {
+    hp = left;
+    inv = 1.0 / (lane == 1 ? hp * TB::gam : hp);
+  }
   const bool tiny = !(hp > 1e-14 * tc);
-  const double inv = 1.0 / (lane == 1 ? hp * TB::gam : hp);
+  if (lane == 0) { W.ctlf = (done ? 1 : 0) | (tiny ? 2 : 0); W.ctl[0] = hp; W.ctl[1] = inv; }
+  if (lane == 1) W.ctl[2] = inv;
+  return (hp == left) ? tend : tc + hp;
+}
+template <int NSL, typename ST>
+__device__ __forceinline__ void lat_publish_times(int lane, LatMem<NSL, ST>& W, double hp, double tc, double te) {
   double c = 0;  // stage time lane - 4 + 1 of the tableau
 #pragma unroll
   for (int q = 1; q < TB::NTIME; ++q) {
@@ -507,8 +563,7 @@ __device__ __forceinline__ void lat_publish(int lane, LatMem<NSL, ST>& W, double
     if (lane == 3 + q) c = TB::c(st);
   }
   const double ts = tc + c * hp;
-  if (lane == 0) { W.ctlf = (done ? 1 : 0) | (tiny ? 2 : 0); W.ctl[0] = hp; W.ctl[1] = inv; W.ctl[3] = te; W.ctl[4 + TB::NTIME - 1] = te; }
-  if (lane == 1) W.ctl[2] = inv;
+  if (lane == 0) { W.ctl[3] = te; W.ctl[4 + TB::NTIME - 1] = te; }
   if (lane >= 4 && lane < 4 + TB::NTIME - 1) W.ctl[lane] = ts;
 }
 
@@ -598,8 +653,11 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
     bar_sync(LB_MAIN, kSolvers);
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) if (R.i[sl] < n) W.x[R.i[sl]] = y[sl];
-    if (g.wq == 1) lat_publish(g.lane, W, h, t, tend);
-    bool nonfinite = false;
+    if (g.wq == 1) {
+      const double te = lat_publish(g.lane, W, h, t, tend);
+      lat_publish_times(g.lane, W, h, t, te);
+    }
+    bool nonfinite = false, moved = false;  // moved: y is new since f0 and ft were formed
     LatFactor<ST> F;
     double dg[NSL];
     int64_t iters = 0;
@@ -613,17 +671,21 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
       if (++iters > A.maxiters) { status = SBZ_MAXITERS; break; }
       if (fl & 2) { status = nonfinite ? SBZ_NONFINITE : SBZ_DTMIN; break; }
       h = W.ctl[0];
-      const double ih = W.ctl[1], s = W.ctl[2], tn = W.ctl[3];
+      const double ih = W.ctl[1], s = W.ctl[2];
       const CSet& CJ = W.cs[sJ];
       ST z1[NSL], z2[NSL], P[NSL];
-      lat_factorize(g, W, F, S, R, CJ, comps, M, k, h, s, dg, at, z1, z2, P);
+      lat_factor_start(g, W, F, R, CJ, comps, n, k, h, s, dg);
+      if (moved) lat_matvec<NSL, ST, true, false>(g, W, R, W.x, CJ, k34, f0, ft, false);  // f(t, y), ∂f/∂τ, beside the chain LU
+      lat_factor_finish(g, W, F, S, R, M, at, z1, z2, P);
+      const double tn = W.ctl[3];
       double b[NSL], Fv[NSL], Y[NSL], Ul[NSL], un[NSL];
       float isk[NSL];  // refinement stopping weights
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) isk[sl] = 1.0f / f64_to_f32(atol + rtol * fabs(y[sl]));
       int rk = A.refine;
-      // the stage count read at run time: one copy of the stage body
-      const int nst = *reinterpret_cast<const volatile int*>(&kRos.nst);
+      // the stage count opaque to the compiler: one copy of the stage body
+      int nst;
+      asm volatile("mov.u32 %0, %1;" : "=r"(nst) : "n"(TB::S));
 #pragma unroll 1
       for (int st = 0; st < nst; ++st) {
         if (st == 0) {
@@ -631,29 +693,28 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
           for (int sl = 0; sl < NSL; ++sl) b[sl] = fma(h * TB::d(0), ft[sl], f0[sl]);
         } else {
           double cu[NSL];
+          const double ka = W.tA[st], kc = W.tC[st], kd = W.td[st];
+          const int kq = W.tq[st], kinc = W.tinc[st];
+          const double hdst = h * kd;
           if (st == 1) {
 #pragma unroll
-            for (int sl = 0; sl < NSL; ++sl) { Y[sl] = fma(kRos.A[1][0], Ul[sl], y[sl]); cu[sl] = kRos.C[1][0] * Ul[sl]; }
+            for (int sl = 0; sl < NSL; ++sl) { Y[sl] = fma(ka, Ul[sl], y[sl]); cu[sl] = kc * Ul[sl]; }
           } else {
             // the companions' sums and the last stage's term; stages 7 and 8 add the previous stage
             bar_sync(LB_SUM, kLatThreads);
-            const double a = kRos.A[st][st - 1], c = kRos.C[st][st - 1];
-            const bool inc = kRos.incr[st] != 0;
 #pragma unroll
             for (int sl = 0; sl < NSL; ++sl) {
-              if (inc) Y[sl] = Y[sl] + Ul[sl];
-              else Y[sl] = fma(a, Ul[sl], W.PA[R.i[sl]]);
-              cu[sl] = fma(c, Ul[sl], W.PC[R.i[sl]]);
+              if (kinc) Y[sl] = Y[sl] + Ul[sl];
+              else Y[sl] = fma(ka, Ul[sl], W.PA[R.i[sl]]);
+              cu[sl] = fma(kc, Ul[sl], W.PC[R.i[sl]]);
             }
           }
 #pragma unroll
           for (int sl = 0; sl < NSL; ++sl) if (R.i[sl] < n) W.x[R.i[sl]] = Y[sl];
           if (st == 1) bar_sync(LB_COEF, kSolvers + 96);
           bar_sync(LB_MAIN, kSolvers);
-          const int q = kRos.tslot[st];
-          lat_matvec<NSL, ST, false, false>(g, W, R, W.x, W.cs[q < TB::NTIME ? q : sE], k34, Fv, un, false);
-          const bool hd = kRos.hasd[st] != 0;
-          const double hdst = h * kRos.d[st];
+          lat_matvec<NSL, ST, false, false>(g, W, R, W.x, W.cs[kq < TB::NTIME ? kq : sE], k34, Fv, un, false);
+          const bool hd = (dkey(kd) & 0x7fffffffffffffffll) != 0;
 #pragma unroll
           for (int sl = 0; sl < NSL; ++sl) {
             b[sl] = fma(ih, cu[sl], Fv[sl]);
@@ -710,13 +771,12 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
         for (int sl = 0; sl < NSL; ++sl) W.Us[st][R.i[sl]] = Ul[sl];
       }
       // new state (stiffly accurate: y1 = last stage input + last stage); the companions form the error
-      // norm and the next step while f(t1, y1), the next step's ∂f/∂τ and the factorisation's inputs are
-      // formed as if it were accepted
-      double y1[NSL], f1[NSL], ft1[NSL];
+      // norm and the next step while the factorisation's inputs are formed as if it were accepted (the
+      // FP64 pipes are left to them: f(t1, y1) waits for the chain LU)
+      double y1[NSL];
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) { y1[sl] = Y[sl] + Ul[sl]; if (R.i[sl] < n) W.x[R.i[sl]] = y1[sl]; }
       bar_sync(LB_STEP, kLatThreads);
-      lat_matvec<NSL, ST, true, false>(g, W, R, W.x, W.cs[sE], k34, f1, ft1, false);
       lat_factor_inputs(g, W, F, R, W.cs[sE], n, dg);
       bar_sync(LB_CTL, kSolvers + 32);
       const int acc = W.accept;
@@ -746,16 +806,21 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
             lat_emit(g, W, R, A, cd, tab, M, mk, tau, yo, item, jout);
             ++jout;
           }
+#pragma unroll
+          for (int sl = 0; sl < NSL; ++sl) if (R.i[sl] < n) W.x[R.i[sl]] = y1[sl];  // operator input of f(t1, y1)
+          bar_sync(LB_MAIN, kSolvers);
         }
         t = tn;
 #pragma unroll
-        for (int sl = 0; sl < NSL; ++sl) { y[sl] = y1[sl]; f0[sl] = f1[sl]; ft[sl] = ft1[sl]; }
+        for (int sl = 0; sl < NSL; ++sl) y[sl] = y1[sl];
         ++nacc;
         nonfinite = false;
+        moved = true;
       } else {
         ++nrej;
         nonfinite = acc == 2;
-        // J's coefficients (at t) and ∂f/∂τ stay valid; the companions now may refill the step-end set
+        moved = false;
+        // J's coefficients (at t), f and ∂f/∂τ stay valid; the companions now may refill the step-end set
         bar_sync(LB_REJ, kLatThreads);
         lat_factor_inputs(g, W, F, R, W.cs[sJ], n, dg);
       }
@@ -798,9 +863,9 @@ __device__ __forceinline__ void lat_head_inverse(int lane, LatMem<NSL, ST>& W) {
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk) {
     int p = kk;
-    ST best = fabs(col[kk]);
+    auto best = mag_key(col[kk]);
 #pragma unroll
-    for (int r = kk + 1; r < 8; ++r) { const ST v = fabs(col[r]); if (v > best) { best = v; p = r; } }
+    for (int r = kk + 1; r < 8; ++r) { const auto v = mag_key(col[r]); if (v > best) { best = v; p = r; } }
     p = __shfl_sync(FULL, p, kk);
     ST vp = col[kk];
 #pragma unroll
@@ -809,7 +874,7 @@ __device__ __forceinline__ void lat_head_inverse(int lane, LatMem<NSL, ST>& W) {
     ST m[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) m[r] = __shfl_sync(FULL, col[r], kk);
-    const ST ip = rcp<ST>(m[kk]);
+    const ST ip = lat_rcp<ST>(m[kk]);
     col[kk] *= ip;
 #pragma unroll
     for (int r = 0; r < 8; ++r) if (r != kk) col[r] -= m[r] * col[kk];
@@ -854,30 +919,52 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
   if (!(t < tend)) return;
   constexpr double kLogErrFloor = -9.210340371976184;  // log(1e-4): the controller's floor on errold
   double lerrold = kLogErrFloor;  // log of the previous accepted error norm
-  bool rejected = false, nonfinite = false;
+  bool rejected = false, nonfinite = false, first = true;
+  double tn = t;
   int sJ = 0, sE = TB::NTIME;
   int64_t iters = 0;
-  int ci[NSL];
-  double y[NSL], y1[NSL];
+  int ci[NSL], si[NSL];  // rows in the error norm (its sum's order) and in the stage sums (slot 1 on warp 3)
+  double y[NSL], y1[NSL], ys = 0, ys1 = 0;  // state rows of ci, and of si[1]
 #pragma unroll
-  for (int sl = 0; sl < NSL; ++sl) ci[sl] = comp_of<4>(gt, sl);
+  for (int sl = 0; sl < NSL; ++sl) { ci[sl] = comp_of<4>(gt, sl); si[sl] = sl * kSolvers + ((gt + 32 * sl) & (kSolvers - 1)); }
+  bool act[NSL];
+#pragma unroll
+  for (int sl = 0; sl < NSL; ++sl) act[sl] = __any_sync(FULL, si[sl] < n);
   bar_sync(LB_STEP, kLatThreads);
 #pragma unroll
   for (int sl = 0; sl < NSL; ++sl) y[sl] = ci[sl] < n ? W.x[ci[sl]] : 0.0;
+  if (NSL > 1) ys = si[NSL - 1] < n ? W.x[si[NSL - 1]] : 0.0;
   for (;;) {
-    if (g.wq == 3) bar_arrive(LB_CTL, kSolvers + 32);
+    if (first && g.wq == 3) bar_arrive(LB_CTL, kSolvers + 32);  // the first step's control is the solvers'
     bar_sync(LB_COMP, kSolvers);  // control seen by every companion warp
-    if (rejected) bar_sync(LB_REJ, kLatThreads);
+    if (!first) {
+      rejected = W.accept != 1;
+      if (rejected) {
+        bar_sync(LB_REJ, kLatThreads);
+      } else {
+        t = tn;
+#pragma unroll
+        for (int sl = 0; sl < NSL; ++sl) y[sl] = y1[sl];
+        ys = ys1;
+        const int tsw = sJ; sJ = sE; sE = tsw;
+      }
+    }
+    first = false;
     const int fl = W.ctlf;  // the solver warps leave the loop on the same tests, in the same order
     if (fl & 1) break;
     if (++iters > A.maxiters) break;
     if (fl & 2) break;
-    const double h = W.ctl[0], tn = W.ctl[3];
+    const double h = W.ctl[0];
+    tn = W.ctl[3];
     if (g.wq < 3) {
       lat_coefs(g, W, sE, cd, tab, M, mk);
       bar_arrive(LB_COEF, kSolvers + 96);
     } else {
-      bar_sync(LB_LU, kSolvers + 32);
+      bar_sync(LB_DD, kSolvers + 32);
+      lat_chain_lu(g.lane, W, M);
+      __syncwarp();
+      bar_arrive(LB_LU, kSolvers + 32);
+      bar_sync(LB_HROW, 64);
       lat_head_inverse(g.lane, W);
       __syncwarp();
       bar_arrive(LB_HEAD, kSolvers + 32);
@@ -887,7 +974,7 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) a[q][sl] = y[sl];
+      for (int q = 0; q < 4; ++q) a[q][sl] = sl == 0 ? y[sl] : ys;
 #pragma unroll
       for (int q = 0; q < 6; ++q) c[q][sl] = 0;
     }
@@ -897,17 +984,17 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
       double u[NSL];
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl) {
-        u[sl] = ci[sl] < n ? W.Us[j][ci[sl]] : 0.0;
-        if ((g.act >> sl) & 1u) {
-          if (j + 2 < 6) { a[j < 4 ? j : 0][sl] = fma(TB::A(j + 2, j), u[sl], a[j < 4 ? j : 0][sl]); W.PA[ci[sl]] = a[j < 4 ? j : 0][sl]; }
+        u[sl] = si[sl] < n ? W.Us[j][si[sl]] : 0.0;
+        if (act[sl]) {
+          if (j + 2 < 6) { a[j < 4 ? j : 0][sl] = fma(TB::A(j + 2, j), u[sl], a[j < 4 ? j : 0][sl]); W.PA[si[sl]] = a[j < 4 ? j : 0][sl]; }
           c[j][sl] = fma(TB::C(j + 2, j), u[sl], c[j][sl]);
-          W.PC[ci[sl]] = c[j][sl];
+          W.PC[si[sl]] = c[j][sl];
         }
       }
       bar_arrive(LB_SUM, kLatThreads);
 #pragma unroll
       for (int sl = 0; sl < NSL; ++sl)
-        if ((g.act >> sl) & 1u) {
+        if (act[sl]) {
 #pragma unroll
           for (int i = j + 3; i < TB::S; ++i) {
             if (i < 6) a[i - 2][sl] = fma(TB::A(i, j), u[sl], a[i - 2][sl]);
@@ -918,6 +1005,7 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
     // FP64 error norm of the last stage
     bar_sync(LB_STEP, kLatThreads);
     double e2 = 0;
+    if (NSL > 1) ys1 = si[NSL - 1] < n ? W.x[si[NSL - 1]] : 0.0;
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) {
       const int i = ci[sl];
@@ -929,13 +1017,23 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
         e2 += q * q;
       }
     }
-    const double err2 = lat_sum(g, W.rede, LB_COMP, e2) * inv_n;  // squared RMS error norm
-    // err2 >= 0: accepted when finite and at most 1, by its bit pattern (inf, NaN and any sign-bit
-    // pattern compare above 1 as unsigned)
-    const bool ok = (unsigned long long)dkey(err2) <= (unsigned long long)dkey(1.0);
-    if (ok) nonfinite = false;
-    else if ((dkey(err2) & 0x7ff0000000000000ll) == 0x7ff0000000000000ll) nonfinite = true;  // inf or NaN, kept until a step is accepted
-    if (g.wq == 3) {
+    e2 = warp_sum(e2);
+    if (g.lane == 0) W.rede[g.wq] = e2;
+    __syncwarp();
+    if (g.wq < 3) {
+      bar_arrive(LB_ERR, kSolvers);
+    } else {  // step control
+      bar_sync(LB_ERR, kSolvers);
+      double err2 = 0;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) err2 += W.rede[w];
+      err2 *= inv_n;  // squared RMS error norm
+      // err2 >= 0: accepted when finite and at most 1, by its bit pattern (inf, NaN and any sign-bit
+      // pattern compare above 1 as unsigned)
+      const bool ok = (unsigned long long)dkey(err2) <= (unsigned long long)dkey(1.0);
+      if (ok) nonfinite = false;
+      else if ((dkey(err2) & 0x7ff0000000000000ll) == 0x7ff0000000000000ll) nonfinite = true;  // inf or NaN, kept until a step is accepted
+      double hp;
       if (ok) {
         // PI controller fac = 0.9 err^-beta1 errold^beta2 (OrdinaryDiffEq's defaults for the method's order)
         const double lerr = 0.5 * log(dmax(err2, 1e-20));
@@ -943,19 +1041,16 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
         fac = dmin(10.0, dmax(0.2, fac));
         if (rejected) fac = dmin(fac, 1.0);
         lerrold = dmax(lerr, kLogErrFloor);
-        lat_publish(g.lane, W, h * fac, tn, tend);
+        hp = h * fac;
       } else {
-        lat_publish(g.lane, W, nonfinite ? 0.2 * h : h * dmax(0.2, 0.9 * exp(-0.5 * TB::rej * log(err2))), t, tend);
+        hp = nonfinite ? 0.2 * h : h * dmax(0.2, 0.9 * exp(-0.5 * TB::rej * log(err2)));
       }
       if (g.lane == 0) W.accept = ok ? 1 : nonfinite ? 2 : 0;
+      const double tc = ok ? tn : t;
+      const double te = lat_publish(g.lane, W, hp, tc, tend);
       __syncwarp();
-    }
-    rejected = !ok;
-    if (ok) {
-      t = tn;
-#pragma unroll
-      for (int sl = 0; sl < NSL; ++sl) y[sl] = y1[sl];
-      const int tsw = sJ; sJ = sE; sE = tsw;
+      bar_arrive(LB_CTL, kSolvers + 32);
+      lat_publish_times(g.lane, W, hp, tc, te);
     }
   }
 }
@@ -972,6 +1067,10 @@ __global__ void __launch_bounds__(kLatThreads, 1) pt_lat_kernel(PtArgs A) {
   for (int i = tid; i < A.model_n * (int)sizeof(CompDesc) / 4; i += kLatThreads) reinterpret_cast<int*>(comps)[i] = reinterpret_cast<const int*>(A.comps)[i];
   for (int i = tid; i < kNSets * (int)(sizeof(CSet) / sizeof(double)); i += kLatThreads) reinterpret_cast<double*>(W.cs)[i] = 0;
   for (int i = tid; i <= kSolvers * NSL; i += kLatThreads) { W.x[i] = 0; W.f[i] = 0; W.r[i] = 0; W.Z1[i] = 0; W.Z2[i] = 0; }
+  if (tid < TB::S) {
+    W.tA[tid] = tid ? kRos.A[tid][tid - 1] : 0.0; W.tC[tid] = tid ? kRos.C[tid][tid - 1] : 0.0; W.td[tid] = kRos.d[tid];
+    W.tq[tid] = kRos.tslot[tid]; W.tinc[tid] = kRos.incr[tid];
+  }
   for (int i = tid; i < kSolvers * NSL; i += kLatThreads) { W.PA[i] = 0; W.PC[i] = 0; W.bP[i] = 0; }
   __syncthreads();
   const bool solver = tid < kSolvers;
@@ -1005,7 +1104,7 @@ __global__ void __launch_bounds__(kLatThreads, 1) pt_lat_kernel(PtArgs A) {
     S.on0 = S.i0 >= f0; S.on1 = S.i1 >= f1;
     S.j0 = S.on0 ? S.i0 : 0; S.j1 = S.on1 ? S.i1 : 0;
     const int L = S.n0 > S.n1 ? S.n0 : S.n1;
-    S.nlev = L > 16 ? 5 : L > 8 ? 4 : L > 4 ? 3 : L > 2 ? 2 : 1;
+    S.more = L > 8;
 #pragma unroll
     for (int q = 0; q < 5; ++q) { S.f0[q] = S.f1[q] = S.b0[q] = S.b1[q] = ST(0); }
     S.d0 = S.d1 = ST(0);
