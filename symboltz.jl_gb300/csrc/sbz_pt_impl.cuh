@@ -406,15 +406,16 @@ __device__ __forceinline__ void coef_eval(const Grp<NW>& g, ModeMem<NW, NSL, ST>
 
 // The τ-independent coefficients of a mode (functions of k and the cosmology), into every set once
 // per mode; coef_eval then forms only the first M.nexpr_t expressions (40 of 53 at nx = 5).
-__device__ __forceinline__ void coef_mode(int tid, int nthr, CSet* cs, const CosmoDesc* cd, const ModelDesc& M, const ModeK& mk) {
-  const int nc = M.nexpr - M.nexpr_t;
+__device__ __forceinline__ void coef_mode_set(int tid, int nthr, double* cv, double* w, const CosmoDesc* cd, const ModelDesc& M, const ModeK& mk) {
   auto base = [&](int b) { return b == B_ONE ? 1.0 : b == B_K ? mk.k : b == B_K2 ? mk.k2 : b == B_IK ? mk.ik : mk.ik2; };
-  for (int p = tid; p < nc * kNSets; p += nthr) {
-    const CoefExpr& X = cd->expr[M.nexpr_t + p % nc];
+  for (int e = M.nexpr_t + tid; e < M.nexpr; e += nthr) {
+    const CoefExpr& X = cd->expr[e];
     const double val = fma(X.K1, base(X.b[0]) * (base(X.b[1]) * base(X.b[2])), X.K2 * (base(X.b[3]) * (base(X.b[4]) * base(X.b[5]))));
-    CSet& C = cs[p / nc];
-    if (X.dest < kNCV) C.cv[X.dest] = val; else C.w[X.dest - kNCV] = val;
+    if (X.dest < kNCV) cv[X.dest] = val; else w[X.dest - kNCV] = val;
   }
+}
+__device__ __forceinline__ void coef_mode(int tid, int nthr, CSet* cs, const CosmoDesc* cd, const ModelDesc& M, const ModeK& mk) {
+  for (int q = 0; q < kNSets; ++q) coef_mode_set(tid, nthr, cs[q].cv, cs[q].w, cd, M, mk);
 }
 
 // Metric functionals of a shared-memory vector v (every warp computes them): Ψ(v) and the δρ
