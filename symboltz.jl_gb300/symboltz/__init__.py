@@ -490,27 +490,26 @@ class CubicSplineInterpolator:
 
     def matrix(self, kfine):
         n = len(self.xs)
-        M = np.zeros((len(kfine), n))
-        for j in range(n):
-            e = np.zeros(n)
-            e[j] = 1.0
-            M[:, j] = _natural_spline(self.ys, e, self.f(np.asarray(kfine, dtype=np.float64)))
+        M = _natural_spline(self.ys, np.eye(n), self.f(np.asarray(kfine, dtype=np.float64)))
         return M
 
 
 def _natural_spline(x, y, xq):
+    """Natural cubic spline through (x, y) at xq; y may have several columns (one solve for all)."""
     n = len(x)
     h = np.diff(x)
     A = np.zeros((n, n))
-    r = np.zeros(n)
+    r = np.zeros(y.shape)
+    i = np.arange(1, n - 1)
     A[0, 0] = A[-1, -1] = 1
-    for i in range(1, n - 1):
-        A[i, i - 1], A[i, i], A[i, i + 1] = h[i - 1], 2 * (h[i - 1] + h[i]), h[i]
-        r[i] = 6 * ((y[i + 1] - y[i]) / h[i] - (y[i] - y[i - 1]) / h[i - 1])
+    A[i, i - 1], A[i, i], A[i, i + 1] = h[:-1], 2 * (h[:-1] + h[1:]), h[1:]
+    col = (slice(None),) + (None,) * (y.ndim - 1)
+    dy = np.diff(y, axis=0) / h[col]
+    r[1:-1] = 6 * np.diff(dy, axis=0)
     z = np.linalg.solve(A, r)
     i = np.clip(np.searchsorted(x, xq) - 1, 0, n - 2)
-    a, b = x[i + 1] - xq, xq - x[i]
-    hh = h[i]
+    a, b = (x[i + 1] - xq)[col], (xq - x[i])[col]
+    hh = h[i][col]
     return z[i] * a**3 / (6 * hh) + z[i + 1] * b**3 / (6 * hh) + (y[i + 1] / hh - z[i + 1] * hh / 6) * b + (y[i] / hh - z[i] * hh / 6) * a
 
 
@@ -652,7 +651,7 @@ def _spectrum_cmb_driver(modes, prob: CosmologyProblem, jl: SphericalBesselCache
         out *= (ls * (ls + 1) / (2 * np.pi))[:, None]
     if ls_out is not None:
         ls_out = np.asarray(ls_out, dtype=np.float64)
-        out = np.stack([_natural_spline(ls, out[:, i], ls_out) for i in range(len(modes))], axis=1)
+        out = _natural_spline(ls, out, ls_out)
     return (out, st) if return_status else out
 
 
