@@ -143,7 +143,7 @@ enum { T_H2D = 0, T_PT, T_KINTERP, T_LOS, T_CL, T_D2H, T_TOTAL };
 struct sbz_bessel {
   sbz::BesselDev J{};
   std::vector<int> ls;
-  DevBuf d_y, d_dy, d_yf2, d_ls;
+  DevBuf d_y, d_dy, d_yf2, d_ls, d_cf;
   DevBuf d_S, d_taus, d_chi, d_w, d_ks, d_out;
   cudaStream_t stream = nullptr;
 };
@@ -736,7 +736,7 @@ static int spectrum_cmb_impl(sbz_problem* pb, int cosmo, const sbz_bessel* jl, i
     // the perturbation kernel saves the sources at taus of *this* cosmology: A.taus + cosmo*ntau
   }
   SBZ_CUDA(cudaEventRecord(pb->ev[2], st));
-  // 2. interpolate to the fine k-grid; zero the last time (χ = 0, angular.jl:296)
+  // 2. interpolate to the fine k-grid, [k][τ][src] (the last time, χ = 0, zero: angular.jl:296)
   SBZ_CUDA(pb->c_Sf.ensure(sizeof(double) * (size_t)ntau * nf * std::max(1, nTE)));
   SBZ_CUDA(pb->c_Sp.ensure(sizeof(double) * (size_t)ntau * nf));
   SBZ_CUDA(pb->c_z.ensure(sizeof(double) * (size_t)nc * ntau * std::max(1, ns_all)));
@@ -748,8 +748,6 @@ static int spectrum_cmb_impl(sbz_problem* pb, int cosmo, const sbz_bessel* jl, i
   };
   if (nTE > 0 && kinterp(nTE, pb->c_src.as<int>(), pb->c_Sf.as<double>()) != 0) return fail(SBZ_ERR_CUDA, "k-interpolation");
   if (use[2] && kinterp(1, pb->c_src.as<int>() + nTE, pb->c_Sp.as<double>()) != 0) return fail(SBZ_ERR_CUDA, "k-interpolation");
-  if (nTE > 0) SBZ_CUDA(cudaMemsetAsync(pb->c_Sf.as<double>() + (size_t)(ntau - 1) * nf * nTE, 0, sizeof(double) * nf * nTE, st));
-  if (use[2]) SBZ_CUDA(cudaMemsetAsync(pb->c_Sp.as<double>() + (size_t)(ntau - 1) * nf, 0, sizeof(double) * nf, st));
   SBZ_CUDA(cudaEventRecord(pb->ev[3], st));
   // 3. line-of-sight integrals and Θ scaling; gather T/E/ψ into one interleaved Θ array
   SBZ_CUDA(pb->c_Th.ensure(sizeof(double) * (size_t)nf * nl * std::max(1, nTE)));
@@ -757,10 +755,10 @@ static int spectrum_cmb_impl(sbz_problem* pb, int cosmo, const sbz_bessel* jl, i
   // mixed precision: FP32 interpolation and chunk sums (the C_l target is ~1e-4); FP64 otherwise
   const int losp = pb->opts.los_precision >= 0 ? pb->opts.los_precision : pb->opts.precision;
   auto los = losp == SBZ_MIXED && nl <= 1024 ? sbz::los_f32_launch : sbz::los_launch;
-  if (nTE > 0 && los(jl->J, const_cast<sbz_bessel*>(jl)->d_ls.as<int>(), nTE, pb->c_Sf.as<double>(), pb->c_taus.as<double>(),
+  if (nTE > 0 && los(jl->J, const_cast<sbz_bessel*>(jl)->d_ls.as<int>(), nTE, pb->c_Sf.as<double>(), nTE, (long long)ntau * nTE, pb->c_taus.as<double>(),
                      pb->c_chi.as<double>(), pb->c_w.as<double>(), ntau, nf, pb->c_ks.as<double>(), nl, pb->c_Th.as<double>(), st) != 0)
     return fail(SBZ_ERR_CUDA, "LOS kernel");
-  if (use[2] && los(jl->J, const_cast<sbz_bessel*>(jl)->d_ls.as<int>(), 1, pb->c_Sp.as<double>(), pb->c_taus.as<double>(),
+  if (use[2] && los(jl->J, const_cast<sbz_bessel*>(jl)->d_ls.as<int>(), 1, pb->c_Sp.as<double>(), 1, ntau, pb->c_taus.as<double>(),
                     pb->c_chi.as<double>(), pb->c_w.as<double>(), ntau, nf, pb->c_ks.as<double>(), ilim, pb->c_Thp.as<double>(), st) != 0)
     return fail(SBZ_ERR_CUDA, "LOS kernel");
   if (nTE > 0 && sbz::theta_scale_launch(nf, nl, nTE, pb->c_ks.as<double>(), const_cast<sbz_bessel*>(jl)->d_ls.as<int>(),
@@ -815,8 +813,10 @@ int sbz_bessel_create(int nl, const int* ls, double xmax, double dx, int hermite
   if (c->d_ls.ensure(sizeof(int) * nl) != cudaSuccess) return bail("allocation");
   c->J.y = c->d_y.as<double>(); c->J.dy = hermite ? c->d_dy.as<double>() : nullptr; c->J.yf2 = c->d_yf2.as<float2>();
   cudaMemcpyAsync(c->d_ls.p, ls, sizeof(int) * nl, cudaMemcpyHostToDevice, c->stream);
-  if (sbz::bessel_build(c->J, c->d_ls.as<int>(), ls[nl - 1], c->stream) != 0) return bail("bessel kernel");
-  if (sbz::bessel_f32_build(c->J, c->stream) != 0) return bail("bessel kernel");
+  std::vector<double> cf(2 * (size_t)nl);
+  for (int i = 0; i < nl; ++i) { cf[2 * i] = ls[i] / (2.0 * ls[i] + 1); cf[2 * i + 1] = (ls[i] + 1) / (2.0 * ls[i] + 1); }
+  if (up(c->d_cf, cf.data(), cf.size(), c->stream) != cudaSuccess) return bail("allocation");
+  if (sbz::bessel_build(c->J, c->d_ls.as<int>(), c->d_cf.as<double>(), ls[nl - 1], c->stream) != 0) return bail("bessel kernel");
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return bail("bessel kernel");
   *out = c;
   return SBZ_OK;
@@ -825,7 +825,7 @@ int sbz_bessel_create(int nl, const int* ls, double xmax, double dx, int hermite
 void sbz_bessel_destroy(sbz_bessel* c) {
   if (!c) return;
   if (c->stream) cudaStreamSynchronize(c->stream);
-  for (DevBuf* b : {&c->d_y, &c->d_dy, &c->d_yf2, &c->d_ls, &c->d_S, &c->d_taus, &c->d_chi, &c->d_w, &c->d_ks, &c->d_out}) b->release();
+  for (DevBuf* b : {&c->d_y, &c->d_dy, &c->d_yf2, &c->d_ls, &c->d_cf, &c->d_S, &c->d_taus, &c->d_chi, &c->d_w, &c->d_ks, &c->d_out}) b->release();
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }
@@ -879,7 +879,7 @@ int sbz_los_integrate(const sbz_bessel* c, int nsrc, const double* S, int ntau, 
   SBZ_CUDA(cudaMemcpyAsync(cc->d_chi.p, chi.data(), sizeof(double) * ntau, cudaMemcpyHostToDevice, st));
   SBZ_CUDA(cudaMemcpyAsync(cc->d_w.p, w.data(), sizeof(double) * ntau, cudaMemcpyHostToDevice, st));
   SBZ_CUDA(cudaMemcpyAsync(cc->d_ks.p, ks, sizeof(double) * nk, cudaMemcpyHostToDevice, st));
-  if (sbz::los_launch(c->J, cc->d_ls.as<int>(), nsrc, cc->d_S.as<double>(), cc->d_taus.as<double>(), cc->d_chi.as<double>(),
+  if (sbz::los_launch(c->J, cc->d_ls.as<int>(), nsrc, cc->d_S.as<double>(), (long long)nk * nsrc, nsrc, cc->d_taus.as<double>(), cc->d_chi.as<double>(),
                       cc->d_w.as<double>(), ntau, nk, cc->d_ks.as<double>(), il_limber_of(c, l_limber), cc->d_out.as<double>(), st) != 0)
     return fail(SBZ_ERR_CUDA, "LOS kernel");
   SBZ_CUDA(cudaMemcpyAsync(out, cc->d_out.p, sizeof(double) * nout, cudaMemcpyDeviceToHost, st));
@@ -900,7 +900,7 @@ int sbz_los_integrate_device(const sbz_bessel* c, int nsrc, const double* S, int
   SBZ_CUDA(cc->d_w.ensure(sizeof(double) * ntau));
   SBZ_CUDA(cudaMemcpyAsync(cc->d_chi.p, chi.data(), sizeof(double) * ntau, cudaMemcpyHostToDevice, st));
   SBZ_CUDA(cudaMemcpyAsync(cc->d_w.p, w.data(), sizeof(double) * ntau, cudaMemcpyHostToDevice, st));
-  if (sbz::los_launch(c->J, cc->d_ls.as<int>(), nsrc, S, taus, cc->d_chi.as<double>(), cc->d_w.as<double>(), ntau, nk, ks,
+  if (sbz::los_launch(c->J, cc->d_ls.as<int>(), nsrc, S, (long long)nk * nsrc, nsrc, taus, cc->d_chi.as<double>(), cc->d_w.as<double>(), ntau, nk, ks,
                       il_limber_of(c, l_limber), out, st) != 0)
     return fail(SBZ_ERR_CUDA, "LOS kernel");
   return SBZ_OK;
@@ -908,39 +908,24 @@ int sbz_los_integrate_device(const sbz_bessel* c, int nsrc, const double* S, int
 
 int sbz_cl_integrate(int nk, const double* ks, const double* P0, int nl, const double* ThA, const double* ThB, double* Cl) {
   if (nk < 2 || nl < 1 || !ks || !P0 || !ThA || !ThB || !Cl) return fail(SBZ_ERR_ARG, "sbz_cl_integrate: bad arguments");
-  const int np = nk + 1;
-  std::vector<double> X(np), cprime(np, 0.0), invden(np, 0.0);
+  std::vector<double> X(nk + 1), wk, g(nk);
   X[0] = 0;
   for (int i = 0; i < nk; ++i) X[i + 1] = ks[i];
-  for (int i = 1; i < np; ++i) if (!(X[i] > X[i - 1])) return fail(SBZ_ERR_ARG, "ks must be positive and increasing");
-  for (int i = 1; i <= np - 2; ++i) {
-    const double h0 = X[i] - X[i - 1], h1 = X[i + 1] - X[i];
-    const double den = 2 * (h0 + h1) - h0 * (i > 1 ? cprime[i - 1] : 0.0);
-    invden[i] = 1.0 / den;
-    cprime[i] = h1 * invden[i];
-  }
-  // every buffer is released on every return path, the early error returns included
-  struct Owned : DevBuf {
+  for (int i = 1; i <= nk; ++i) if (!(X[i] > X[i - 1])) return fail(SBZ_ERR_ARG, "ks must be positive and increasing");
+  // the natural-spline integral of 2/π k² P0 Θ_A Θ_B as a weighted sum over k
+  spline_integral_weights(X, wk);
+  for (int i = 0; i < nk; ++i) g[i] = wk[i + 1] * (2.0 / M_PI) * ks[i] * ks[i] * P0[i];
+  struct Owned : DevBuf {  // released on every return path
     ~Owned() { release(); }
-  } d_ks, d_P0, d_A, d_B, d_c, d_i, d_z, d_Cl;
-  const size_t th = sizeof(double) * (size_t)nk * nl;
-  SBZ_CUDA(d_ks.ensure(sizeof(double) * nk));
-  SBZ_CUDA(d_P0.ensure(sizeof(double) * nk));
-  SBZ_CUDA(d_A.ensure(th));
-  SBZ_CUDA(d_B.ensure(th));
-  SBZ_CUDA(d_c.ensure(sizeof(double) * np));
-  SBZ_CUDA(d_i.ensure(sizeof(double) * np));
-  SBZ_CUDA(d_z.ensure(sizeof(double) * (size_t)np * nl));
-  SBZ_CUDA(d_Cl.ensure(sizeof(double) * nl));
-  SBZ_CUDA(cudaMemcpy(d_ks.p, ks, sizeof(double) * nk, cudaMemcpyHostToDevice));
-  SBZ_CUDA(cudaMemcpy(d_P0.p, P0, sizeof(double) * nk, cudaMemcpyHostToDevice));
-  SBZ_CUDA(cudaMemcpy(d_A.p, ThA, th, cudaMemcpyHostToDevice));
-  SBZ_CUDA(cudaMemcpy(d_B.p, ThB, th, cudaMemcpyHostToDevice));
-  SBZ_CUDA(cudaMemcpy(d_c.p, cprime.data(), sizeof(double) * np, cudaMemcpyHostToDevice));
-  SBZ_CUDA(cudaMemcpy(d_i.p, invden.data(), sizeof(double) * np, cudaMemcpyHostToDevice));
-  int r = sbz::cl_launch(nk, d_ks.as<double>(), d_P0.as<double>(), nl, d_A.as<double>(), d_B.as<double>(), d_c.as<double>(),
-                         d_i.as<double>(), d_z.as<double>(), d_Cl.as<double>(), 0);
-  if (r == 0) SBZ_CUDA(cudaMemcpy(Cl, d_Cl.p, sizeof(double) * nl, cudaMemcpyDeviceToHost));
+  } buf;
+  const size_t th = (size_t)nk * nl;
+  SBZ_CUDA(buf.ensure(sizeof(double) * (nk + 2 * th + nl)));
+  double *d_g = buf.as<double>(), *d_A = d_g + nk, *d_B = d_A + th, *d_Cl = d_B + th;
+  SBZ_CUDA(cudaMemcpy(d_g, g.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
+  SBZ_CUDA(cudaMemcpy(d_A, ThA, sizeof(double) * th, cudaMemcpyHostToDevice));
+  SBZ_CUDA(cudaMemcpy(d_B, ThB, sizeof(double) * th, cudaMemcpyHostToDevice));
+  const int r = sbz::cl_pair_launch(nk, d_g, nl, d_A, d_B, d_Cl, 0);
+  if (r == 0) SBZ_CUDA(cudaMemcpy(Cl, d_Cl, sizeof(double) * nl, cudaMemcpyDeviceToHost));
   return r == 0 ? SBZ_OK : fail(SBZ_ERR_CUDA, "C_l kernel");
 }
 

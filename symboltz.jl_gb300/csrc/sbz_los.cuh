@@ -13,18 +13,21 @@ struct BesselDev {
   int hermite;
 };
 
-int bessel_build(BesselDev& J, const int* d_ls, int Lmax, cudaStream_t st);
-int bessel_f32_build(const BesselDev& J, cudaStream_t st);
+// d_cf: l/(2l+1), (l+1)/(2l+1) per multipole; fills y, dy (Hermite) and the FP32 copy
+int bessel_build(BesselDev& J, const int* d_ls, const double* d_cf, int Lmax, cudaStream_t st);
+// Line of sight; sources at S[it * st_t + ik * st_k + s].
 // FP32 line of sight (interpolation and chunk sums in FP32, chunk totals in FP64); il_limber ≤ 1024
-int los_f32_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S, const double* d_taus, const double* d_chi,
+int los_f32_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S, long long st_t, long long st_k, const double* d_taus, const double* d_chi,
                    const double* d_w, int ntau, int nk, const double* d_ks, int il_limber, double* d_out, cudaStream_t st);
 // C_l[q*nl + il] = Σ_k g_k Θ_a(k,l) Θ_b(k,l) with g_k the spline-integral weights times 2/π k² P0
 int cl_dot_launch(int nk, const double* d_g, int nl, int ns, const double* d_Th, int npair, const int* d_pa, const int* d_pb,
                   double* d_Cl, cudaStream_t st);
 int bessel_eval(const BesselDev& J, int il, int n, const double* d_x, double* d_out, cudaStream_t st);
-int los_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S, const double* d_taus,
+int los_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S, long long st_t, long long st_k, const double* d_taus,
                const double* d_chi, const double* d_w, int ntau, int nk, const double* d_ks, int il_limber,
                double* d_out, cudaStream_t st);
+// C_l = Σ_k g_k A(k,l) B(k,l) for two [nk][nl] arrays
+int cl_pair_launch(int nk, const double* d_g, int nl, const double* d_A, const double* d_B, double* d_Cl, cudaStream_t st);
 int cl_launch(int nk, const double* d_ks, const double* d_P0, int nl, const double* d_ThA, const double* d_ThB,
               const double* d_cprime, const double* d_invden, double* d_zbuf, double* d_Cl, cudaStream_t st);
 
