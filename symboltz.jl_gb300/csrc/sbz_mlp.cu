@@ -27,14 +27,18 @@ bool get_encode() {
   return true;
 }
 
-// 2-D tensor map of a bf16 [rows][K] row-major matrix, box 64 (K) x box_rows, 128-byte swizzle
-bool tmap_rows_k(CUtensorMap* tm, const void* ptr, int rows, int K, int box_rows) {
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+// 2-D tensor map of a bf16 [rows][cols] row-major matrix (row stride ld elements), box box_cols x box_rows
+bool tmap(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_cols, int box_rows, CUtensorMapSwizzle sw) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t es[2] = {1, 1};
   return g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+                  sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// operand [rows][K], box 64 (K) x box_rows, 128-byte swizzle
+bool tmap_rows_k(CUtensorMap* tm, const void* ptr, int rows, int K, int box_rows) {
+  return tmap(tm, ptr, rows, K, K, BK, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 int num_sms() {
@@ -47,34 +51,52 @@ int num_sms() {
   return n;
 }
 
-template <int BN>
-int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
-  CUtensorMap ta, tb;
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// Activation epilogue through TMA: whole 64-column groups, 16-byte row strides and bases.
+bool tma_epilogue(const GemmArgs& g, int bn) {
+  if (g.epi == EPI_F32 || bn < 128 || g.n_valid != g.N || g.ldo % 8 || !aligned16(g.out_bf16)) return false;
+  if (g.epi == EPI_DACT && !aligned16(g.z_in)) return false;
+  if (g.epi == EPI_ACT && g.z_out && !aligned16(g.z_out)) return false;
+  return !g.out_t || (g.ldt % 8 == 0 && g.ldt >= g.M && aligned16(g.out_t));
+}
+
+template <int BN, bool TS>
+int launch_k(const GemmArgs& g, const void* A, const void* B, int splits, cudaStream_t st) {
+  CUtensorMap ta, tb, to, tz, tt;
   if (!tmap_rows_k(&ta, A, g.M, g.K, BM) || !tmap_rows_k(&tb, B, g.N, g.K, BN)) return SBZ_ERR_CUDA;
+  to = tz = tt = ta;
+  if (TS) {
+    const void* z = g.epi == EPI_DACT ? static_cast<const void*>(g.z_in) : g.z_out;
+    if (!tmap(&to, g.out_bf16, g.M, g.N, g.ldo, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return SBZ_ERR_CUDA;
+    if (z && !tmap(&tz, z, g.M, g.N, g.ldo, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return SBZ_ERR_CUDA;
+    if (g.out_t && !tmap(&tt, g.out_t, g.N, g.M, g.ldt, 32, 64, CU_TENSOR_MAP_SWIZZLE_NONE)) return SBZ_ERR_CUDA;
+  }
   const size_t smem = gemm_smem_bytes<BN>();
-  auto k = gemm_tn_kernel<BN>;
+  auto k = gemm_tn_kernel<BN, TS>;
   static bool attr_set = false;  // set once, outside any stream capture of a later call
   if (!attr_set) {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
     attr_set = true;
   }
+  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, to, tz, tt, g);
+  return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
+}
+
+template <int BN>
+int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   const int tiles = (g.N / BN) * (g.M / BM), KT = g.K / BK;
   // weight gradients have few output tiles and a long K (the batch): split K over about two CTAs
   // per SM, at least 4 K-steps each, and add the partial tiles atomically into a zeroed output
   int splits = 1;
   if (g.epi == EPI_F32 && tiles < 2 * num_sms()) splits = std::max(1, std::min(KT / 4, 2 * num_sms() / tiles));
-  if (splits > 1 && !g.accumulate) {
-    for (int r = 0; r < g.M; ++r) {  // rows of the output region (ldo may exceed N)
-      if (g.ldo == g.n_valid) {
-        if (cudaMemsetAsync(g.out_f32, 0, sizeof(float) * (size_t)g.M * g.ldo, st) != cudaSuccess) return SBZ_ERR_CUDA;
-        break;
-      }
-      if (cudaMemsetAsync(g.out_f32 + (size_t)r * g.ldo, 0, sizeof(float) * g.n_valid, st) != cudaSuccess) return SBZ_ERR_CUDA;
-    }
-  }
-  const dim3 grid(g.N / BN, g.M / BM, splits);
-  k<<<grid, kThreads, smem, st>>>(ta, tb, g);
-  return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
+  // one 2-D fill of the output region (its rows may be longer than n_valid)
+  if (splits > 1 && !g.accumulate &&
+      cudaMemset2DAsync(g.out_f32, sizeof(float) * (size_t)g.ldo, 0, sizeof(float) * (size_t)g.n_valid, (size_t)g.M, st) != cudaSuccess)
+    return SBZ_ERR_CUDA;
+  if constexpr (BN >= 128)
+    if (tma_epilogue(g, BN)) return launch_k<BN, true>(g, A, B, 1, st);
+  return launch_k<BN, false>(g, A, B, splits, st);
 }
 
 }  // namespace
