@@ -60,7 +60,9 @@ struct sbz_surrogate {
   float* Yf = nullptr;        // [batch][64] last-layer product (before bias)
   bf16 *dY = nullptr, *dYt = nullptr;
   float* T = nullptr;         // [batch][nout] targets of the step
-  double* loss = nullptr;
+  double* loss = nullptr;     // first entry of grads
+  unsigned char* grads = nullptr;  // loss and every layer's gW and gb: one memset per step
+  size_t grads_bytes = 0;
   unsigned* err = nullptr;
   float *dataX = nullptr, *dataY = nullptr;
   long long ndata = 0;
@@ -71,7 +73,7 @@ struct sbz_surrogate {
   float* dlr = nullptr;        // device learning rate
   void* segs = nullptr;        // device table of Adam segments
   int nseg = 0;
-  long long nparam_all = 0;    // padded parameter count over all segments
+  int nadam = 0;               // blocks of the Adam launch
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
 };
@@ -88,49 +90,62 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
   return z ^ (z >> 31);
 }
 
-// dstep (if not null) replaces step: the graph-captured training step reads the device counter.
-// X0t (if not null) receives the transposed copy [kPadIn][batch].
-__global__ void gather_batch(int batch, int nin, int nout, const float* __restrict__ dX, const float* __restrict__ dY, long long n,
-                             long long step, const long long* __restrict__ dstep, unsigned long long seed, long long offset, int random,
-                             bf16* __restrict__ X0, bf16* __restrict__ X0t, float* __restrict__ T) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= batch) return;
-  if (dstep) step = *dstep;
-  long long r;
-  if (random) r = (long long)(mix64(seed ^ mix64((unsigned long long)step * 0x100000001B3ull + (unsigned long long)i)) % (unsigned long long)n);
-  else r = offset + i;
-  const bool live = r < n;
-  bf16* x = X0 + (size_t)i * kPadIn;
-  for (int j = 0; j < kPadIn; ++j) {
-    const bf16 v = __float2bfloat16(live && j < nin ? dX[(size_t)r * nin + j] : 0.0f);
-    x[j] = v;
-    if (X0t) X0t[(size_t)j * batch + i] = v;
+// dstep (if not null): the step is *dstep + 1 (the graph-captured training step reads the device counter,
+// which loss_grad advances).  X0 rows are written whole (padding zero); X0t (if not null) receives the
+// transposed copy of the first nin columns (the others stay zero).  A warp assembles 32 rows: one hash per
+// lane, row pieces along the row, the transposed copy along the batch (one thread per row wrote 2-byte
+// pieces of 64 rows and columns: 47 µs for 65,536 rows).
+__global__ void __launch_bounds__(128) gather_batch(int batch, int nin, int nout, const float* __restrict__ dX, const float* __restrict__ dY,
+                                                    long long n, const long long* __restrict__ dstep, unsigned long long seed, int random,
+                                                    bf16* __restrict__ X0, bf16* __restrict__ X0t, float* __restrict__ T) {
+  __shared__ long long rows[4][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i0 = (blockIdx.x * 4 + warp) * 32;
+  if (i0 >= batch) return;  // batch is a multiple of 32
+  {
+    const int i = i0 + lane;
+    long long r = i;
+    if (random) {
+      const unsigned long long step = (unsigned long long)(dstep ? *dstep + 1 : 0);
+      r = (long long)(mix64(seed ^ mix64(step * 0x100000001B3ull + (unsigned long long)i)) % (unsigned long long)n);
+    }
+    rows[warp][lane] = r < n ? r : -1;
   }
+  __syncwarp();
+#pragma unroll 8
+  for (int q = 0; q < 32; ++q) {
+    const long long r = rows[warp][q];
+    const float* x = dX + (r < 0 ? 0 : r) * nin;
+    const int j = 2 * lane;
+    const float a = r >= 0 && j < nin ? x[j] : 0.0f, b = r >= 0 && j + 1 < nin ? x[j + 1] : 0.0f;
+    reinterpret_cast<__nv_bfloat162*>(X0 + (size_t)(i0 + q) * kPadIn)[lane] = __floats2bfloat162_rn(a, b);
+  }
+  const long long r = rows[warp][lane];
+  if (X0t)
+    for (int j = 0; j < nin; ++j) X0t[(size_t)j * batch + i0 + lane] = __float2bfloat16(r >= 0 ? dX[r * nin + j] : 0.0f);
   if (T)
-    for (int j = 0; j < nout; ++j) T[(size_t)i * nout + j] = live ? dY[(size_t)r * nout + j] : 0.0f;
-}
-
-__global__ void begin_step(long long* step, double* loss) {
-  ++*step;
-  *loss = 0.0;
+    for (int e = lane; e < 32 * nout; e += 32) {
+      const int q = e / nout;
+      const long long rq = rows[warp][q];
+      T[(size_t)i0 * nout + e] = rq >= 0 ? dY[rq * nout + (e - q * nout)] : 0.0f;
+    }
 }
 
 __global__ void set_value(float* dst, float v) { *dst = v; }
 
-// loss and output gradient: y = Yf + b (FP32), r = y - t, dY = 2 r / (batch · nout) (BF16, padding 0);
-// also dYᵀ [kPadOut][batch] and the bias gradient gb[j] += Σ_rows dY[.][j] (as rounded), when not null.
-// 256 threads per block.
+// loss and output gradient: y = Yf + b (FP32), r = y - t, dY = 2 r / (batch · nout) (BF16; padding columns
+// stay zero), dYᵀ [kPadOut][batch] and the bias gradient gb[j] += Σ_rows dY[.][j] (as rounded).
+// 256 threads per block.  Advances the device step counter (if not null; nothing else here reads it).
 constexpr int kLossThreads = 256;
 __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, const float* __restrict__ Yf, const float* __restrict__ b,
                                                            const float* __restrict__ T, bf16* __restrict__ dY, bf16* __restrict__ dYt,
-                                                           float* __restrict__ gb, double* __restrict__ loss) {
+                                                           float* __restrict__ gb, double* __restrict__ loss, long long* __restrict__ dstep) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   __shared__ float cs[kLossThreads / 32][kPadOut];
   double l = 0;
   const float sc = 2.0f / ((float)batch * nout);
-  for (int j = 0; j < kPadOut; ++j) {
+  for (int j = 0; j < nout; ++j) {
     float g = 0.0f;
-    if (i < batch && j < nout) {
+    if (i < batch) {
       const float r = Yf[(size_t)i * kPadOut + j] + b[j] - T[(size_t)i * nout + j];
       l += (double)r * r;
       g = sc * r;
@@ -138,13 +153,11 @@ __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, c
     const bf16 gh = __float2bfloat16(g);
     if (i < batch) {
       dY[(size_t)i * kPadOut + j] = gh;
-      if (dYt) dYt[(size_t)j * batch + i] = gh;
+      dYt[(size_t)j * batch + i] = gh;
     }
-    if (gb && j < nout) {
-      float w = __bfloat162float(gh);
-      for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
-      if ((threadIdx.x & 31) == 0) cs[threadIdx.x >> 5][j] = w;
-    }
+    float w = __bfloat162float(gh);
+    for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+    if ((threadIdx.x & 31) == 0) cs[threadIdx.x >> 5][j] = w;
   }
   __shared__ double red[kLossThreads / 32];
   for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
@@ -154,42 +167,68 @@ __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, c
     double s = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
     atomicAdd(loss, s / ((double)batch * nout));
+    if (dstep && blockIdx.x == 0) ++*dstep;
   }
-  if (gb && threadIdx.x < nout) {
+  if (threadIdx.x < nout) {
     float s = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += cs[w][threadIdx.x];
     atomicAdd(gb + threadIdx.x, s);
   }
 }
 
-// Adam over every parameter in one launch.  A segment is one layer's weights (with BF16 copies
-// [nrow][kin] and [kin][nrow]; its gradient possibly transposed) or biases; `start` is its first
-// index in the concatenation.  The bias corrections use the device step counter.
+// Adam over every parameter in one launch, one 32 x 32 tile of a layer's weights (with BF16 copies
+// [nrow][kin] and [kin][nrow], the second written through shared memory along its rows; the gradient possibly
+// transposed) or 1,024 biases per block.  `start` is the segment's first block.  The bias corrections use
+// the device step counter.
 struct AdamSeg {
   float *p, *m, *v;
   const float* g;
   bf16 *ph, *pt;
-  long long start;
-  int n, gT, nrow, kin;
+  int start, n, gT, nrow, kin;
 };
 
-__global__ void adam_all(const AdamSeg* __restrict__ segs, int nseg, long long total, const long long* __restrict__ step,
-                         const float* __restrict__ lr, float b1, float b2, float eps) {
+__global__ void __launch_bounds__(256) adam_all(const AdamSeg* __restrict__ segs, int nseg, const long long* __restrict__ step,
+                                                const float* __restrict__ lr, float b1, float b2, float eps) {
+  __shared__ float tile[32][33];
+  int q = 0;
+  while (q + 1 < nseg && segs[q + 1].start <= (int)blockIdx.x) ++q;
+  const AdamSeg S = segs[q];
+  const int blk = blockIdx.x - S.start, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const float t = (float)*step, rate = *lr;
   const float c1 = 1.0f / (1.0f - exp2f(t * log2f(b1))), c2 = 1.0f / (1.0f - exp2f(t * log2f(b2)));
-  int q = 0;  // a thread's indices increase, so its segment index only moves forward
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-    while (q + 1 < nseg && segs[q + 1].start <= e) ++q;
-    const AdamSeg& S = segs[q];
-    const int i = (int)(e - S.start);
-    int r = 0, k = i;
-    if (S.ph) { r = i / S.kin; k = i - r * S.kin; }
-    const float gi = (S.ph && S.gT) ? S.g[(size_t)k * S.nrow + r] : S.g[i];
+  auto update = [&](size_t i, float gi) {
     const float mi = b1 * S.m[i] + (1 - b1) * gi, vi = b2 * S.v[i] + (1 - b2) * gi * gi;
     S.m[i] = mi; S.v[i] = vi;
     const float pi = S.p[i] - rate * (mi * c1) / (sqrtf(vi * c2) + eps);
     S.p[i] = pi;
-    if (S.ph) { S.ph[i] = __float2bfloat16(pi); S.pt[(size_t)k * S.nrow + r] = __float2bfloat16(pi); }
+    return pi;
+  };
+  if (!S.ph) {
+    for (int i = blk * 1024 + threadIdx.x; i < min(S.n, (blk + 1) * 1024); i += 256) update(i, S.g[i]);
+    return;
+  }
+  const int kt = S.kin / 32, r0 = blk / kt * 32, k0 = blk % kt * 32;
+  if (S.gT) {
+#pragma unroll
+    for (int y = 0; y < 4; ++y) tile[tx][ty + 8 * y] = S.g[(size_t)(k0 + ty + 8 * y) * S.nrow + r0 + tx];  // [r][k]
+    __syncthreads();
+  }
+  float p[4];
+#pragma unroll
+  for (int y = 0; y < 4; ++y) {
+    const int r = ty + 8 * y;
+    const size_t i = (size_t)(r0 + r) * S.kin + k0 + tx;
+    p[y] = update(i, S.gT ? tile[r][tx] : S.g[i]);
+    S.ph[i] = __float2bfloat16(p[y]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int y = 0; y < 4; ++y) tile[ty + 8 * y][tx] = p[y];
+  __syncthreads();
+#pragma unroll
+  for (int y = 0; y < 4; ++y) {
+    const int k = ty + 8 * y;
+    S.pt[(size_t)(k0 + k) * S.nrow + r0 + tx] = __float2bfloat16(tile[tx][k]);
   }
 }
 
@@ -226,12 +265,11 @@ unsigned long long splitmix(unsigned long long& s) {
 
 void free_all(sbz_surrogate* s) {
   for (auto& l : s->L)
-    for (void* p : {(void*)l.W, (void*)l.b, (void*)l.mW, (void*)l.vW, (void*)l.mb, (void*)l.vb, (void*)l.gW, (void*)l.gb, (void*)l.Wh,
-                    (void*)l.Wt})
+    for (void* p : {(void*)l.W, (void*)l.b, (void*)l.mW, (void*)l.vW, (void*)l.mb, (void*)l.vb, (void*)l.Wh, (void*)l.Wt})
       if (p) cudaFree(p);
   for (auto* v : {&s->X, &s->Z, &s->Xt, &s->dZ, &s->dZt})
     for (bf16* p : *v) if (p) cudaFree(p);
-  for (void* p : {(void*)s->Yf, (void*)s->dY, (void*)s->dYt, (void*)s->T, (void*)s->loss, (void*)s->err, (void*)s->dataX, (void*)s->dataY,
+  for (void* p : {(void*)s->Yf, (void*)s->dY, (void*)s->dYt, (void*)s->T, (void*)s->grads, (void*)s->err, (void*)s->dataX, (void*)s->dataY,
                   (void*)s->dstep, (void*)s->dlr, s->segs})
     if (p) cudaFree(p);
   if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
@@ -260,28 +298,29 @@ int gemm(sbz_surrogate* s, int M, int N, int K, const bf16* A, const bf16* B, in
 }
 
 // forward pass of `rows` (multiple of 128, ≤ batch) rows already in X[0]; result in Yf.  With
-// `train`, the transposed activations X_lᵀ (row stride `rows`) are written for the backward pass.
+// `train`, the pre-activations and the transposed activations X_lᵀ (row stride `rows`) are written for the
+// backward pass.
 int forward(sbz_surrogate* s, int rows, bool train) {
   using namespace sbz::mlp;
   const int nl = (int)s->L.size();
   for (int l = 0; l < nl - 1; ++l) {
     const Layer& y = s->L[l];
-    int r = gemm(s, rows, y.nrow, y.kin, s->X[l], y.Wh, EPI_ACT, ACT_SILU, y.b, s->X[l + 1], y.nrow, y.nrow, 0, s->Z[l + 1], nullptr,
-                 train ? s->Xt[l + 1] : nullptr);
+    int r = gemm(s, rows, y.nrow, y.kin, s->X[l], y.Wh, EPI_ACT, ACT_SILU, y.b, s->X[l + 1], y.nrow, y.nrow, 0,
+                 train ? s->Z[l + 1] : nullptr, nullptr, train ? s->Xt[l + 1] : nullptr);
     if (r) return r;
   }
   const Layer& o = s->L[nl - 1];
-  return gemm(s, rows, o.nrow, o.kin, s->X[nl - 1], o.Wh, EPI_F32, ACT_NONE, nullptr, s->Yf, kPadOut, kPadOut, 0, nullptr, nullptr);
+  return gemm(s, rows, o.nrow, o.kin, s->X[nl - 1], o.Wh, EPI_F32, ACT_NONE, nullptr, s->Yf, kPadOut, s->nout, 0, nullptr, nullptr);
 }
 
 // backward pass after forward(train) + loss_grad (dY, dYᵀ and the output layer's gb set): weight
-// gradients into gW, bias gradients accumulated into gb by the EPI_DACT epilogues
+// gradients added into gW, bias gradients into gb by the EPI_DACT epilogues (both zeroed before)
 int backward(sbz_surrogate* s) {
   using namespace sbz::mlp;
   const int B = s->batch, nl = (int)s->L.size();
   // output layer: dW_Lᵀ = X_{L-1}ᵀ dY ([kin][64]); dZ_{L-1} = (dY W_L) ⊙ SiLU'(Z_{L-1})
   Layer& o = s->L[nl - 1];
-  int r = gemm(s, o.kin, kPadOut, B, s->Xt[nl - 1], s->dYt, EPI_F32, ACT_NONE, nullptr, o.gW, kPadOut, kPadOut, 0, nullptr, nullptr);
+  int r = gemm(s, o.kin, kPadOut, B, s->Xt[nl - 1], s->dYt, EPI_F32, ACT_NONE, nullptr, o.gW, kPadOut, kPadOut, 1, nullptr, nullptr);
   if (r) return r;
   r = gemm(s, B, o.kin, kPadOut, s->dY, o.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[nl - 1], o.kin, o.kin, 0, nullptr, s->Z[nl - 1],
            s->dZt[nl - 1], s->L[nl - 2].gb);
@@ -289,7 +328,7 @@ int backward(sbz_surrogate* s) {
   // hidden layers l = nl-2 .. 0: input X[l], output gradient dZ[l+1]
   for (int l = nl - 2; l >= 0; --l) {
     Layer& y = s->L[l];
-    r = gemm(s, y.nrow, y.kin, B, s->dZt[l + 1], s->Xt[l], EPI_F32, ACT_NONE, nullptr, y.gW, y.kin, y.kin, 0, nullptr, nullptr);
+    r = gemm(s, y.nrow, y.kin, B, s->dZt[l + 1], s->Xt[l], EPI_F32, ACT_NONE, nullptr, y.gW, y.kin, y.kin, 1, nullptr, nullptr);
     if (r) return r;
     if (l > 0) {
       r = gemm(s, B, y.kin, y.nrow, s->dZ[l + 1], y.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[l], y.kin, y.kin, 0, nullptr, s->Z[l], s->dZt[l],
@@ -300,26 +339,24 @@ int backward(sbz_surrogate* s) {
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : F(SBZ_ERR_CUDA, "surrogate: backward");
 }
 
-// forward + loss + backward of the `rows` rows in X[0] (and X[0]ᵀ) with targets T
-int forward_backward(sbz_surrogate* s, int rows) {
+// forward + loss + backward of the `rows` rows in X[0] (and X[0]ᵀ) with targets T; advances dstep (if given)
+int forward_backward(sbz_surrogate* s, int rows, long long* dstep) {
+  SCU(cudaMemsetAsync(s->grads, 0, s->grads_bytes, s->stream));
   int r = forward(s, rows, true);
   if (r) return r;
-  for (auto& l : s->L) SCU(cudaMemsetAsync(l.gb, 0, sizeof(float) * l.nrow, s->stream));
   loss_grad<<<(rows + kLossThreads - 1) / kLossThreads, kLossThreads, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, s->T, s->dY, s->dYt,
-                                                                                  s->L.back().gb, s->loss);
+                                                                                  s->L.back().gb, s->loss, dstep);
   return backward(s);
 }
 
 // one training step on the stream (captured into the step graph)
 int train_step(sbz_surrogate* s) {
   const int B = s->batch;
-  begin_step<<<1, 1, 0, s->stream>>>(s->dstep, s->loss);
-  gather_batch<<<(B + 127) / 128, 128, 0, s->stream>>>(B, s->nin, s->nout, s->dataX, s->dataY, s->ndata, 0, s->dstep, s->seed, 0, 1, s->X[0],
-                                                      s->Xt[0], s->T);
-  int r = forward_backward(s, B);
+  gather_batch<<<(B + 127) / 128, 128, 0, s->stream>>>(B, s->nin, s->nout, s->dataX, s->dataY, s->ndata, s->dstep, s->seed, 1, s->X[0], s->Xt[0],
+                                                      s->T);
+  int r = forward_backward(s, B, s->dstep);
   if (r) return r;
-  adam_all<<<2 * 152, 256, 0, s->stream>>>(static_cast<const AdamSeg*>(s->segs), s->nseg, s->nparam_all, s->dstep, s->dlr, 0.9f, 0.999f,
-                                           1e-8f);
+  adam_all<<<s->nadam, 256, 0, s->stream>>>(static_cast<const AdamSeg*>(s->segs), s->nseg, s->dstep, s->dlr, 0.9f, 0.999f, 1e-8f);
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : F(SBZ_ERR_CUDA, "surrogate: training step");
 }
 
@@ -361,8 +398,8 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
     y.nrow = l == nl - 1 ? kPadOut : width;
     y.gT = l == nl - 1;
     const size_t nw = (size_t)y.nrow * y.kin;
-    if (dalloc(&y.W, nw) || dalloc(&y.mW, nw) || dalloc(&y.vW, nw) || dalloc(&y.gW, nw) || dalloc(&y.b, y.nrow) || dalloc(&y.mb, y.nrow) ||
-        dalloc(&y.vb, y.nrow) || dalloc(&y.gb, y.nrow) || dalloc(&y.Wh, nw) || dalloc(&y.Wt, nw))
+    if (dalloc(&y.W, nw) || dalloc(&y.mW, nw) || dalloc(&y.vW, nw) || dalloc(&y.b, y.nrow) || dalloc(&y.mb, y.nrow) ||
+        dalloc(&y.vb, y.nrow) || dalloc(&y.Wh, nw) || dalloc(&y.Wt, nw))
       return bail("surrogate: weight allocation");
     // Glorot-uniform weights on the logical block, zero padding and biases
     std::vector<float> w(nw, 0.0f);
@@ -371,8 +408,22 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
       for (int k = 0; k < y.nin; ++k) w[(size_t)r * y.kin + k] = a * (2.0f * (float)((splitmix(rs) >> 11) * 0x1.0p-53) - 1.0f);
     cudaMemcpy(y.W, w.data(), sizeof(float) * nw, cudaMemcpyHostToDevice);
     cudaMemset(y.b, 0, sizeof(float) * y.nrow);
-    for (float* p : {y.mW, y.vW, y.gW}) cudaMemset(p, 0, sizeof(float) * nw);
-    for (float* p : {y.mb, y.vb, y.gb}) cudaMemset(p, 0, sizeof(float) * y.nrow);
+    for (float* p : {y.mW, y.vW}) cudaMemset(p, 0, sizeof(float) * nw);
+    for (float* p : {y.mb, y.vb}) cudaMemset(p, 0, sizeof(float) * y.nrow);
+  }
+  {
+    size_t off = 256;  // the loss, then gW and gb per layer on 256-byte boundaries
+    auto take = [&](size_t n) { const size_t o = off; off += (sizeof(float) * n + 255) & ~size_t(255); return o; };
+    std::vector<size_t> ow, ob;
+    for (auto& y : s->L) { ow.push_back(take((size_t)y.nrow * y.kin)); ob.push_back(take(y.nrow)); }
+    if (dalloc(&s->grads, off)) return bail("surrogate: gradient allocation");
+    s->grads_bytes = off;
+    cudaMemset(s->grads, 0, off);
+    s->loss = reinterpret_cast<double*>(s->grads);
+    for (int l = 0; l < nl; ++l) {
+      s->L[l].gW = reinterpret_cast<float*>(s->grads + ow[l]);
+      s->L[l].gb = reinterpret_cast<float*>(s->grads + ob[l]);
+    }
   }
   s->X.assign(nl, nullptr); s->Z.assign(nl, nullptr); s->Xt.assign(nl, nullptr); s->dZ.assign(nl, nullptr); s->dZt.assign(nl, nullptr);
   for (int l = 0; l < nl; ++l) {
@@ -382,21 +433,24 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
       return bail("surrogate: activation allocation");
   }
   if (dalloc(&s->Yf, (size_t)batch * kPadOut) || dalloc(&s->dY, (size_t)batch * kPadOut) || dalloc(&s->dYt, (size_t)batch * kPadOut) ||
-      dalloc(&s->T, (size_t)batch * nout) || dalloc(&s->loss, 1) || dalloc(&s->err, 1))
+      dalloc(&s->T, (size_t)batch * nout) || dalloc(&s->err, 1))
     return bail("surrogate: buffer allocation");
   cudaMemset(s->err, 0, sizeof(unsigned));
+  // padding columns and rows that no kernel writes
+  cudaMemset(s->Xt[0], 0, sizeof(bf16) * (size_t)batch * kPadIn);
+  cudaMemset(s->dY, 0, sizeof(bf16) * (size_t)batch * kPadOut);
+  cudaMemset(s->dYt, 0, sizeof(bf16) * (size_t)batch * kPadOut);
   {
     std::vector<AdamSeg> segs;
-    long long start = 0;
+    int start = 0;
     for (auto& l : s->L) {
-      const int n = l.nrow * l.kin;
-      segs.push_back(AdamSeg{l.W, l.mW, l.vW, l.gW, l.Wh, l.Wt, start, n, l.gT ? 1 : 0, l.nrow, l.kin});
-      start += n;
+      segs.push_back(AdamSeg{l.W, l.mW, l.vW, l.gW, l.Wh, l.Wt, start, l.nrow * l.kin, l.gT ? 1 : 0, l.nrow, l.kin});
+      start += l.nrow / 32 * (l.kin / 32);
       segs.push_back(AdamSeg{l.b, l.mb, l.vb, l.gb, nullptr, nullptr, start, l.nrow, 0, l.nrow, 1});
-      start += l.nrow;
+      start += (l.nrow + 1023) / 1024;
     }
     s->nseg = (int)segs.size();
-    s->nparam_all = start;
+    s->nadam = start;
     if (dalloc(&s->dstep, 1) || dalloc(&s->dlr, 1) || cudaMalloc(&s->segs, sizeof(AdamSeg) * segs.size()) != cudaSuccess)
       return bail("surrogate: buffer allocation");
     cudaMemcpy(s->segs, segs.data(), sizeof(AdamSeg) * segs.size(), cudaMemcpyHostToDevice);
@@ -503,9 +557,8 @@ int sbz_surrogate_gradients(sbz_surrogate* s, int n, const float* X, const float
   SCU(dalloc(&dy, (size_t)n * s->nout));
   SCU(cudaMemcpy(dx, X, sizeof(float) * n * s->nin, cudaMemcpyHostToDevice));
   SCU(cudaMemcpy(dy, Y, sizeof(float) * n * s->nout, cudaMemcpyHostToDevice));
-  gather_batch<<<(n + 127) / 128, 128, 0, s->stream>>>(n, s->nin, s->nout, dx, dy, n, 0, nullptr, 0, 0, 0, s->X[0], s->Xt[0], s->T);
-  cudaMemsetAsync(s->loss, 0, sizeof(double), s->stream);
-  int r = forward_backward(s, n);
+  gather_batch<<<(n + 127) / 128, 128, 0, s->stream>>>(n, s->nin, s->nout, dx, dy, n, nullptr, 0, 0, s->X[0], s->Xt[0], s->T);
+  int r = forward_backward(s, n, nullptr);
   s->batch = keepB;
   cudaFree(dx); cudaFree(dy);
   if (r) return r;
@@ -540,7 +593,7 @@ int sbz_surrogate_infer(sbz_surrogate* s, long long n, const float* X, float* Y)
     for (long long b0 = 0; b0 < cn && !r; b0 += B) {
       const int rows = (int)std::min<long long>(B, cn - b0);
       const int prow = (rows + 127) / 128 * 128;
-      gather_batch<<<(prow + 127) / 128, 128, 0, s->stream>>>(prow, s->nin, s->nout, dx + b0 * s->nin, nullptr, rows, 0, nullptr, 0, 0, 0, s->X[0],
+      gather_batch<<<(prow + 127) / 128, 128, 0, s->stream>>>(prow, s->nin, s->nout, dx + b0 * s->nin, nullptr, rows, nullptr, 0, 0, s->X[0],
                                                               nullptr, nullptr);
       if ((r = forward(s, prow, false))) break;
       add_bias_out<<<(rows * s->nout + 255) / 256, 256, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, dyo);
