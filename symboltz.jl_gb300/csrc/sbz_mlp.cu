@@ -27,18 +27,19 @@ bool get_encode() {
   return true;
 }
 
-// 2-D tensor map of a bf16 [rows][cols] row-major matrix (row stride ld elements), box box_cols x box_rows
-bool tmap(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_cols, int box_rows, CUtensorMapSwizzle sw) {
+// 2-D tensor map of a bf16 [rows][cols] row-major matrix (row stride ld elements), box box_cols x box_rows,
+// 128-byte swizzle
+bool tmap(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_cols, int box_rows) {
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
   const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t es[2] = {1, 1};
   return g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-// operand [rows][K], box 64 (K) x box_rows, 128-byte swizzle
-bool tmap_rows_k(CUtensorMap* tm, const void* ptr, int rows, int K, int box_rows) {
-  return tmap(tm, ptr, rows, K, K, BK, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+// operand [rows][cols] without padding, box 64 x box_rows
+bool tmap_operand(CUtensorMap* tm, const void* ptr, int rows, int cols, int box_rows) {
+  return tmap(tm, ptr, rows, cols, cols, BK, box_rows);
 }
 
 int num_sms() {
@@ -57,20 +58,22 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 bool tma_epilogue(const GemmArgs& g, int bn) {
   if (g.epi == EPI_F32 || bn < 128 || g.n_valid != g.N || g.ldo % 8 || !aligned16(g.out_bf16)) return false;
   if (g.epi == EPI_DACT && !aligned16(g.z_in)) return false;
-  if (g.epi == EPI_ACT && g.z_out && !aligned16(g.z_out)) return false;
-  return !g.out_t || (g.ldt % 8 == 0 && g.ldt >= g.M && aligned16(g.out_t));
+  return g.epi != EPI_ACT || !g.z_out || aligned16(g.z_out);
 }
 
 template <int BN, bool TS>
 int launch_k(const GemmArgs& g, const void* A, const void* B, int splits, cudaStream_t st) {
-  CUtensorMap ta, tb, to, tz, tt;
-  if (!tmap_rows_k(&ta, A, g.M, g.K, BM) || !tmap_rows_k(&tb, B, g.N, g.K, BN)) return SBZ_ERR_CUDA;
-  to = tz = tt = ta;
+  CUtensorMap ta, tb, to, tz;
+  if (g.rows_k) {  // [K][M], [K][N] in pieces of 64 x 64
+    if (!tmap_operand(&ta, A, g.K, g.M, BK) || !tmap_operand(&tb, B, g.K, g.N, BK)) return SBZ_ERR_CUDA;
+  } else if (!tmap_operand(&ta, A, g.M, g.K, BM) || !tmap_operand(&tb, B, g.N, g.K, BN)) {
+    return SBZ_ERR_CUDA;
+  }
+  to = tz = ta;
   if (TS) {
     const void* z = g.epi == EPI_DACT ? static_cast<const void*>(g.z_in) : g.z_out;
-    if (!tmap(&to, g.out_bf16, g.M, g.N, g.ldo, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return SBZ_ERR_CUDA;
-    if (z && !tmap(&tz, z, g.M, g.N, g.ldo, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return SBZ_ERR_CUDA;
-    if (g.out_t && !tmap(&tt, g.out_t, g.N, g.M, g.ldt, 32, 64, CU_TENSOR_MAP_SWIZZLE_NONE)) return SBZ_ERR_CUDA;
+    if (!tmap(&to, g.out_bf16, g.M, g.N, g.ldo, 64, 32)) return SBZ_ERR_CUDA;
+    if (z && !tmap(&tz, z, g.M, g.N, g.ldo, 64, 32)) return SBZ_ERR_CUDA;
   }
   const size_t smem = gemm_smem_bytes<BN>();
   auto k = gemm_tn_kernel<BN, TS>;
@@ -79,7 +82,7 @@ int launch_k(const GemmArgs& g, const void* A, const void* B, int splits, cudaSt
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
     attr_set = true;
   }
-  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, to, tz, tt, g);
+  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, to, tz, g);
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
 }
 
@@ -96,16 +99,17 @@ int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
     return SBZ_ERR_CUDA;
   if constexpr (BN >= 128)
     if (tma_epilogue(g, BN)) return launch_k<BN, true>(g, A, B, 1, st);
+  if (g.colsum) return SBZ_ERR_ARG;  // only the shared-memory epilogue forms column sums
   return launch_k<BN, false>(g, A, B, splits, st);
 }
 
 }  // namespace
 
-// D = A Bᵀ with the fused epilogue of g; M % 128 == 0, N % 64 == 0, K % 64 == 0, A and B 16-byte
+// D = A Bᵀ (AᵀB of [K][M] and [K][N] operands with rows_k) with the fused epilogue of g; M % 128 == 0, N % 64 == 0, K % 64 == 0, A and B 16-byte
 // aligned (TMA).  The widest tile that divides N is used.
 int gemm(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   if (g.M <= 0 || g.M % BM || g.N <= 0 || g.N % 64 || g.K <= 0 || g.K % BK) return SBZ_ERR_ARG;
-  if (((uintptr_t)A | (uintptr_t)B) & 15) return SBZ_ERR_ARG;
+  if (((uintptr_t)A | (uintptr_t)B) & 15 || (g.rows_k && g.epi != EPI_F32)) return SBZ_ERR_ARG;
   if (!get_encode()) return SBZ_ERR_CUDA;
   if (g.N % 256 == 0) return launch<256>(g, A, B, st);
   if (g.N % 128 == 0) return launch<128>(g, A, B, st);

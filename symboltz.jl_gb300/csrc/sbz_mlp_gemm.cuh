@@ -1,6 +1,7 @@
 // BF16 tensor-core GEMM for the source surrogate's dense layers (sm_103a: TMA + tcgen05 + TMEM).
 //
 //   D[M x N] = A[M x K] · B[N x K]ᵀ   (A, B bf16 row-major with K contiguous, FP32 accumulation)
+//   D[M x N] = A[K x M]ᵀ · B[K x N]   (the same with rows along K: the weight gradients, whose K is the batch)
 //
 // One CTA computes a 128 x BN tile; two CTAs share an SM (≈ 100 KB of shared memory and at most
 // 128 registers per thread each), so one CTA's epilogue overlaps the other's loads.  Warp 0 lane 0
@@ -13,10 +14,8 @@
 //   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add with 16-byte atomics)
 //   EPI_ACT   z = D + bias; out = bf16(act(z)); optional z_out = bf16(z)    forward layers
 //   EPI_DACT  out = bf16(D · act'(z_in))                                   backward layers
-// EPI_ACT / EPI_DACT can also store the output transposed (out_t[col][row], the operand layout of
-// the weight-gradient GEMMs) and, for EPI_DACT, add its column sums into colsum (the bias gradient).
-// Whole 64-column groups go through shared memory and TMA stores (epilogue_tma), other shapes are
-// stored from registers.
+// Whole 64-column groups go through shared memory and TMA stores (epilogue_tma), where EPI_DACT can also
+// add the output's column sums into colsum (the bias gradient); other shapes are stored from registers.
 // Every mbarrier wait is bounded: a wait that runs out sets *err and the CTA skips ahead to its
 // TMEM release, so a fault in the pipeline cannot hang the GPU.
 #pragma once
@@ -46,9 +45,8 @@ struct GemmArgs {
   int accumulate;               // EPI_F32: add to the output
   __nv_bfloat16* z_out;         // EPI_ACT: pre-activation (ldo stride), may be null
   const __nv_bfloat16* z_in;    // EPI_DACT: pre-activation of this layer (ldo stride)
-  __nv_bfloat16* out_t;         // EPI_ACT / EPI_DACT: transposed output, (col, row) at col * ldt + row; may be null
-  int ldt;                      // its row stride (even)
-  float* colsum;                // EPI_DACT: colsum[col] += Σ_rows out (as stored, bf16-rounded); may be null
+  int rows_k;                   // operands are [K][M] and [K][N] (EPI_F32)
+  float* colsum;                // EPI_DACT: colsum[col] += Σ_rows out (as stored, bf16-rounded; 8-byte aligned); may be null
   unsigned* err;                // set to 1 by a CTA whose pipeline wait ran out
 };
 
@@ -100,58 +98,47 @@ __device__ __forceinline__ uint64_t desc_sw128(const void* p) {
   return d;
 }
 
+// the same for a tile with rows along K ([64 K-rows][64 columns] pieces of 8 KB as TMA writes them): 128-byte rows
+// of 64 columns, 8-row groups 1024 B apart, the next 64 columns one piece further
+__device__ __forceinline__ uint64_t desc_sw128_rows_k(const void* p) {
+  uint64_t d = (uint64_t)((smem_u32(p) & 0x3FFFFu) >> 4);
+  d |= (uint64_t)(8192 >> 4) << 16;  // leading-dimension offset: next 64 columns
+  d |= (uint64_t)(1024 >> 4) << 32;  // stride-dimension offset: next 8 K-rows
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+
 template <int BN>
-__device__ __forceinline__ uint32_t idesc_bf16() {
-  return (1u << 4)                    // D: FP32
+__device__ __forceinline__ uint32_t idesc_bf16(bool rows_k) {
+  return (rows_k ? (1u << 15) | (1u << 16) : 0u)  // A, B: M (N) contiguous
+         | (1u << 4)                  // D: FP32
          | (1u << 7) | (1u << 10)     // A, B: BF16
          | ((uint32_t)(BN >> 3) << 17) // N
          | ((uint32_t)(BM >> 4) << 24); // M
 }
 
-// SiLU and its derivative with the fast exponential and division (the results are rounded to
-// bf16; for z < -87 e^{-z} overflows to inf and both give the correct limit 0)
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+// SiLU and its derivative with the hardware's exponential and reciprocal.  Their flush-to-zero forms: e^{-z} below
+// 2^-126 vanishes beside 1, and above 2^126 the reciprocal is 0 as it is from __fdividef (the limits 0 and 1 are
+// right); the plain forms' range scaling was about a quarter of the epilogue's instructions.
+__device__ __forceinline__ float sigmoid_fast(float z) {
+  float e, s;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.0f + e));
+  return s;
+}
+__device__ __forceinline__ float silu(float z) { return z * sigmoid_fast(z); }
 __device__ __forceinline__ float dsilu(float z) {
-  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+  const float s = sigmoid_fast(z);
   return s * (1.0f + z * (1.0f - s));
 }
 
-// lane l ends with the sum over the warp's 32 lanes of a[l] (a transposing butterfly, 31 shuffles)
-__device__ __forceinline__ float warp_column_sum(float (&a)[32], int lane) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) {
-    const bool up = (lane & off) != 0;
-#pragma unroll
-    for (int i = 0; i < off; ++i) {
-      const float send = up ? a[i] : a[i + off];
-      const float keep = up ? a[i + off] : a[i];
-      a[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-    }
-  }
-  return a[0];
-}
-
 __device__ __forceinline__ unsigned pack_bf16(float a, float b) {
-  return (unsigned)__bfloat16_as_ushort(__float2bfloat16(a)) | ((unsigned)__bfloat16_as_ushort(__float2bfloat16(b)) << 16);
+  const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const unsigned*>(&p);
 }
 __device__ __forceinline__ float bf16_lo(unsigned u) { return __uint_as_float(u << 16); }
 __device__ __forceinline__ float bf16_hi(unsigned u) { return __uint_as_float(u & 0xFFFF0000u); }
-
-// transposed store of a warp's 32 rows x 32 columns (yp[p] = this lane's row, columns col0 + 2p and
-// col0 + 2p + 1 packed): lanes 2i and 2i+1 swap halves so each stores two consecutive rows of one
-// column as 4 bytes
-__device__ __forceinline__ void store_transposed(const unsigned (&yp)[16], __nv_bfloat16* out_t, int ldt, int col0, int row, int ncol,
-                                                 int lane) {
-  const bool odd = lane & 1;
-#pragma unroll
-  for (int p = 0; p < 16; ++p) {
-    const unsigned lo = yp[p] & 0xFFFFu, hi = yp[p] >> 16;
-    const unsigned got = __shfl_xor_sync(0xffffffffu, odd ? lo : hi, 1);
-    const int j = 2 * p + (odd ? 1 : 0);
-    const unsigned pair = odd ? (got | (hi << 16)) : (lo | (got << 16));
-    if (j < ncol) *reinterpret_cast<unsigned*>(out_t + (size_t)(col0 + j) * ldt + (row & ~1)) = pair;
-  }
-}
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, int x, int y, const void* src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(tm)),
@@ -160,7 +147,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, int x, int y
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // 32 accumulator columns of the warp's 32 rows (lane = row)
@@ -177,24 +163,21 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
 }
 
 // Activation epilogues through shared memory (EPI_ACT, EPI_DACT with whole 64-column groups).  A warp owns 32
-// rows and BN/2 columns; per 64 columns it stages the 32 x 64 tiles of its outputs in 12 KB of the operand
+// rows and BN/2 columns; per 64 columns it stages the 32 x 64 tiles of its outputs in 8 KB of the operand
 // ring (free once the accumulator is complete) and one lane stores each with TMA: every global sector is
-// written whole, where 16-byte stores from 32 rows at a stride of 1 KB wrote halves.  Row tiles: 128-byte
-// rows, 128-byte swizzle (16-byte piece p of row r at p ^ (r mod 8): conflict-free both ways); the transposed
-// tile: 64 bytes per column.  EPI_DACT loads its 32 x 64 pre-activations by TMA into the same place and
-// overwrites them.  65,536 rows x 512 columns of 512 inputs: 108 µs before, 72 µs now (backward 97 and 71; 201 MB
-// written and 67 MB read each way).
+// written whole, where 16-byte stores from 32 rows at a stride of 1 KB wrote halves.  128-byte rows, 128-byte
+// swizzle (16-byte piece p of row r at p ^ (r mod 8): conflict-free by rows and by columns).  EPI_DACT loads its
+// 32 x 64 pre-activations by TMA into the same place and overwrites them; its column sums are read back down the
+// columns, two per lane.
 template <int BN>
-__device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMap* tmO, const CUtensorMap* tmZ, const CUtensorMap* tmT,
-                                             uint32_t tmem, unsigned char* ring, const float* sbias, uint64_t* zbar, int n0, int m0, int warp,
-                                             int lane) {
+__device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMap* tmO, const CUtensorMap* tmZ, uint32_t tmem,
+                                             unsigned char* ring, const float* sbias, uint64_t* zbar, int n0, int m0, int warp, int lane) {
   const int quarter = warp & 3, half = warp >> 2;
-  unsigned char* b0 = ring + warp * 12288;  // output rows (EPI_DACT: of even groups)
-  unsigned char* b1 = b0 + 4096;            // EPI_ACT: pre-activations; EPI_DACT: output rows of odd groups
-  unsigned char* bt = b0 + 8192;            // transposed output
+  unsigned char* b0 = ring + warp * 8192;  // output rows (without a pre-activation output: of even groups)
+  unsigned char* b1 = b0 + 4096;           // pre-activations of EPI_ACT, or output rows of odd groups
   const int row0 = m0 + quarter * 32;
-  constexpr int NG = BN / 128;              // 64-column groups per warp
-  const bool dact = g.epi == EPI_DACT;
+  constexpr int NG = BN / 128;             // 64-column groups per warp
+  const bool dact = g.epi == EPI_DACT, two = dact || !g.z_out;
   if (dact && lane == 0) {  // the pre-activations of the warp's groups (at most two)
     proxy_fence();
     mbar_expect_tx(zbar, NG * 4096);
@@ -205,8 +188,8 @@ __device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMa
 #pragma unroll 1
   for (int q = 0; q < NG; ++q) {
     const int c0 = half * (BN / 2) + q * 64, col = n0 + c0;
-    unsigned char* rows = dact && q ? b1 : b0;
-    if (q) {  // the previous group's stores have read their tiles
+    unsigned char* rows = two && q ? b1 : b0;
+    if (q && !two) {  // the previous group's stores have read their tiles
       if (lane == 0) tma_store_wait_read();
       __syncwarp();
     }
@@ -214,7 +197,6 @@ __device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMa
     for (int hc = 0; hc < 2; ++hc) {
       uint32_t v[32];
       tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c0 + hc * 32), v);
-      unsigned yp[16];
 #pragma unroll
       for (int p = 0; p < 4; ++p) {  // 16-byte pieces of the lane's row
         const int off = lane * 128 + (((hc * 4 + p) ^ (lane & 7)) << 4);
@@ -229,29 +211,14 @@ __device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMa
             const float d0 = __uint_as_float(v[j]), d1 = __uint_as_float(v[j + 1]);
             o[e] = g.act == ACT_SILU ? pack_bf16(d0 * dsilu(bf16_lo(z[e])), d1 * dsilu(bf16_hi(z[e]))) : pack_bf16(d0, d1);
           } else {
-            const float z0 = __uint_as_float(v[j]) + sbias[c0 + hc * 32 + j], z1 = __uint_as_float(v[j + 1]) + sbias[c0 + hc * 32 + j + 1];
+            const float2 b = *reinterpret_cast<const float2*>(sbias + c0 + hc * 32 + j);
+            const float z0 = __uint_as_float(v[j]) + b.x, z1 = __uint_as_float(v[j + 1]) + b.y;
             z[e] = pack_bf16(z0, z1);
             o[e] = g.act == ACT_SILU ? pack_bf16(silu(z0), silu(z1)) : z[e];
           }
-          yp[4 * p + e] = o[e];
         }
         *reinterpret_cast<uint4*>(rows + off) = out;
         if (!dact && g.z_out) *reinterpret_cast<uint4*>(b1 + off) = zz;
-      }
-      if (g.out_t) {
-        unsigned short* t = reinterpret_cast<unsigned short*>(bt) + hc * 32 * 32 + lane;
-#pragma unroll
-        for (int p = 0; p < 16; ++p) {
-          t[(2 * p) * 32] = (unsigned short)(yp[p] & 0xFFFFu);
-          t[(2 * p + 1) * 32] = (unsigned short)(yp[p] >> 16);
-        }
-      }
-      if (dact && g.colsum) {
-        float a[32];
-#pragma unroll
-        for (int p = 0; p < 16; ++p) { a[2 * p] = bf16_lo(yp[p]); a[2 * p + 1] = bf16_hi(yp[p]); }
-        const float cs = warp_column_sum(a, lane);
-        atomicAdd(g.colsum + col + hc * 32 + lane, cs);
       }
     }
     proxy_fence();
@@ -259,21 +226,30 @@ __device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMa
     if (lane == 0) {
       tma_store_2d(tmO, col, row0, rows);
       if (!dact && g.z_out) tma_store_2d(tmZ, col, row0, b1);
-      if (g.out_t) tma_store_2d(tmT, row0, col, bt);
       tma_store_commit();
     }
+    if (dact && g.colsum) {  // columns col + 2 lane, + 1 (the stores above only read the tile)
+      float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+      for (int r = 0; r < 32; ++r) {
+        const unsigned u = *reinterpret_cast<const unsigned*>(rows + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+        float2& t = (r & 1) ? s1 : s0;
+        t.x += bf16_lo(u);
+        t.y += bf16_hi(u);
+      }
+      atomicAdd(reinterpret_cast<float2*>(g.colsum + col) + lane, make_float2(s0.x + s1.x, s0.y + s1.y));
+    }
   }
-  if (lane == 0) tma_store_wait();
+  if (lane == 0) tma_store_wait_read();  // the ring is read; the writes are complete when the kernel is
   __syncwarp();
   return true;
 }
 
-// TS: activation epilogue through shared memory and TMA stores (tmO, tmZ, tmT), else straight from registers.
+// TS: activation epilogue through shared memory and TMA stores (tmO, tmZ), else straight from registers.
 template <int BN, bool TS>
 __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA,
                                                          const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmO,
-                                                         const __grid_constant__ CUtensorMap tmZ, const __grid_constant__ CUtensorMap tmT,
-                                                         GemmArgs g) {
+                                                         const __grid_constant__ CUtensorMap tmZ, GemmArgs g) {
   constexpr int STAGES = stages_for<BN>();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -313,23 +289,35 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       const uint32_t ph = (uint32_t)(kt / STAGES) & 1u;
       if (!mbar_wait(&empty[s], ph ^ 1u)) { ok = false; break; }
       mbar_expect_tx(&full[s], (unsigned)((BM + BN) * BK * 2));
-      tma_load_2d(sA + (size_t)s * BM * BK * 2, &tmA, (kt0 + kt) * BK, m0, &full[s]);
-      tma_load_2d(sB + (size_t)s * BN * BK * 2, &tmB, (kt0 + kt) * BK, n0, &full[s]);
+      unsigned char* a = sA + (size_t)s * BM * BK * 2;
+      unsigned char* b = sB + (size_t)s * BN * BK * 2;
+      const int k0 = (kt0 + kt) * BK;
+      if (!TS && g.rows_k) {
+        for (int i = 0; i < BM / 64; ++i) tma_load_2d(a + i * 8192, &tmA, m0 + i * 64, k0, &full[s]);
+        for (int i = 0; i < BN / 64; ++i) tma_load_2d(b + i * 8192, &tmB, n0 + i * 64, k0, &full[s]);
+      } else {
+        tma_load_2d(a, &tmA, k0, m0, &full[s]);
+        tma_load_2d(b, &tmB, k0, n0, &full[s]);
+      }
     }
   } else if (warp == 1 && lane == 0) {  // MMA issuer
-    const uint32_t idesc = idesc_bf16<BN>();
+    const bool rows_k = !TS && g.rows_k;
+    const uint32_t idesc = idesc_bf16<BN>(rows_k);
+    const uint64_t kstep = rows_k ? 2048 >> 4 : 32 >> 4;  // 16 elements of K: 16 rows, or 32 B inside the swizzled row
     for (int kt = 0; kt < KT; ++kt) {
       const int s = kt % STAGES;
       const uint32_t ph = (uint32_t)(kt / STAGES) & 1u;
       if (!mbar_wait(&full[s], ph)) { ok = false; break; }
       tc_fence_after();
-      const uint64_t ad = desc_sw128(sA + (size_t)s * BM * BK * 2), bd = desc_sw128(sB + (size_t)s * BN * BK * 2);
+      const unsigned char* a = sA + (size_t)s * BM * BK * 2;
+      const unsigned char* b = sB + (size_t)s * BN * BK * 2;
+      const uint64_t ad = rows_k ? desc_sw128_rows_k(a) : desc_sw128(a), bd = rows_k ? desc_sw128_rows_k(b) : desc_sw128(b);
 #pragma unroll
-      for (int kk = 0; kk < BK / 16; ++kk) {  // advance 16 elements = 32 B inside the swizzled row
+      for (int kk = 0; kk < BK / 16; ++kk) {
         const uint32_t acc = (kt | kk) != 0;
         asm volatile(
             "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-            "l"(ad + 2 * kk), "l"(bd + 2 * kk), "r"(idesc), "r"(acc)
+            "l"(ad + kstep * kk), "l"(bd + kstep * kk), "r"(idesc), "r"(acc)
             : "memory");
       }
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty[s])) : "memory");
@@ -344,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   const int quarter = warp & 3, half = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
   if constexpr (TS) {
-    if (ok) ok = epilogue_tma<BN>(g, &tmO, &tmZ, &tmT, tmem, base, sbias, &zbar[warp], n0, m0, warp, lane);
+    if (ok) ok = epilogue_tma<BN>(g, &tmO, &tmZ, tmem, base, sbias, &zbar[warp], n0, m0, warp, lane);
   } else if (ok) {
 #pragma unroll 1
     for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
@@ -443,15 +431,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
               if (j < nv) g.out_bf16[o + j] = __ushort_as_bfloat16((unsigned short)((j & 1) ? yp[j >> 1] >> 16 : yp[j >> 1] & 0xFFFFu));
           }
         }
-        if (g.colsum) {  // warp-collective; rows beyond M contribute zeros
-          float a[32];
-#pragma unroll
-          for (int p = 0; p < 16; ++p) { a[2 * p] = bf16_lo(yp[p]); a[2 * p + 1] = bf16_hi(yp[p]); }
-          const float cs = warp_column_sum(a, lane);
-          if (lane < nv) atomicAdd(g.colsum + col + lane, cs);
-        }
       }
-      if (g.out_t && m0 + quarter * 32 < g.M) store_transposed(yp, g.out_t, g.ldt, col, row, nv, lane);
     }
   }
   tc_fence_before();

@@ -4,15 +4,14 @@
 // Layout: layer l maps kin_l → nrow_l features; the input is padded to 64 columns and the output
 // to 64 rows (TMA/UMMA granularity), padding weights stay zero (their gradients are zero).  Master
 // weights, Adam moments and gradients are FP32 [nrow][kin]; the GEMMs read BF16 copies W [nrow][kin]
-// (forward) and Wt [kin][nrow] (backward).  Activations are BF16 [batch][features], each with a
-// transposed copy [features][batch] written by the same epilogue (the weight-gradient GEMMs read
-// the batch as their K dimension); the last layer writes FP32 so the loss is not quantised.  A
-// training step:
-//   gather    X_0 (and X_0ᵀ), targets T of the step's random batch
-//   forward   X_l = SiLU(X_{l-1} W_lᵀ + b_l)          (EPI_ACT, pre-activations Z_l kept, X_lᵀ)
-//   loss      Y = X_L W_Lᵀ + b_L (FP32), dY = 2 (Y - T) / (batch · nout), dYᵀ, db_L = Σ_batch dY
-//   backward  dZ_{l-1} = (dZ_l W_l) ⊙ SiLU'(Z_{l-1})  (EPI_DACT, dZ_{l-1}ᵀ and db_{l-1} = Σ_batch dZ_{l-1})
-//             dW_l = dZ_lᵀ X_{l-1} (EPI_F32 on the transposed copies, split K)
+// (forward) and Wt [kin][nrow] (backward).  Activations are BF16 [batch][features] (the weight-gradient
+// GEMMs read them with the batch as their K dimension); the last layer writes FP32 so the loss is not
+// quantised.  A training step:
+//   gather    X_0, targets T of the step's random batch
+//   forward   X_l = SiLU(X_{l-1} W_lᵀ + b_l)          (EPI_ACT, pre-activations Z_l kept)
+//   loss      Y = X_L W_Lᵀ + b_L (FP32), dY = 2 (Y - T) / (batch · nout), db_L = Σ_batch dY
+//   backward  dZ_{l-1} = (dZ_l W_l) ⊙ SiLU'(Z_{l-1})  (EPI_DACT, db_{l-1} = Σ_batch dZ_{l-1})
+//             dW_l = dZ_lᵀ X_{l-1} (EPI_F32 with rows along K, split K)
 //   Adam      one launch over every parameter: FP32 update, BF16 W and Wt refreshed.
 // The step (about 20 launches) is captured once in a CUDA graph and replayed; the step counter
 // and the learning rate live in device memory so the replayed graph needs no new parameters.
@@ -56,9 +55,9 @@ struct sbz_surrogate {
   int nin = 0, width = 0, nhidden = 0, nout = 0, batch = 0;
   std::vector<Layer> L;
   // activations (batch rows): X[0] input, X[l] output of hidden layer l; Z[l] pre-activations
-  std::vector<bf16*> X, Z, Xt, dZ, dZt;
+  std::vector<bf16*> X, Z, dZ;
   float* Yf = nullptr;        // [batch][64] last-layer product (before bias)
-  bf16 *dY = nullptr, *dYt = nullptr;
+  bf16* dY = nullptr;
   float* T = nullptr;         // [batch][nout] targets of the step
   double* loss = nullptr;     // first entry of grads
   unsigned char* grads = nullptr;  // loss and every layer's gW and gb: one memset per step
@@ -91,13 +90,11 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
 }
 
 // dstep (if not null): the step is *dstep + 1 (the graph-captured training step reads the device counter,
-// which loss_grad advances).  X0 rows are written whole (padding zero); X0t (if not null) receives the
-// transposed copy of the first nin columns (the others stay zero).  A warp assembles 32 rows: one hash per
-// lane, row pieces along the row, the transposed copy along the batch (one thread per row wrote 2-byte
-// pieces of 64 rows and columns: 47 µs for 65,536 rows).
+// which loss_grad advances).  X0 rows are written whole (padding zero).  A warp assembles 32 rows: one hash per
+// lane, row pieces along the row (one thread per row wrote 2-byte pieces of 64 rows: 47 µs for 65,536 rows).
 __global__ void __launch_bounds__(128) gather_batch(int batch, int nin, int nout, const float* __restrict__ dX, const float* __restrict__ dY,
                                                     long long n, const long long* __restrict__ dstep, unsigned long long seed, int random,
-                                                    bf16* __restrict__ X0, bf16* __restrict__ X0t, float* __restrict__ T) {
+                                                    bf16* __restrict__ X0, float* __restrict__ T) {
   __shared__ long long rows[4][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, i0 = (blockIdx.x * 4 + warp) * 32;
   if (i0 >= batch) return;  // batch is a multiple of 32
@@ -119,9 +116,6 @@ __global__ void __launch_bounds__(128) gather_batch(int batch, int nin, int nout
     const float a = r >= 0 && j < nin ? x[j] : 0.0f, b = r >= 0 && j + 1 < nin ? x[j + 1] : 0.0f;
     reinterpret_cast<__nv_bfloat162*>(X0 + (size_t)(i0 + q) * kPadIn)[lane] = __floats2bfloat162_rn(a, b);
   }
-  const long long r = rows[warp][lane];
-  if (X0t)
-    for (int j = 0; j < nin; ++j) X0t[(size_t)j * batch + i0 + lane] = __float2bfloat16(r >= 0 ? dX[r * nin + j] : 0.0f);
   if (T)
     for (int e = lane; e < 32 * nout; e += 32) {
       const int q = e / nout;
@@ -133,12 +127,12 @@ __global__ void __launch_bounds__(128) gather_batch(int batch, int nin, int nout
 __global__ void set_value(float* dst, float v) { *dst = v; }
 
 // loss and output gradient: y = Yf + b (FP32), r = y - t, dY = 2 r / (batch · nout) (BF16; padding columns
-// stay zero), dYᵀ [kPadOut][batch] and the bias gradient gb[j] += Σ_rows dY[.][j] (as rounded).
+// stay zero) and the bias gradient gb[j] += Σ_rows dY[.][j] (as rounded).
 // 256 threads per block.  Advances the device step counter (if not null; nothing else here reads it).
 constexpr int kLossThreads = 256;
 __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, const float* __restrict__ Yf, const float* __restrict__ b,
-                                                           const float* __restrict__ T, bf16* __restrict__ dY, bf16* __restrict__ dYt,
-                                                           float* __restrict__ gb, double* __restrict__ loss, long long* __restrict__ dstep) {
+                                                           const float* __restrict__ T, bf16* __restrict__ dY, float* __restrict__ gb,
+                                                           double* __restrict__ loss, long long* __restrict__ dstep) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   __shared__ float cs[kLossThreads / 32][kPadOut];
   double l = 0;
@@ -151,10 +145,7 @@ __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, c
       g = sc * r;
     }
     const bf16 gh = __float2bfloat16(g);
-    if (i < batch) {
-      dY[(size_t)i * kPadOut + j] = gh;
-      dYt[(size_t)j * batch + i] = gh;
-    }
+    if (i < batch) dY[(size_t)i * kPadOut + j] = gh;
     float w = __bfloat162float(gh);
     for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
     if ((threadIdx.x & 31) == 0) cs[threadIdx.x >> 5][j] = w;
@@ -267,9 +258,9 @@ void free_all(sbz_surrogate* s) {
   for (auto& l : s->L)
     for (void* p : {(void*)l.W, (void*)l.b, (void*)l.mW, (void*)l.vW, (void*)l.mb, (void*)l.vb, (void*)l.Wh, (void*)l.Wt})
       if (p) cudaFree(p);
-  for (auto* v : {&s->X, &s->Z, &s->Xt, &s->dZ, &s->dZt})
+  for (auto* v : {&s->X, &s->Z, &s->dZ})
     for (bf16* p : *v) if (p) cudaFree(p);
-  for (void* p : {(void*)s->Yf, (void*)s->dY, (void*)s->dYt, (void*)s->T, (void*)s->grads, (void*)s->err, (void*)s->dataX, (void*)s->dataY,
+  for (void* p : {(void*)s->Yf, (void*)s->dY, (void*)s->T, (void*)s->grads, (void*)s->err, (void*)s->dataX, (void*)s->dataY,
                   (void*)s->dstep, (void*)s->dlr, s->segs})
     if (p) cudaFree(p);
   if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
@@ -286,52 +277,51 @@ int refresh_bf16(sbz_surrogate* s) {
 }
 
 int gemm(sbz_surrogate* s, int M, int N, int K, const bf16* A, const bf16* B, int epi, int act, const float* bias, void* out, int ldo,
-         int n_valid, int acc, bf16* z_out, const bf16* z_in, bf16* out_t = nullptr, float* colsum = nullptr) {
+         int n_valid, int acc, bf16* z_out, const bf16* z_in, float* colsum = nullptr, int rows_k = 0) {
   using namespace sbz::mlp;
   GemmArgs g{};
   g.M = M; g.N = N; g.K = K; g.epi = epi; g.act = act; g.bias = bias;
   g.out_bf16 = static_cast<bf16*>(out); g.out_f32 = static_cast<float*>(out); g.ldo = ldo; g.n_valid = n_valid; g.accumulate = acc;
   g.z_out = z_out; g.z_in = z_in; g.err = s->err;
-  g.out_t = out_t; g.ldt = M; g.colsum = colsum;
+  g.colsum = colsum; g.rows_k = rows_k;
   const int r = sbz::mlp::gemm(g, A, B, s->stream);
   return r == SBZ_OK ? SBZ_OK : F(r, "surrogate: GEMM launch");
 }
 
 // forward pass of `rows` (multiple of 128, ≤ batch) rows already in X[0]; result in Yf.  With
-// `train`, the pre-activations and the transposed activations X_lᵀ (row stride `rows`) are written for the
-// backward pass.
+// `train`, the pre-activations are written for the backward pass.
 int forward(sbz_surrogate* s, int rows, bool train) {
   using namespace sbz::mlp;
   const int nl = (int)s->L.size();
   for (int l = 0; l < nl - 1; ++l) {
     const Layer& y = s->L[l];
     int r = gemm(s, rows, y.nrow, y.kin, s->X[l], y.Wh, EPI_ACT, ACT_SILU, y.b, s->X[l + 1], y.nrow, y.nrow, 0,
-                 train ? s->Z[l + 1] : nullptr, nullptr, train ? s->Xt[l + 1] : nullptr);
+                 train ? s->Z[l + 1] : nullptr, nullptr);
     if (r) return r;
   }
   const Layer& o = s->L[nl - 1];
   return gemm(s, rows, o.nrow, o.kin, s->X[nl - 1], o.Wh, EPI_F32, ACT_NONE, nullptr, s->Yf, kPadOut, s->nout, 0, nullptr, nullptr);
 }
 
-// backward pass after forward(train) + loss_grad (dY, dYᵀ and the output layer's gb set): weight
+// backward pass after forward(train) + loss_grad (dY and the output layer's gb set): weight
 // gradients added into gW, bias gradients into gb by the EPI_DACT epilogues (both zeroed before)
 int backward(sbz_surrogate* s) {
   using namespace sbz::mlp;
   const int B = s->batch, nl = (int)s->L.size();
   // output layer: dW_Lᵀ = X_{L-1}ᵀ dY ([kin][64]); dZ_{L-1} = (dY W_L) ⊙ SiLU'(Z_{L-1})
   Layer& o = s->L[nl - 1];
-  int r = gemm(s, o.kin, kPadOut, B, s->Xt[nl - 1], s->dYt, EPI_F32, ACT_NONE, nullptr, o.gW, kPadOut, kPadOut, 1, nullptr, nullptr);
+  int r = gemm(s, o.kin, kPadOut, B, s->X[nl - 1], s->dY, EPI_F32, ACT_NONE, nullptr, o.gW, kPadOut, kPadOut, 1, nullptr, nullptr, nullptr, 1);
   if (r) return r;
   r = gemm(s, B, o.kin, kPadOut, s->dY, o.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[nl - 1], o.kin, o.kin, 0, nullptr, s->Z[nl - 1],
-           s->dZt[nl - 1], s->L[nl - 2].gb);
+           s->L[nl - 2].gb);
   if (r) return r;
   // hidden layers l = nl-2 .. 0: input X[l], output gradient dZ[l+1]
   for (int l = nl - 2; l >= 0; --l) {
     Layer& y = s->L[l];
-    r = gemm(s, y.nrow, y.kin, B, s->dZt[l + 1], s->Xt[l], EPI_F32, ACT_NONE, nullptr, y.gW, y.kin, y.kin, 1, nullptr, nullptr);
+    r = gemm(s, y.nrow, y.kin, B, s->dZ[l + 1], s->X[l], EPI_F32, ACT_NONE, nullptr, y.gW, y.kin, y.kin, 1, nullptr, nullptr, nullptr, 1);
     if (r) return r;
     if (l > 0) {
-      r = gemm(s, B, y.kin, y.nrow, s->dZ[l + 1], y.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[l], y.kin, y.kin, 0, nullptr, s->Z[l], s->dZt[l],
+      r = gemm(s, B, y.kin, y.nrow, s->dZ[l + 1], y.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[l], y.kin, y.kin, 0, nullptr, s->Z[l],
                s->L[l - 1].gb);
       if (r) return r;
     }
@@ -344,16 +334,15 @@ int forward_backward(sbz_surrogate* s, int rows, long long* dstep) {
   SCU(cudaMemsetAsync(s->grads, 0, s->grads_bytes, s->stream));
   int r = forward(s, rows, true);
   if (r) return r;
-  loss_grad<<<(rows + kLossThreads - 1) / kLossThreads, kLossThreads, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, s->T, s->dY, s->dYt,
-                                                                                  s->L.back().gb, s->loss, dstep);
+  loss_grad<<<(rows + kLossThreads - 1) / kLossThreads, kLossThreads, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, s->T, s->dY, s->L.back().gb,
+                                                                                  s->loss, dstep);
   return backward(s);
 }
 
 // one training step on the stream (captured into the step graph)
 int train_step(sbz_surrogate* s) {
   const int B = s->batch;
-  gather_batch<<<(B + 127) / 128, 128, 0, s->stream>>>(B, s->nin, s->nout, s->dataX, s->dataY, s->ndata, s->dstep, s->seed, 1, s->X[0], s->Xt[0],
-                                                      s->T);
+  gather_batch<<<(B + 127) / 128, 128, 0, s->stream>>>(B, s->nin, s->nout, s->dataX, s->dataY, s->ndata, s->dstep, s->seed, 1, s->X[0], s->T);
   int r = forward_backward(s, B, s->dstep);
   if (r) return r;
   adam_all<<<s->nadam, 256, 0, s->stream>>>(static_cast<const AdamSeg*>(s->segs), s->nseg, s->dstep, s->dlr, 0.9f, 0.999f, 1e-8f);
@@ -425,21 +414,19 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
       s->L[l].gb = reinterpret_cast<float*>(s->grads + ob[l]);
     }
   }
-  s->X.assign(nl, nullptr); s->Z.assign(nl, nullptr); s->Xt.assign(nl, nullptr); s->dZ.assign(nl, nullptr); s->dZt.assign(nl, nullptr);
+  s->X.assign(nl, nullptr); s->Z.assign(nl, nullptr); s->dZ.assign(nl, nullptr);
   for (int l = 0; l < nl; ++l) {
     const int w = l == 0 ? kPadIn : width;
-    if (dalloc(&s->X[l], (size_t)batch * w) || dalloc(&s->Xt[l], (size_t)batch * w)) return bail("surrogate: activation allocation");
-    if (l > 0 && (dalloc(&s->Z[l], (size_t)batch * w) || dalloc(&s->dZ[l], (size_t)batch * w) || dalloc(&s->dZt[l], (size_t)batch * w)))
+    if (dalloc(&s->X[l], (size_t)batch * w)) return bail("surrogate: activation allocation");
+    if (l > 0 && (dalloc(&s->Z[l], (size_t)batch * w) || dalloc(&s->dZ[l], (size_t)batch * w)))
       return bail("surrogate: activation allocation");
   }
-  if (dalloc(&s->Yf, (size_t)batch * kPadOut) || dalloc(&s->dY, (size_t)batch * kPadOut) || dalloc(&s->dYt, (size_t)batch * kPadOut) ||
+  if (dalloc(&s->Yf, (size_t)batch * kPadOut) || dalloc(&s->dY, (size_t)batch * kPadOut) ||
       dalloc(&s->T, (size_t)batch * nout) || dalloc(&s->err, 1))
     return bail("surrogate: buffer allocation");
   cudaMemset(s->err, 0, sizeof(unsigned));
-  // padding columns and rows that no kernel writes
-  cudaMemset(s->Xt[0], 0, sizeof(bf16) * (size_t)batch * kPadIn);
+  // padding columns that no kernel writes
   cudaMemset(s->dY, 0, sizeof(bf16) * (size_t)batch * kPadOut);
-  cudaMemset(s->dYt, 0, sizeof(bf16) * (size_t)batch * kPadOut);
   {
     std::vector<AdamSeg> segs;
     int start = 0;
@@ -557,7 +544,7 @@ int sbz_surrogate_gradients(sbz_surrogate* s, int n, const float* X, const float
   SCU(dalloc(&dy, (size_t)n * s->nout));
   SCU(cudaMemcpy(dx, X, sizeof(float) * n * s->nin, cudaMemcpyHostToDevice));
   SCU(cudaMemcpy(dy, Y, sizeof(float) * n * s->nout, cudaMemcpyHostToDevice));
-  gather_batch<<<(n + 127) / 128, 128, 0, s->stream>>>(n, s->nin, s->nout, dx, dy, n, nullptr, 0, 0, s->X[0], s->Xt[0], s->T);
+  gather_batch<<<(n + 127) / 128, 128, 0, s->stream>>>(n, s->nin, s->nout, dx, dy, n, nullptr, 0, 0, s->X[0], s->T);
   int r = forward_backward(s, n, nullptr);
   s->batch = keepB;
   cudaFree(dx); cudaFree(dy);
@@ -593,8 +580,7 @@ int sbz_surrogate_infer(sbz_surrogate* s, long long n, const float* X, float* Y)
     for (long long b0 = 0; b0 < cn && !r; b0 += B) {
       const int rows = (int)std::min<long long>(B, cn - b0);
       const int prow = (rows + 127) / 128 * 128;
-      gather_batch<<<(prow + 127) / 128, 128, 0, s->stream>>>(prow, s->nin, s->nout, dx + b0 * s->nin, nullptr, rows, nullptr, 0, 0, s->X[0],
-                                                              nullptr, nullptr);
+      gather_batch<<<(prow + 127) / 128, 128, 0, s->stream>>>(prow, s->nin, s->nout, dx + b0 * s->nin, nullptr, rows, nullptr, 0, 0, s->X[0], nullptr);
       if ((r = forward(s, prow, false))) break;
       add_bias_out<<<(rows * s->nout + 255) / 256, 256, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, dyo);
       if (cudaMemcpyAsync(Y + (c0 + b0) * s->nout, dyo, sizeof(float) * rows * s->nout, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess)
