@@ -54,40 +54,40 @@ int num_sms() {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
-// Activation epilogue through TMA: whole 64-column groups, 16-byte row strides and bases.
-bool tma_epilogue(const GemmArgs& g, int bn) {
-  if (g.epi == EPI_F32 || bn < 128 || g.n_valid != g.N || g.ldo % 8 || !aligned16(g.out_bf16)) return false;
+// Shapes of gemm_act_kernel: whole 128-column tiles, 16-byte row strides and bases.  65,536 x 512
+// x 512 forward and backward: 45 and 46 µs, where one tile per CTA and two CTAs per SM with the same epilogue took
+// 55 and 57 (64 inputs: 30 and 33).
+bool act_tiles(const GemmArgs& g, int bn) {
+  if (g.epi == EPI_F32 || bn < 128 || g.n_valid != g.N || g.ldo % 8 || !aligned16(g.out_bf16) || !aligned16(g.bias)) return false;
   if (g.epi == EPI_DACT && !aligned16(g.z_in)) return false;
   return g.epi != EPI_ACT || !g.z_out || aligned16(g.z_out);
 }
 
-template <int BN, bool TS>
-int launch_k(const GemmArgs& g, const void* A, const void* B, int splits, cudaStream_t st) {
+template <int BN>
+int launch_act(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   CUtensorMap ta, tb, to, tz;
-  if (g.rows_k) {  // [K][M], [K][N] in pieces of 64 x 64
-    if (!tmap_operand(&ta, A, g.K, g.M, BK) || !tmap_operand(&tb, B, g.K, g.N, BK)) return SBZ_ERR_CUDA;
-  } else if (!tmap_operand(&ta, A, g.M, g.K, BM) || !tmap_operand(&tb, B, g.N, g.K, BN)) {
+  const void* z = g.epi == EPI_DACT ? static_cast<const void*>(g.z_in) : g.z_out;
+  if (!tmap_operand(&ta, A, g.M, g.K, BM) || !tmap_operand(&tb, B, g.N, g.K, BN) || !tmap(&to, g.out_bf16, g.M, g.N, g.ldo, 64, 32))
     return SBZ_ERR_CUDA;
-  }
-  to = tz = ta;
-  if (TS) {
-    const void* z = g.epi == EPI_DACT ? static_cast<const void*>(g.z_in) : g.z_out;
-    if (!tmap(&to, g.out_bf16, g.M, g.N, g.ldo, 64, 32)) return SBZ_ERR_CUDA;
-    if (z && !tmap(&tz, z, g.M, g.N, g.ldo, 64, 32)) return SBZ_ERR_CUDA;
-  }
-  const size_t smem = gemm_smem_bytes<BN>();
-  auto k = gemm_tn_kernel<BN, TS>;
+  tz = to;
+  if (z && !tmap(&tz, z, g.M, g.N, g.ldo, 64, 32)) return SBZ_ERR_CUDA;
+  constexpr size_t smem = gemm_act_smem_bytes<BN>();
+  static_assert(smem <= 227 * 1024, "shared memory of an SM");
   static bool attr_set = false;  // set once, outside any stream capture of a later call
   if (!attr_set) {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
+    if (cudaFuncSetAttribute(gemm_act_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
     attr_set = true;
   }
-  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, to, tz, g);
+  const int tiles = (g.N / BN) * (g.M / BM);
+  gemm_act_kernel<BN><<<std::min(tiles, num_sms()), kActThreads, smem, st>>>(ta, tb, to, tz, g);
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
 }
 
 template <int BN>
 int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
+  if constexpr (BN >= 128)
+    if (act_tiles(g, BN)) return launch_act<BN>(g, A, B, st);
+  if (g.colsum) return SBZ_ERR_ARG;  // only gemm_act_kernel forms column sums
   const int tiles = (g.N / BN) * (g.M / BM), KT = g.K / BK;
   // weight gradients have few output tiles and a long K (the batch): split K over about two CTAs
   // per SM, at least 4 K-steps each, and add the partial tiles atomically into a zeroed output
@@ -97,10 +97,21 @@ int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   if (splits > 1 && !g.accumulate &&
       cudaMemset2DAsync(g.out_f32, sizeof(float) * (size_t)g.ldo, 0, sizeof(float) * (size_t)g.n_valid, (size_t)g.M, st) != cudaSuccess)
     return SBZ_ERR_CUDA;
-  if constexpr (BN >= 128)
-    if (tma_epilogue(g, BN)) return launch_k<BN, true>(g, A, B, 1, st);
-  if (g.colsum) return SBZ_ERR_ARG;  // only the shared-memory epilogue forms column sums
-  return launch_k<BN, false>(g, A, B, splits, st);
+  CUtensorMap ta, tb;
+  if (g.rows_k) {  // [K][M], [K][N] in pieces of 64 x 64
+    if (!tmap_operand(&ta, A, g.K, g.M, BK) || !tmap_operand(&tb, B, g.K, g.N, BK)) return SBZ_ERR_CUDA;
+  } else if (!tmap_operand(&ta, A, g.M, g.K, BM) || !tmap_operand(&tb, B, g.N, g.K, BN)) {
+    return SBZ_ERR_CUDA;
+  }
+  const size_t smem = gemm_smem_bytes<BN>();
+  auto k = gemm_tn_kernel<BN>;
+  static bool attr_set = false;  // set once, outside any stream capture of a later call
+  if (!attr_set) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
+    attr_set = true;
+  }
+  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, g);
+  return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
 }
 
 }  // namespace

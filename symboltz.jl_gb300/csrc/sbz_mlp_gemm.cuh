@@ -3,19 +3,16 @@
 //   D[M x N] = A[M x K] · B[N x K]ᵀ   (A, B bf16 row-major with K contiguous, FP32 accumulation)
 //   D[M x N] = A[K x M]ᵀ · B[K x N]   (the same with rows along K: the weight gradients, whose K is the batch)
 //
-// One CTA computes a 128 x BN tile; two CTAs share an SM (≈ 100 KB of shared memory and at most
-// 128 registers per thread each), so one CTA's epilogue overlaps the other's loads.  Warp 0 lane 0
-// streams 128 x 64 and BN x 64 K-slices into a shared-memory ring of stages_for<BN>() slots with
-// TMA (128-byte swizzle); warp 1 lane 0 issues
-// tcgen05.mma (kind::f16, M = 128, N = BN, K = 16) into a TMEM accumulator and releases ring
-// slots with tcgen05.commit; all eight warps then read the accumulator with tcgen05.ld (warp w owns
-// TMEM lanes 32(w mod 4).. = tile rows, and half w / 4 of the tile's columns) and apply the fused
-// epilogue:
+// Warp 0 lane 0 streams 128 x 64 and BN x 64 K-slices into a shared-memory ring of stages_for<BN>() slots with
+// TMA (128-byte swizzle); warp 1 lane 0 issues tcgen05.mma (kind::f16, M = 128, N = BN, K = 16) into a TMEM
+// accumulator and releases ring slots with tcgen05.commit; the epilogue warps read the accumulator with
+// tcgen05.ld (warp w owns TMEM lanes 32(w mod 4).. = tile rows) and apply the fused epilogue:
 //   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add with 16-byte atomics)
 //   EPI_ACT   z = D + bias; out = bf16(act(z)); optional z_out = bf16(z)    forward layers
 //   EPI_DACT  out = bf16(D · act'(z_in))                                   backward layers
-// Whole 64-column groups go through shared memory and TMA stores (epilogue_tma), where EPI_DACT can also
-// add the output's column sums into colsum (the bias gradient); other shapes are stored from registers.
+// Two kernels: gemm_act_kernel (whole tiles of the activation epilogues) is persistent, and its epilogue runs
+// beside the next tile's product; gemm_tn_kernel (one 128 x BN tile per CTA, two CTAs per SM) does EPI_F32 and
+// activation outputs that TMA cannot store.
 // Every mbarrier wait is bounded: a wait that runs out sets *err and the CTA skips ahead to its
 // TMEM release, so a fault in the pipeline cannot hang the GPU.
 #pragma once
@@ -53,7 +50,7 @@ struct GemmArgs {
 template <int BN>
 constexpr size_t gemm_smem_bytes() {
   constexpr int STAGES = stages_for<BN>();
-  return 1024 /* alignment slack */ + (size_t)STAGES * (BM + BN) * BK * 2 + (2 * STAGES + 1 + 8) * 8 + 16 + BN * 4 /* bias */;
+  return 1024 /* alignment slack */ + (size_t)STAGES * (BM + BN) * BK * 2 + (2 * STAGES + 1) * 8 + 16 + BN * 4 /* bias */;
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -76,6 +73,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
     if (ready) return true;
   }
   return false;
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* b) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
   asm volatile(
@@ -116,6 +116,15 @@ __device__ __forceinline__ uint32_t idesc_bf16(bool rows_k) {
          | (1u << 7) | (1u << 10)     // A, B: BF16
          | ((uint32_t)(BN >> 3) << 17) // N
          | ((uint32_t)(BM >> 4) << 24); // M
+}
+
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d), "l"(a),
+               "l"(b), "r"(idesc), "r"((uint32_t)accumulate)
+               : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) {  // arrives when the products issued so far are done
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // SiLU and its derivative with the hardware's exponential and reciprocal.  Their flush-to-zero forms: e^{-z} below
@@ -162,94 +171,196 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// Activation epilogues through shared memory (EPI_ACT, EPI_DACT with whole 64-column groups).  A warp owns 32
-// rows and BN/2 columns; per 64 columns it stages the 32 x 64 tiles of its outputs in 8 KB of the operand
-// ring (free once the accumulator is complete) and one lane stores each with TMA: every global sector is
-// written whole, where 16-byte stores from 32 rows at a stride of 1 KB wrote halves.  128-byte rows, 128-byte
-// swizzle (16-byte piece p of row r at p ^ (r mod 8): conflict-free by rows and by columns).  EPI_DACT loads its
-// 32 x 64 pre-activations by TMA into the same place and overwrites them; its column sums are read back down the
-// columns, two per lane.
+// Activation layers (EPI_ACT, EPI_DACT) of whole 128 x BN tiles: one CTA per SM takes every gridDim-th tile, and
+// the accumulator is double-buffered in TMEM, so the epilogue of a tile (about 25 µs per 65,536 x 512 layer, bound
+// by instruction issue) runs beside the loads and the product of the next one (402 MB from
+// L2, the bound at 512 inputs: 45 µs with three ring slots of 48 KB, 55 with two).  Warp 0 loads, warp 1 issues the products, 16 epilogue warps take
+// 32 rows x 64 columns each (BN = 128: eight of them per tile, in turn).  A warp stages its tiles in 8 KB of
+// shared memory and one lane stores them with TMA: every global sector is written whole, where 16-byte stores
+// from 32 rows at a stride of 1 KB wrote halves.  128-byte rows, 128-byte swizzle (16-byte piece p of row r at
+// p ^ (r mod 8): conflict-free by rows and by columns).  EPI_DACT loads its pre-activations by TMA one tile ahead
+// and overwrites them; its column sums are read back down the columns, two per lane.
+constexpr int kActWarps = 16, kActThreads = 64 + 32 * kActWarps, kStage = 4096;
 template <int BN>
-__device__ __forceinline__ bool epilogue_tma(const GemmArgs& g, const CUtensorMap* tmO, const CUtensorMap* tmZ, uint32_t tmem,
-                                             unsigned char* ring, const float* sbias, uint64_t* zbar, int n0, int m0, int warp, int lane) {
-  const int quarter = warp & 3, half = warp >> 2;
-  unsigned char* b0 = ring + warp * 8192;  // output rows (without a pre-activation output: of even groups)
-  unsigned char* b1 = b0 + 4096;           // pre-activations of EPI_ACT, or output rows of odd groups
-  const int row0 = m0 + quarter * 32;
-  constexpr int NG = BN / 128;             // 64-column groups per warp
-  const bool dact = g.epi == EPI_DACT, two = dact || !g.z_out;
-  if (dact && lane == 0) {  // the pre-activations of the warp's groups (at most two)
-    proxy_fence();
-    mbar_expect_tx(zbar, NG * 4096);
-#pragma unroll
-    for (int q = 0; q < NG; ++q) tma_load_2d(q ? b1 : b0, tmZ, n0 + half * (BN / 2) + q * 64, row0, zbar);
-  }
-  if (dact && !mbar_wait(zbar, 0)) return false;
-#pragma unroll 1
-  for (int q = 0; q < NG; ++q) {
-    const int c0 = half * (BN / 2) + q * 64, col = n0 + c0;
-    unsigned char* rows = two && q ? b1 : b0;
-    if (q && !two) {  // the previous group's stores have read their tiles
-      if (lane == 0) tma_store_wait_read();
-      __syncwarp();
-    }
-#pragma unroll
-    for (int hc = 0; hc < 2; ++hc) {
-      uint32_t v[32];
-      tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(c0 + hc * 32), v);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {  // 16-byte pieces of the lane's row
-        const int off = lane * 128 + (((hc * 4 + p) ^ (lane & 7)) << 4);
-        uint4 out, zz;
-        unsigned* o = reinterpret_cast<unsigned*>(&out);
-        unsigned* z = reinterpret_cast<unsigned*>(&zz);
-        if (dact) zz = *reinterpret_cast<const uint4*>(rows + off);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = 8 * p + 2 * e;
-          if (dact) {
-            const float d0 = __uint_as_float(v[j]), d1 = __uint_as_float(v[j + 1]);
-            o[e] = g.act == ACT_SILU ? pack_bf16(d0 * dsilu(bf16_lo(z[e])), d1 * dsilu(bf16_hi(z[e]))) : pack_bf16(d0, d1);
-          } else {
-            const float2 b = *reinterpret_cast<const float2*>(sbias + c0 + hc * 32 + j);
-            const float z0 = __uint_as_float(v[j]) + b.x, z1 = __uint_as_float(v[j + 1]) + b.y;
-            z[e] = pack_bf16(z0, z1);
-            o[e] = g.act == ACT_SILU ? pack_bf16(silu(z0), silu(z1)) : z[e];
-          }
-        }
-        *reinterpret_cast<uint4*>(rows + off) = out;
-        if (!dact && g.z_out) *reinterpret_cast<uint4*>(b1 + off) = zz;
-      }
-    }
-    proxy_fence();
-    __syncwarp();
-    if (lane == 0) {
-      tma_store_2d(tmO, col, row0, rows);
-      if (!dact && g.z_out) tma_store_2d(tmZ, col, row0, b1);
-      tma_store_commit();
-    }
-    if (dact && g.colsum) {  // columns col + 2 lane, + 1 (the stores above only read the tile)
-      float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
-#pragma unroll
-      for (int r = 0; r < 32; ++r) {
-        const unsigned u = *reinterpret_cast<const unsigned*>(rows + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
-        float2& t = (r & 1) ? s1 : s0;
-        t.x += bf16_lo(u);
-        t.y += bf16_hi(u);
-      }
-      atomicAdd(reinterpret_cast<float2*>(g.colsum + col) + lane, make_float2(s0.x + s1.x, s0.y + s1.y));
-    }
-  }
-  if (lane == 0) tma_store_wait_read();  // the ring is read; the writes are complete when the kernel is
-  __syncwarp();
-  return true;
+__host__ __device__ constexpr int act_stages() { return BN >= 256 ? 3 : 5; }  // what the staging leaves of 227 KB
+template <int BN>
+constexpr size_t gemm_act_smem_bytes() {
+  return 1024 /* alignment slack */ + (size_t)act_stages<BN>() * (BM + BN) * BK * 2 + kActWarps * kStage +
+         (2 * act_stages<BN>() + 4 + kActWarps) * 8 + 16;
 }
 
-// TS: activation epilogue through shared memory and TMA stores (tmO, tmZ), else straight from registers.
-template <int BN, bool TS>
+template <int BN>
+__global__ void __launch_bounds__(kActThreads, 1) gemm_act_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                                                                  const __grid_constant__ CUtensorMap tmO, const __grid_constant__ CUtensorMap tmZ,
+                                                                  GemmArgs g) {
+  constexpr int STAGES = act_stages<BN>(), SETS = 256 / BN;  // warp sets that take tiles in turn
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* sA = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sB = sA + (size_t)STAGES * BM * BK * 2;
+  unsigned char* stage = sB + (size_t)STAGES * BN * BK * 2;
+  uint64_t* full = (uint64_t*)(stage + kActWarps * kStage);
+  uint64_t* empty = full + STAGES;
+  uint64_t* tfull = empty + STAGES;   // accumulator ready / read, per TMEM buffer
+  uint64_t* tempty = tfull + 2;
+  uint64_t* zbar = tempty + 2;        // one per epilogue warp (pre-activation tiles)
+  uint32_t* tmem_slot = (uint32_t*)(zbar + kActWarps);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nt = g.N / BN, ntiles = nt * (g.M / BM), KT = g.K / BK;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], kActWarps / SETS); }
+    for (int w = 0; w < kActWarps; ++w) mbar_init(&zbar[w], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {  // TMA producer
+      int c = 0;
+      for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x)
+        for (int kt = 0; kt < KT; ++kt, ++c) {
+          const int s = c % STAGES;
+          if (!mbar_wait(&empty[s], ((uint32_t)(c / STAGES) & 1u) ^ 1u)) { ok = false; break; }
+          mbar_expect_tx(&full[s], (unsigned)((BM + BN) * BK * 2));
+          tma_load_2d(sA + (size_t)s * BM * BK * 2, &tmA, kt * BK, t / nt * BM, &full[s]);
+          tma_load_2d(sB + (size_t)s * BN * BK * 2, &tmB, kt * BK, t % nt * BN, &full[s]);
+        }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issuer
+      const uint32_t idesc = idesc_bf16<BN>(false);
+      int c = 0, it = 0;
+      for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x, ++it) {
+        const uint32_t acc_addr = tmem + (uint32_t)(it & 1) * BN;
+        if (!mbar_wait(&tempty[it & 1], ((uint32_t)(it >> 1) & 1u) ^ 1u)) { ok = false; break; }
+        tc_fence_after();
+        for (int kt = 0; kt < KT; ++kt, ++c) {
+          const int s = c % STAGES;
+          if (!mbar_wait(&full[s], (uint32_t)(c / STAGES) & 1u)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t ad = desc_sw128(sA + (size_t)s * BM * BK * 2), bd = desc_sw128(sB + (size_t)s * BN * BK * 2);
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk) mma_f16(acc_addr, ad + 2 * kk, bd + 2 * kk, idesc, (kt | kk) != 0);
+          mma_commit(&empty[s]);
+        }
+        mma_commit(&tfull[it & 1]);
+      }
+    }
+  } else {
+    const int e = warp - 2, set = e / (kActWarps / SETS), group = (e >> 2) % (BN / 64), quarter = warp & 3;
+    unsigned char* buf = stage + e * kStage;
+    uint64_t* zb = zbar + e;
+    const bool dact = g.epi == EPI_DACT;
+    auto load_z = [&](int t) {
+      mbar_expect_tx(zb, kStage);
+      tma_load_2d(buf, &tmZ, t % nt * BN + group * 64, t / nt * BM + quarter * 32, zb);
+    };
+    const int step = SETS * gridDim.x, t0 = blockIdx.x + set * gridDim.x;
+    if (dact && lane == 0 && t0 < ntiles) load_z(t0);
+    int h = 0;  // tiles of this warp
+    for (int t = t0; t < ntiles; t += step, ++h) {
+      const int it = h * SETS + set, col = t % nt * BN + group * 64, row0 = t / nt * BM + quarter * 32;
+      ok = mbar_wait(&tfull[it & 1], (uint32_t)(it >> 1) & 1u) && (!dact || mbar_wait(zb, (uint32_t)h & 1u));
+      ok = __all_sync(0xffffffffu, ok) != 0;  // the TMEM loads below are warp-collective
+      if (!ok) break;
+      tc_fence_after();
+      uint4 zp[8];  // EPI_ACT: pre-activations, staged after the outputs
+      if (!dact) {  // the last tile's stores have read the buffer (EPI_DACT: before its pre-activations were loaded)
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
+      }
+#pragma unroll
+      for (int hc = 0; hc < 2; ++hc) {
+        uint32_t v[32];
+        tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((it & 1) * BN + group * 64 + hc * 32), v);
+        if (hc == 1) {  // the accumulator is in registers
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[it & 1]);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {  // 16-byte pieces of the lane's row
+          const int off = lane * 128 + (((hc * 4 + p) ^ (lane & 7)) << 4);
+          uint4 out, zz;
+          unsigned* o = reinterpret_cast<unsigned*>(&out);
+          unsigned* z = reinterpret_cast<unsigned*>(&zz);
+          float4 b[2] = {};
+          if (dact) {
+            zz = *reinterpret_cast<const uint4*>(buf + off);
+          } else if (g.bias) {
+            b[0] = __ldg(reinterpret_cast<const float4*>(g.bias + col + hc * 32) + 2 * p);
+            b[1] = __ldg(reinterpret_cast<const float4*>(g.bias + col + hc * 32) + 2 * p + 1);
+          }
+          const float* bias = reinterpret_cast<const float*>(b);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int j = 8 * p + 2 * q;
+            if (dact) {
+              const float d0 = __uint_as_float(v[j]), d1 = __uint_as_float(v[j + 1]);
+              o[q] = g.act == ACT_SILU ? pack_bf16(d0 * dsilu(bf16_lo(z[q])), d1 * dsilu(bf16_hi(z[q]))) : pack_bf16(d0, d1);
+            } else {
+              const float z0 = __uint_as_float(v[j]) + bias[2 * q], z1 = __uint_as_float(v[j + 1]) + bias[2 * q + 1];
+              z[q] = pack_bf16(z0, z1);
+              o[q] = g.act == ACT_SILU ? pack_bf16(silu(z0), silu(z1)) : z[q];
+            }
+          }
+          *reinterpret_cast<uint4*>(buf + off) = out;
+          zp[hc * 4 + p] = zz;
+        }
+      }
+      proxy_fence();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tmO, col, row0, buf);
+        tma_store_commit();
+      }
+      if (!dact && g.z_out) {
+        if (lane == 0) tma_store_wait_read();
+        __syncwarp();
+#pragma unroll
+        for (int p = 0; p < 8; ++p) *reinterpret_cast<uint4*>(buf + lane * 128 + ((p ^ (lane & 7)) << 4)) = zp[p];
+        proxy_fence();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tmZ, col, row0, buf);
+          tma_store_commit();
+        }
+      }
+      if (dact && g.colsum) {  // columns col + 2 lane, + 1 (the store above only reads the tile)
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+          const unsigned u = *reinterpret_cast<const unsigned*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+          float2& a = (r & 1) ? s1 : s0;
+          a.x += bf16_lo(u);
+          a.y += bf16_hi(u);
+        }
+        atomicAdd(reinterpret_cast<float2*>(g.colsum + col) + lane, make_float2(s0.x + s1.x, s0.y + s1.y));
+      }
+      if (dact && t + step < ntiles) {  // the next tile's pre-activations, once this tile is read
+        __syncwarp();
+        if (lane == 0) { tma_store_wait_read(); load_z(t + step); }
+      }
+    }
+    if (lane == 0) tma_store_wait_read();  // shared memory is read; the writes are complete when the kernel is
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * BN) : "memory");
+  if (!ok) atomicExch(g.err, 1u);
+}
+
+template <int BN>
 __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                         const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmO,
-                                                         const __grid_constant__ CUtensorMap tmZ, GemmArgs g) {
+                                                         const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
   constexpr int STAGES = stages_for<BN>();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -258,8 +369,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   uint64_t* full = (uint64_t*)(sB + (size_t)STAGES * BN * BK * 2);
   uint64_t* empty = full + STAGES;
   uint64_t* done = empty + STAGES;
-  uint64_t* zbar = done + 1;  // one per warp (EPI_DACT pre-activation tiles)
-  uint32_t* tmem_slot = (uint32_t*)(zbar + 8);
+  uint32_t* tmem_slot = (uint32_t*)(done + 1);
   float* sbias = (float*)(tmem_slot + 4);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
@@ -270,7 +380,6 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(done, 1);
-    for (int w = 0; w < 8; ++w) mbar_init(&zbar[w], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int j = threadIdx.x; j < BN; j += kThreads) sbias[j] = (g.bias && n0 + j < g.n_valid) ? g.bias[n0 + j] : 0.0f;
@@ -292,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       unsigned char* a = sA + (size_t)s * BM * BK * 2;
       unsigned char* b = sB + (size_t)s * BN * BK * 2;
       const int k0 = (kt0 + kt) * BK;
-      if (!TS && g.rows_k) {
+      if (g.rows_k) {
         for (int i = 0; i < BM / 64; ++i) tma_load_2d(a + i * 8192, &tmA, m0 + i * 64, k0, &full[s]);
         for (int i = 0; i < BN / 64; ++i) tma_load_2d(b + i * 8192, &tmB, n0 + i * 64, k0, &full[s]);
       } else {
@@ -301,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       }
     }
   } else if (warp == 1 && lane == 0) {  // MMA issuer
-    const bool rows_k = !TS && g.rows_k;
+    const bool rows_k = g.rows_k;
     const uint32_t idesc = idesc_bf16<BN>(rows_k);
     const uint64_t kstep = rows_k ? 2048 >> 4 : 32 >> 4;  // 16 elements of K: 16 rows, or 32 B inside the swizzled row
     for (int kt = 0; kt < KT; ++kt) {
@@ -314,15 +423,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       const uint64_t ad = rows_k ? desc_sw128_rows_k(a) : desc_sw128(a), bd = rows_k ? desc_sw128_rows_k(b) : desc_sw128(b);
 #pragma unroll
       for (int kk = 0; kk < BK / 16; ++kk) {
-        const uint32_t acc = (kt | kk) != 0;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem),
-            "l"(ad + kstep * kk), "l"(bd + kstep * kk), "r"(idesc), "r"(acc)
-            : "memory");
+        mma_f16(tmem, ad + kstep * kk, bd + kstep * kk, idesc, (kt | kk) != 0);
       }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty[s])) : "memory");
+      mma_commit(&empty[s]);
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(done)) : "memory");
+    mma_commit(done);
   }
   __syncwarp();
   // epilogue: thread = tile row m0 + 32 (warp mod 4) + lane, columns of half warp / 4
@@ -331,9 +436,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   tc_fence_after();
   const int quarter = warp & 3, half = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
-  if constexpr (TS) {
-    if (ok) ok = epilogue_tma<BN>(g, &tmO, &tmZ, tmem, base, sbias, &zbar[warp], n0, m0, warp, lane);
-  } else if (ok) {
+  if (ok) {
 #pragma unroll 1
     for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
       uint32_t v[32];
