@@ -77,6 +77,7 @@ struct LatMem {
   double ctl[4 + kMaxT];
   int ctlf, accept;
   double tA[TB::S], tC[TB::S], td[TB::S];  // tableau: last A and C of each stage, d
+  double hd[TB::S];                        // h d of the step
   int tq[TB::S], tinc[TB::S];              // stage time set, incremental input
   CosmoDesc cdesc;
   int item;
@@ -536,21 +537,22 @@ __device__ void lat_emit(const LGrp& g, LatMem<NSL, ST>& W, const Rows<NSL>& R, 
 }
 
 // Step control as ptk::pt_body publishes it, in two parts: flags, h, 1/h and 1/(hγ) (what the solver warps
-// wait for; the divisions one per lane), then the step end and the stage times.  Returns the step end.
+// wait for; the divisions one per lane), then the step end and the stage times.  Returns the step end.  Each FP64
+// instruction of this chain is 65 cycles of every warp's wait: times are positive and compared as integers, and
+// left = tend - tc and tmin = 1e-14 tc come from the caller.
 template <int NSL, typename ST>
-__device__ __forceinline__ double lat_publish(int lane, LatMem<NSL, ST>& W, double& hp, double tc, double tend) {
+__device__ __forceinline__ double lat_publish(int lane, LatMem<NSL, ST>& W, double& hp, double tc, double tend, double left, double tmin) {
   // the divisions start before the clamp to the end point, which is rare, is decided
   double inv = 1.0 / (lane == 1 ? hp * TB::gam : hp);
-  const bool done = !(tc < tend);
-  const double left = tend - tc;
-  if (tc + 1.01 * hp >= tend) {
+  const bool done = dkey(tc) >= dkey(tend);
+  if (dkey(tc + 1.01 * hp) >= dkey(tend)) {
     hp = left;
     inv = 1.0 / (lane == 1 ? hp * TB::gam : hp);
   }
-  const bool tiny = !(hp > 1e-14 * tc);
+  const bool tiny = dkey(hp) <= dkey(tmin);
   if (lane == 0) { W.ctlf = (done ? 1 : 0) | (tiny ? 2 : 0); W.ctl[0] = hp; W.ctl[1] = inv; }
   if (lane == 1) W.ctl[2] = inv;
-  return (hp == left) ? tend : tc + hp;
+  return dkey(hp) == dkey(left) ? tend : tc + hp;
 }
 template <int NSL, typename ST>
 __device__ __forceinline__ void lat_publish_times(int lane, LatMem<NSL, ST>& W, double hp, double tc, double te) {
@@ -563,6 +565,7 @@ __device__ __forceinline__ void lat_publish_times(int lane, LatMem<NSL, ST>& W, 
     if (lane == 3 + q) c = TB::c(st);
   }
   const double ts = tc + c * hp;
+  if (lane < TB::S) W.hd[lane] = hp * W.td[lane];
   if (lane == 0) { W.ctl[3] = te; W.ctl[4 + TB::NTIME - 1] = te; }
   if (lane >= 4 && lane < 4 + TB::NTIME - 1) W.ctl[lane] = ts;
 }
@@ -654,7 +657,7 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) if (R.i[sl] < n) W.x[R.i[sl]] = y[sl];
     if (g.wq == 1) {
-      const double te = lat_publish(g.lane, W, h, t, tend);
+      const double te = lat_publish(g.lane, W, h, t, tend, tend - t, 1e-14 * t);
       lat_publish_times(g.lane, W, h, t, te);
     }
     bool nonfinite = false, moved = false;  // moved: y is new since f0 and ft were formed
@@ -690,12 +693,12 @@ __device__ void lat_solver(const PtArgs& A, const ModelDesc& M, const CompDesc* 
       for (int st = 0; st < nst; ++st) {
         if (st == 0) {
 #pragma unroll
-          for (int sl = 0; sl < NSL; ++sl) b[sl] = fma(h * TB::d(0), ft[sl], f0[sl]);
+          for (int sl = 0; sl < NSL; ++sl) b[sl] = fma(W.hd[0], ft[sl], f0[sl]);
         } else {
           double cu[NSL];
           const double ka = W.tA[st], kc = W.tC[st], kd = W.td[st];
           const int kq = W.tq[st], kinc = W.tinc[st];
-          const double hdst = h * kd;
+          const double hdst = W.hd[st];
           if (st == 1) {
 #pragma unroll
             for (int sl = 0; sl < NSL; ++sl) { Y[sl] = fma(ka, Ul[sl], y[sl]); cu[sl] = kc * Ul[sl]; }
@@ -923,17 +926,20 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
   double tn = t;
   int sJ = 0, sE = TB::NTIME;
   int64_t iters = 0;
-  int ci[NSL], si[NSL];  // rows in the error norm (its sum's order) and in the stage sums (slot 1 on warp 3)
-  double y[NSL], y1[NSL], ys = 0, ys1 = 0;  // state rows of ci, and of si[1]
+  // rows in the error norm (its sum's order) and in the stage sums: slot 1 on warp 3, and with two warps of rows
+  // those of warp 0 on warp 2, whose sub-partition's solver warp has none (warp 0's has the head rows)
+  int ci[NSL], si[NSL];
+  double y[NSL], y1[NSL], ys[NSL], ys1[NSL];  // state rows of ci and si
 #pragma unroll
   for (int sl = 0; sl < NSL; ++sl) { ci[sl] = comp_of<4>(gt, sl); si[sl] = sl * kSolvers + ((gt + 32 * sl) & (kSolvers - 1)); }
+  if (n <= 64 && (g.wq & 1) == 0) si[0] = gt ^ 64;
+  const int nw = n > 96 ? 4 : (n + 31) / 32;  // warps with rows in the error norm
   bool act[NSL];
 #pragma unroll
   for (int sl = 0; sl < NSL; ++sl) act[sl] = __any_sync(FULL, si[sl] < n);
   bar_sync(LB_STEP, kLatThreads);
 #pragma unroll
-  for (int sl = 0; sl < NSL; ++sl) y[sl] = ci[sl] < n ? W.x[ci[sl]] : 0.0;
-  if (NSL > 1) ys = si[NSL - 1] < n ? W.x[si[NSL - 1]] : 0.0;
+  for (int sl = 0; sl < NSL; ++sl) { y[sl] = ci[sl] < n ? W.x[ci[sl]] : 0.0; ys[sl] = si[sl] < n ? W.x[si[sl]] : 0.0; }
   for (;;) {
     if (first && g.wq == 3) bar_arrive(LB_CTL, kSolvers + 32);  // the first step's control is the solvers'
     bar_sync(LB_COMP, kSolvers);  // control seen by every companion warp
@@ -944,8 +950,7 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
       } else {
         t = tn;
 #pragma unroll
-        for (int sl = 0; sl < NSL; ++sl) y[sl] = y1[sl];
-        ys = ys1;
+        for (int sl = 0; sl < NSL; ++sl) { y[sl] = y1[sl]; ys[sl] = ys1[sl]; }
         const int tsw = sJ; sJ = sE; sE = tsw;
       }
     }
@@ -974,7 +979,7 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) a[q][sl] = sl == 0 ? y[sl] : ys;
+      for (int q = 0; q < 4; ++q) a[q][sl] = ys[sl];
 #pragma unroll
       for (int q = 0; q < 6; ++q) c[q][sl] = 0;
     }
@@ -1005,10 +1010,10 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
     // FP64 error norm of the last stage
     bar_sync(LB_STEP, kLatThreads);
     double e2 = 0;
-    if (NSL > 1) ys1 = si[NSL - 1] < n ? W.x[si[NSL - 1]] : 0.0;
 #pragma unroll
     for (int sl = 0; sl < NSL; ++sl) {
       const int i = ci[sl];
+      ys1[sl] = si[sl] < n ? W.x[si[sl]] : 0.0;
       if (i < n) {
         y1[sl] = W.x[i];
         const double ul = W.Us[TB::S - 1][i];
@@ -1023,10 +1028,10 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
     if (g.wq < 3) {
       bar_arrive(LB_ERR, kSolvers);
     } else {  // step control
+      double left = tend - tn, tmin = 1e-14 * tn;  // of an accepted step, before the wait
       bar_sync(LB_ERR, kSolvers);
-      double err2 = 0;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) err2 += W.rede[w];
+      double err2 = W.rede[0];
+      for (int w = 1; w < nw; ++w) err2 += W.rede[w];  // the others are zero
       err2 *= inv_n;  // squared RMS error norm
       // err2 >= 0: accepted when finite and at most 1, by its bit pattern (inf, NaN and any sign-bit
       // pattern compare above 1 as unsigned)
@@ -1047,7 +1052,8 @@ __device__ void lat_companion(const PtArgs& A, const ModelDesc& M, LatMem<NSL, S
       }
       if (g.lane == 0) W.accept = ok ? 1 : nonfinite ? 2 : 0;
       const double tc = ok ? tn : t;
-      const double te = lat_publish(g.lane, W, hp, tc, tend);
+      if (!ok) { left = tend - t; tmin = 1e-14 * t; }
+      const double te = lat_publish(g.lane, W, hp, tc, tend, left, tmin);
       __syncwarp();
       bar_arrive(LB_CTL, kSolvers + 32);
       lat_publish_times(g.lane, W, hp, tc, te);
