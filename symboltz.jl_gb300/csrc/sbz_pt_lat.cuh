@@ -98,7 +98,8 @@ __device__ __forceinline__ int lat_comp(int gt, int s) { return s * kSolvers + (
 template <int NSL>
 struct Rows {
   double A[NSL], C[NSL];
-  int i[NSL], ip[NSL], in[NSL], sp[NSL], dg[NSL], phid[NSL], psid[NSL];
+  int i[NSL], ip[NSL], in[NSL], sp[NSL], dg[NSL];
+  int fd[NSL], fx[NSL];  // coupling to the metric functionals: coefficient, and 0 for Ψ or 1 for Φ̇ (no row has both)
   int e0, e0c, e1, e1c, e3, e3a, e3b;  // head rows (slot 0): cv[e0] x[e0c] + cv[e1] x[e1c] + cv[e3] (x[e3a] - (3k/4) x[e3b])
   bool extra;
 };
@@ -113,7 +114,8 @@ __device__ __forceinline__ Rows<NSL> load_rows(const LGrp& g, const ModelDesc& M
     R.i[s] = i;
     R.A[s] = on ? D.A : 0.0; R.C[s] = on ? D.C : 0.0;
     R.ip[s] = on ? D.ip : M.n; R.in[s] = on ? D.inx : M.n;
-    R.sp[s] = on ? D.sp : 0; R.dg[s] = on ? D.dg : 0; R.phid[s] = on ? D.phid : 0; R.psid[s] = on ? D.psid : 0;
+    R.sp[s] = on ? D.sp : 0; R.dg[s] = on ? D.dg : 0; 
+    R.fx[s] = on && D.psid != CV_ZERO ? 0 : 1; R.fd[s] = on ? (R.fx[s] ? D.phid : D.psid) : 0;
   }
   const CompDesc& D = comps[R.i[0] < M.n ? R.i[0] : 0];
   R.extra = g.gt < 32;
@@ -157,14 +159,14 @@ __device__ __forceinline__ void lat_coef1(const LGrp& g, LatMem<NSL, ST>& W, CSe
 }
 
 // Ψ(v) and the δρ sum, as ptk::functionals with the butterfly started at the distance the model's
-// terms need (the skipped levels only add zeros).
+// terms need (the skipped levels only add zeros); valid on lane 0.
 __device__ __forceinline__ void lat_functionals(const LGrp& g, const double* v, const double* w, double& psi, double& rho) {
   double t = w[g.lane] * v[g.fc];
 #pragma unroll
   for (int o = 8; o; o >>= 1)
     if (o <= g.ftop) t += __shfl_xor_sync(FULL, t, o);
-  psi = __shfl_sync(FULL, t, 0);
-  rho = __shfl_sync(FULL, t, 16);
+  psi = t;
+  rho = __shfl_down_sync(FULL, t, 16);
 }
 
 // Metric functionals as every thread that uses them sees them.
@@ -216,16 +218,18 @@ __device__ __forceinline__ Fun lat_matvec(const LGrp& g, LatMem<NSL, ST>& W, con
     if (DT) dout[s] = d;
   }
   if (uses) {
-    if (!isf) {
-      bar_sync(LB_FUN, kSolvers);
+    if (!isf) bar_sync(LB_FUN, kSolvers);
+    if (want) {
       F.psi = W.fun[0]; F.phd = W.fun[1];
       if (DT) { F.dpsi = W.fun[2]; F.dphd = W.fun[3]; }
     }
 #pragma unroll
     for (int s = 0; s < NSL; ++s)
       if ((g.pp >> s) & 1u) {
-        out[s] += cv[R.phid[s]] * F.phd + cv[R.psid[s]] * F.psi;
-        if (DT) dout[s] += cvd[R.phid[s]] * F.phd + cv[R.phid[s]] * F.dphd + cvd[R.psid[s]] * F.psi + cv[R.psid[s]] * F.dpsi;
+        // one product per row (the generic kernel's other one has a zero coefficient), rounded by itself as there
+        const double v = W.fun[R.fx[s]], c = cv[R.fd[s]];
+        out[s] = __dadd_rn(out[s], __dmul_rn(c, v));
+        if (DT) dout[s] = __dadd_rn(dout[s], fma(c, W.fun[2 + R.fx[s]], __dmul_rn(cvd[R.fd[s]], v)));
       }
   }
   if (DT && DSRC && R.extra) {
@@ -375,8 +379,9 @@ __device__ __forceinline__ void lat_factor_inputs(const LGrp& g, LatMem<NSL, ST>
       const double spv = cv[R.sp[sl]];
       W.sup[i] = to_st<ST>(-spv * R.C[sl]);
       W.sub[i] = to_st<ST>(-spv * R.A[sl]);
-      W.Z1[i] = to_st<ST>(cv[R.phid[sl]]);
-      W.Z2[i] = to_st<ST>(cv[R.psid[sl]]);
+      const ST c = to_st<ST>(cv[R.fd[sl]]);
+      W.Z1[i] = R.fx[sl] ? c : ST(0);
+      W.Z2[i] = R.fx[sl] ? ST(0) : c;
     }
   }
   F.wS = to_st<ST>(C.w[g.lane]);

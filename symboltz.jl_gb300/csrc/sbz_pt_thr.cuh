@@ -103,7 +103,7 @@ template <int G>
 __device__ __forceinline__ int thr_comp(int gt, int s) { return s * 32 * G + ((gt + (G == 2 ? 32 : 64) * s) & (32 * G - 1)); }
 
 template <int NSL>
-struct TRows {  // indices packed: ip | in << 8 | sp << 16 | dg << 24, phid | psid << 8 | at << 16
+struct TRows {  // indices packed: ip | in << 8 | sp << 16 | dg << 24, coupling to the metric functionals (coefficient | (0: Ψ, 1: Φ̇) << 8) | at << 16
   double A[NSL], C[NSL];
   unsigned a[NSL], b[NSL];
   unsigned ea, eb;  // head rows' extra terms: e0 | e0c << 8 | e1 << 16 | e1c << 24, e3 | e3a << 8 | e3b << 16
@@ -122,8 +122,8 @@ __device__ __forceinline__ Fun thr_matvec(const TGrp<G>& g, const ThrMem<ST>& W,
 #pragma unroll
       for (int o = 8; o; o >>= 1)
         if (o <= g.ftop) t += __shfl_xor_sync(FULL, t, o);
-      psi = __shfl_sync(FULL, t, 0);
-      rho = __shfl_sync(FULL, t, 16);
+      psi = t;  // valid on lane 0
+      rho = __shfl_down_sync(FULL, t, 16);
     };
     double rho, drho = 0;
     sum(C.w, F.psi, rho);
@@ -158,17 +158,18 @@ __device__ __forceinline__ Fun thr_matvec(const TGrp<G>& g, const ThrMem<ST>& W,
     out[s] = o;
     if (DT) dout[s] = d;
   }
-  if (uses && g.wq != g.fw) {
-    bar_sync(g.bar + 1, 32 * G);
+  if (uses && g.wq != g.fw) bar_sync(g.bar + 1, 32 * G);
+  if (want && g.wq == 0) {
     F.psi = W.s->fun[0]; F.phd = W.s->fun[1];
     if (DT) { F.dpsi = W.s->fun[2]; F.dphd = W.s->fun[3]; }
   }
 #pragma unroll
   for (int s = 0; s < NSL; ++s)
-    if ((g.pp >> s) & 1u) {
-      const int ph = R.b[s] & 255, ps = (R.b[s] >> 8) & 255;
-      out[s] += cv[ph] * F.phd + cv[ps] * F.psi;
-      if (DT) dout[s] += cvd[ph] * F.phd + cv[ph] * F.dphd + cvd[ps] * F.psi + cv[ps] * F.dpsi;
+    if ((g.pp >> s) & 1u) {  // see lat_matvec
+      const int fd = R.b[s] & 255, fx = (R.b[s] >> 8) & 1;
+      const double v = W.s->fun[fx], c = cv[fd];
+      out[s] = __dadd_rn(out[s], __dmul_rn(c, v));
+      if (DT) dout[s] = __dadd_rn(dout[s], fma(c, W.s->fun[2 + fx], __dmul_rn(cvd[fd], v)));
     }
   if (DT && DSRC && g.wq == 0) {
     const unsigned ea = R.ea, eb = R.eb;
@@ -317,8 +318,9 @@ __device__ __forceinline__ void thr_factorize(const TGrp<G>& g, const ThrMem<ST>
       W.dd[i] = to_st<ST>(s - cv[a >> 24]);
       W.sup[i] = to_st<ST>(-spv * R.C[sl]);
       W.sub[i] = to_st<ST>(-spv * R.A[sl]);
-      W.Z1[i] = to_st<ST>(cv[b & 255]);
-      W.Z2[i] = to_st<ST>(cv[(b >> 8) & 255]);
+      const ST c = to_st<ST>(cv[b & 255]);
+      W.Z1[i] = (b >> 8) & 1 ? c : ST(0);
+      W.Z2[i] = (b >> 8) & 1 ? ST(0) : c;
     }
   }
   if (g.wq == 0) W.s->wS[lane] = to_st<ST>(C.w[lane]);
@@ -880,7 +882,8 @@ __global__ void __launch_bounds__(NT, MINB) pt_thr_kernel(PtArgs A) {
     int at = 0;
     for (int c = 0; c < 2; ++c) if (i >= M.chFirst[c] && i <= M.chLast[c]) at = M.chAttach[c];
     R.a[s] = on ? (unsigned)D.ip | (unsigned)D.inx << 8 | (unsigned)D.sp << 16 | (unsigned)D.dg << 24 : (unsigned)n | (unsigned)n << 8;
-    R.b[s] = on ? (unsigned)D.phid | (unsigned)D.psid << 8 | (unsigned)at << 16 : 0u;
+    const unsigned fx = D.psid != CV_ZERO ? 0u : 1u;  // no row has both couplings
+    R.b[s] = on ? (unsigned)(fx ? D.phid : D.psid) | fx << 8 | (unsigned)at << 16 : 0u;
     if (__any_sync(FULL, on)) g.act |= 1u << s;
     if (__any_sync(FULL, on && (D.phid != CV_ZERO || D.psid != CV_ZERO))) g.pp |= 1u << s;
   }
