@@ -393,11 +393,29 @@ static void pt_model_args(const sbz_problem* pb, sbz::PtArgs& A) {
   A.table_stride = pb->table_stride;
 }
 
-static int pt_run(sbz_problem* pb, int nk, const int* d_cosmo, const double* d_ks, const double* d_ti, const int* d_order,
+// Expected work of a launch in units of its longest mode, for the number of modes that share an SM (see
+// thr_modes_per_sm); ks on the host.  Steps of a mode ∝ a + A ln(1 + k/A) with k in H0/c: the evolution that every
+// mode has, then its oscillations, of which a loose tolerance resolves fewer at high k.  A = 180 and a = 14.5 at
+// atol 1e-5, A growing as 1/atol and a as its cube root, give the mean over the longest of the models measured (k from
+// 1e-4 to 0.02 .. 1 h/Mpc): 0.38, 0.24, 0.23, 0.23 where 0.35, 0.22, 0.23, 0.23 was found at 1e-5, 0.21 (0.21) at 1e-6
+// and 0.19 (0.19) at 3e-8.  Saved times come with an
+// early start (about 55 steps) and cost a third of a step each.
+static double pt_load(const sbz_problem* pb, const double* ks, int nk, int ntau) {
+  const double x = 1e-5 / std::max(pb->opts.pt_atol, 1e-12), A = 180 * x, a = 14.5 * std::cbrt(x) + (ntau > 0 ? 10 + 0.06 * ntau : 0);
+  double sum = 0, top = 0;
+  for (int i = 0; i < nk; ++i) {
+    const double v = a + A * std::log1p(ks[i] / A);
+    sum += v;
+    if (v > top) top = v;
+  }
+  return top > 0 ? sum / top : 0;
+}
+
+static int pt_run(sbz_problem* pb, int nk, double load, const int* d_cosmo, const double* d_ks, const double* d_ti, const int* d_order,
                   int ntau, const double* d_taus, int output, double* d_out, int* d_status, int64_t* d_steps) {
   sbz::PtArgs A{};
   pt_model_args(pb, A);
-  A.item_cosmo = d_cosmo; A.item_k = d_ks; A.item_tau_ini = d_ti; A.order = d_order; A.nitems = nk;
+  A.item_cosmo = d_cosmo; A.item_k = d_ks; A.item_tau_ini = d_ti; A.order = d_order; A.nitems = nk; A.load = load;
   A.taus = ntau > 0 ? d_taus : nullptr; A.ntau = ntau;
   A.output = output; A.out = d_out; A.status = d_status; A.steps = d_steps;
   A.rtol = pb->opts.pt_rtol; A.atol = pb->opts.pt_atol; A.maxiters = pb->opts.maxiters;
@@ -455,7 +473,7 @@ int sbz_solve_pt_device(sbz_problem* pb, int nk, const int* cosmo, const double*
                         const double* taus, int output, double* out, int* status, int64_t* steps) {
   if (!check_pt_args(pb, nk, ntau, output)) return SBZ_ERR_ARG;
   if (nk == 0) return SBZ_OK;
-  return pt_run(pb, nk, cosmo, ks, tau_ini, nullptr, ntau, taus, output, out, status, steps);
+  return pt_run(pb, nk, 0.0, cosmo, ks, tau_ini, nullptr, ntau, taus, output, out, status, steps);
 }
 
 int sbz_solve_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks, const double* tau_ini, int ntau,
@@ -490,7 +508,7 @@ int sbz_solve_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks, co
   SBZ_CUDA(cudaMemcpyAsync(pb->d_cosmo.p, cos.data(), sizeof(int) * nk, cudaMemcpyHostToDevice, st));
   SBZ_CUDA(cudaMemcpyAsync(pb->d_order.p, order.data(), sizeof(int) * nk, cudaMemcpyHostToDevice, st));
   if (ntau > 0) SBZ_CUDA(cudaMemcpyAsync(pb->d_taus.p, taus, sizeof(double) * ntau * pb->ncosmo, cudaMemcpyHostToDevice, st));
-  int r = pt_run(pb, nk, pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
+  int r = pt_run(pb, nk, pt_load(pb, ks, nk, ntau), pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
                  pb->d_taus.as<double>(), output, pb->d_out.as<double>(), pb->d_status.as<int>(), pb->d_steps.as<int64_t>());
   if (r != SBZ_OK) return r;
   if (out) SBZ_CUDA(cudaMemcpyAsync(out, pb->d_out.p, sizeof(double) * nout, cudaMemcpyDeviceToHost, st));
@@ -547,7 +565,7 @@ int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks,
     pb->opts.warps_per_mode = cand[c][0];
     pb->opts.blocks_per_sm = cand[c][1];
     SBZ_CUDA(cudaEventRecord(pb->ev[8], s));
-    r = pt_run(pb, ns, pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
+    r = pt_run(pb, ns, pt_load(pb, sk.data(), ns, ntau), pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
                pb->d_taus.as<double>(), output, pb->d_out.as<double>(), pb->d_status.as<int>(), pb->d_steps.as<int64_t>());
     if (r != SBZ_OK) { pb->opts.warps_per_mode = keep_nw; pb->opts.blocks_per_sm = keep_bps; return r; }
     SBZ_CUDA(cudaEventRecord(pb->ev[9], s));
@@ -723,7 +741,7 @@ static int spectrum_cmb_impl(sbz_problem* pb, int cosmo, const sbz_bessel* jl, i
     sbz::PtArgs A{};
     pt_model_args(pb, A);
     A.item_cosmo = pb->d_cosmo.as<int>(); A.item_k = pb->d_k.as<double>(); A.item_tau_ini = pb->d_ti.as<double>();
-    A.order = pb->d_order.as<int>(); A.nitems = nc;
+    A.order = pb->d_order.as<int>(); A.nitems = nc; A.load = pt_load(pb, ks_coarse, nc, ntau);
     A.taus = pb->d_taus.as<double>(); A.ntau = ntau; A.output = SBZ_OUT_SOURCES;
     A.out = pb->d_out.as<double>(); A.status = pb->d_status.as<int>(); A.steps = pb->d_steps.as<int64_t>();
     A.rtol = pb->opts.pt_rtol; A.atol = pb->opts.pt_atol; A.maxiters = pb->opts.maxiters;

@@ -30,13 +30,13 @@ def _sms():
     return torch.cuda.get_device_properties(0).multi_processor_count
 
 
-def _solve(S, model, per_sm, output="delta_m", taus=None, **kw):
+def _solve(S, model, per_sm, output="delta_m", taus=None, kmax=15.0, **kw):
     """per_sm modes per SM (one more than a multiple) of three cosmologies, 40 of them distinct in k."""
     M = S.ΛCDM(**model)
     base = S.parameters_Planck18(M)
     p = S.CosmologyProblem(M, [dict(base, h=0.66 + 0.01 * i) for i in range(3)], **kw)
     n = per_sm * _sms() - 3
-    ks = np.geomspace(0.3, 15.0, 40)[np.arange(n) % 40]
+    ks = np.geomspace(0.3, kmax, 40)[np.arange(n) % 40]
     cos = np.arange(n) % 3
     if taus is not None:
         bg = p.solvebg()
@@ -62,6 +62,13 @@ def _check(a, b, exact=True):
 @pytest.mark.parametrize("model", ["n47", "n129"])
 def test_same_bits_as_the_generic_kernel(S, model, per_sm, generic):
     _check(_solve(S, MODELS[model], per_sm), _solve(S, MODELS[model], per_sm, **generic))
+
+
+# modes of far different lengths: fewer share an SM (one to four at these counts)
+@pytest.mark.parametrize("per_sm", [4, 7, 10, 17])
+@pytest.mark.parametrize("model", ["n47", "n129"])
+def test_far_apart_lengths(S, model, per_sm):
+    _check(_solve(S, MODELS[model], per_sm, kmax=300.0), _solve(S, MODELS[model], per_sm, kmax=300.0, warps_per_mode=4, blocks_per_sm=2))
 
 
 @pytest.mark.parametrize("per_sm", [9, 33])
