@@ -10,8 +10,9 @@ pytestmark = pytest.mark.gpu
 
 
 # N picks the tile (256, 128 or 64 columns; only the first two have the shared-memory route), K = 64 is one
-# pipeline step, N / 8 is odd in units of the staging groups at 384 and 640
-@pytest.mark.parametrize("M,N,K", [(128, 128, 64), (384, 256, 192), (128, 384, 128), (256, 512, 64), (128, 640, 320), (128, 192, 64)])
+# pipeline step; the last three have several tiles per CTA
+@pytest.mark.parametrize("M,N,K", [(128, 128, 64), (384, 256, 192), (128, 384, 128), (256, 512, 64), (128, 640, 320), (128, 192, 64),
+                                   (41216, 256, 64), (41216, 128, 192), (41088, 256, 128)])
 @pytest.mark.parametrize("act", [0, 1])
 def test_shared_memory_epilogue_has_the_register_epilogue_s_bits(M, N, K, act):
     torch = pytest.importorskip("torch")
