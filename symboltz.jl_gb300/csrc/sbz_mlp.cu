@@ -27,14 +27,14 @@ bool get_encode() {
   return true;
 }
 
-// 2-D tensor map of a bf16 [rows][cols] row-major matrix (row stride ld elements), box box_cols x box_rows,
+// 2-D tensor map of a bf16 (or FP32) [rows][cols] row-major matrix (row stride ld elements), box box_cols x box_rows,
 // 128-byte swizzle
-bool tmap(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_cols, int box_rows) {
+bool tmap(CUtensorMap* tm, const void* ptr, int rows, int cols, int ld, int box_cols, int box_rows, bool f32 = false) {
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
   const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
   const cuuint32_t es[2] = {1, 1};
-  return g_encode(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+  return g_encode(tm, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 // operand [rows][cols] without padding, box 64 x box_rows
@@ -84,7 +84,7 @@ int launch_act(const GemmArgs& g, const void* A, const void* B, cudaStream_t st)
 }
 
 template <int BN>
-int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
+int launch(GemmArgs g, const void* A, const void* B, cudaStream_t st) {
   if constexpr (BN >= 128)
     if (act_tiles(g, BN)) return launch_act<BN>(g, A, B, st);
   if (g.colsum) return SBZ_ERR_ARG;  // only gemm_act_kernel forms column sums
@@ -97,12 +97,15 @@ int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   if (splits > 1 && !g.accumulate &&
       cudaMemset2DAsync(g.out_f32, sizeof(float) * (size_t)g.ldo, 0, sizeof(float) * (size_t)g.n_valid, (size_t)g.M, st) != cudaSuccess)
     return SBZ_ERR_CUDA;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, td;
   if (g.rows_k) {  // [K][M], [K][N] in pieces of 64 x 64
     if (!tmap_operand(&ta, A, g.K, g.M, BK) || !tmap_operand(&tb, B, g.K, g.N, BK)) return SBZ_ERR_CUDA;
   } else if (!tmap_operand(&ta, A, g.M, g.K, BM) || !tmap_operand(&tb, B, g.N, g.K, BN)) {
     return SBZ_ERR_CUDA;
   }
+  td = ta;
+  g.tma_add = splits > 1 && g.n_valid == g.N && g.ldo % 4 == 0 && g.ldo >= g.N && aligned16(g.out_f32);  // else atomics from registers
+  if (g.tma_add && !tmap(&td, g.out_f32, g.M, g.N, g.ldo, 32, 32, true)) return SBZ_ERR_CUDA;
   const size_t smem = gemm_smem_bytes<BN>();
   auto k = gemm_tn_kernel<BN>;
   static bool attr_set = false;  // set once, outside any stream capture of a later call
@@ -110,7 +113,7 @@ int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
     attr_set = true;
   }
-  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, g);
+  k<<<dim3(g.N / BN, g.M / BM, splits), kThreads, smem, st>>>(ta, tb, td, g);
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : SBZ_ERR_CUDA;
 }
 

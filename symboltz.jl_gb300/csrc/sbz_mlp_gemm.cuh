@@ -43,6 +43,7 @@ struct GemmArgs {
   __nv_bfloat16* z_out;         // EPI_ACT: pre-activation (ldo stride), may be null
   const __nv_bfloat16* z_in;    // EPI_DACT: pre-activation of this layer (ldo stride)
   int rows_k;                   // operands are [K][M] and [K][N] (EPI_F32)
+  int tma_add;                  // EPI_F32: the tile is added to the output by TMA
   float* colsum;                // EPI_DACT: colsum[col] += Σ_rows out (as stored, bf16-rounded; 8-byte aligned); may be null
   unsigned* err;                // set to 1 by a CTA whose pipeline wait ran out
 };
@@ -151,6 +152,12 @@ __device__ __forceinline__ float bf16_hi(unsigned u) { return __uint_as_float(u 
 
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, int x, int y, const void* src) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(tm)),
+               "r"(x), "r"(y), "r"(smem_u32(src))
+               : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* tm, int x, int y, const void* src) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                   reinterpret_cast<uint64_t>(tm)),
                "r"(x), "r"(y), "r"(smem_u32(src))
                : "memory");
 }
@@ -360,7 +367,8 @@ __global__ void __launch_bounds__(kActThreads, 1) gemm_act_kernel(const __grid_c
 
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_constant__ CUtensorMap tmA,
-                                                         const __grid_constant__ CUtensorMap tmB, GemmArgs g) {
+                                                         const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmD,
+                                                         GemmArgs g) {
   constexpr int STAGES = stages_for<BN>();
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -436,7 +444,30 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   tc_fence_after();
   const int quarter = warp & 3, half = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
-  if (ok) {
+  if (ok && g.tma_add) {
+    // split K: 32 x 32 tiles staged in the operand ring (12 KB per warp, three buffers; rows of 128 bytes,
+    // 128-byte swizzle) and added by TMA.  16-byte atomics straight from the lanes' rows touched half a sector
+    // each: ADDFIG
+    unsigned char* buf = base + warp * 12288;
+    int q = 0;
+#pragma unroll 1
+    for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32, ++q) {
+      uint32_t v[32];
+      tmem_load32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+      unsigned char* b = buf + q % 3 * 4096;
+      if (q >= 3) {
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 2;" ::: "memory");
+        __syncwarp();
+      }
+#pragma unroll
+      for (int p = 0; p < 8; ++p) *reinterpret_cast<uint4*>(b + lane * 128 + ((p ^ (lane & 7)) << 4)) = make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
+      proxy_fence();
+      __syncwarp();
+      if (lane == 0) { tma_add_2d(&tmD, n0 + c0, m0 + quarter * 32, b); tma_store_commit(); }
+    }
+    if (lane == 0) tma_store_wait_read();
+    __syncwarp();
+  } else if (ok) {
 #pragma unroll 1
     for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 32) {
       uint32_t v[32];

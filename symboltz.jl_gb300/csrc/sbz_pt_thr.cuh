@@ -16,7 +16,7 @@
 // PtArgs::norm_warps), so the results are the same bit for bit in mixed precision.
 //
 // Modes per SM: the more, the better the FP64 pipes are used and the slower each mode, so a launch takes as
-// many as its slowest modes allow (thr_modes_per_sm in sbz_pt.cu).  16 cosmologies, k to 0.2 h/Mpc, default
+// many as its longest modes allow (thr_modes_per_sm in sbz_pt.cu).  16 cosmologies, k to 0.2 h/Mpc, default
 // tolerances, ms (the generic kernel's shape for the launch / 2 / 3 / 4 / 8 modes per SM here):
 //   n = 47   1,328 modes 69.5 / 56.8 / 61.7   2,400 122 / - / 72.0 / 77.4   4,800 237 / - / - / 136 / 115
 //   n = 133  1,328 modes 79.5 / 78.3 / 85.3   2,400 140 / - / 103 / 104     4,800 276 / - / - / 187 / 183

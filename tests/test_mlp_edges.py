@@ -43,6 +43,27 @@ def test_shared_memory_epilogue_has_the_register_epilogue_s_bits(M, N, K, act):
     torch.testing.assert_close(res[N + 8][1].float(), ref, rtol=2.0 ** -8, atol=1e-5 * K)
 
 
+# split K: partial tiles added by TMA (16-byte output rows) or by atomics (ldo = N + 2), in every tile width
+@pytest.mark.parametrize("M,N,K", [(128, 64, 512), (128, 128, 4096), (256, 256, 8192), (128, 192, 2048)])
+@pytest.mark.parametrize("pad", [0, 4, 2])
+def test_split_k_sums(M, N, K, pad):
+    torch = pytest.importorskip("torch")
+    from symboltz import _lib
+    L = _lib.lib()
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    A = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
+    B = torch.randn(N, K, device="cuda", generator=g).to(torch.bfloat16)
+    ref = A.double() @ B.double().T
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    out = torch.full((M, N + pad), 3.0, device="cuda")
+    for acc in (0, 1):
+        assert L.sbz_mlp_gemm(M, N, K, p(A), p(B), 0, 0, None, p(out), N + pad, 0, acc, None, None, st) == 0
+        # FP32 sums of K products of order 1: K^(1/2) terms of one rounding (2^-24 of a partial sum of K^(1/2)) and margin
+        torch.testing.assert_close(out[:, :N].double(), (1 + acc) * ref, rtol=0, atol=1e-6 * K * (1 + acc))
+        assert (out[:, N:] == 3.0).all()
+
+
 # widths of both tile sizes, odd input and output counts, batches of one and several row tiles; the gradient
 # batch is smaller than the training batch (other strides in the same buffers), and comes after training steps
 # (weights and their transposed copies as the optimiser left them)
