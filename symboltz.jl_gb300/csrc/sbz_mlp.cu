@@ -10,6 +10,8 @@ namespace sbz {
 int capi_fail(int code, const char* msg);
 
 namespace mlp {
+int gemm_splits(int M, int N, int K);
+
 namespace {
 
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
@@ -84,17 +86,14 @@ int launch_act(const GemmArgs& g, const void* A, const void* B, cudaStream_t st)
 }
 
 template <int BN>
-int launch(GemmArgs g, const void* A, const void* B, cudaStream_t st) {
+int launch(const GemmArgs& g, const void* A, const void* B, cudaStream_t st) {
   if constexpr (BN >= 128)
     if (act_tiles(g, BN)) return launch_act<BN>(g, A, B, st);
-  if (g.colsum) return SBZ_ERR_ARG;  // only gemm_act_kernel forms column sums
-  const int tiles = (g.N / BN) * (g.M / BM), KT = g.K / BK;
-  // weight gradients have few output tiles and a long K (the batch): split K over about two CTAs
-  // per SM, at least 4 K-steps each, and add the partial tiles atomically into a zeroed output
-  int splits = 1;
-  if (g.epi == EPI_F32 && tiles < 2 * num_sms()) splits = std::max(1, std::min(KT / 4, 2 * num_sms() / tiles));
-  // one 2-D fill of the output region (its rows may be longer than n_valid)
-  if (splits > 1 && !g.accumulate &&
+  if (g.colpart) return SBZ_ERR_ARG;  // only gemm_act_kernel forms column sums
+  int splits = g.epi == EPI_F32 ? gemm_splits(g.M, g.N, g.K) : 1;
+  if (!g.part && g.max_splits > 0) splits = std::min(splits, g.max_splits);
+  // partial tiles are added atomically into a zeroed output: one 2-D fill of its region (its rows may be longer than n_valid)
+  if (splits > 1 && !g.part && !g.accumulate &&
       cudaMemset2DAsync(g.out_f32, sizeof(float) * (size_t)g.ldo, 0, sizeof(float) * (size_t)g.n_valid, (size_t)g.M, st) != cudaSuccess)
     return SBZ_ERR_CUDA;
   CUtensorMap ta, tb, td;
@@ -104,8 +103,7 @@ int launch(GemmArgs g, const void* A, const void* B, cudaStream_t st) {
     return SBZ_ERR_CUDA;
   }
   td = ta;
-  g.tma_add = splits > 1 && g.n_valid == g.N && g.ldo % 4 == 0 && g.ldo >= g.N && aligned16(g.out_f32);  // else atomics from registers
-  if (g.tma_add && !tmap(&td, g.out_f32, g.M, g.N, g.ldo, 32, 32, true)) return SBZ_ERR_CUDA;
+  if (g.part && !tmap(&td, g.part, splits * g.M, g.N, g.N, 32, 32, true)) return SBZ_ERR_CUDA;
   const size_t smem = gemm_smem_bytes<BN>();
   auto k = gemm_tn_kernel<BN>;
   static bool attr_set = false;  // set once, outside any stream capture of a later call
@@ -118,6 +116,14 @@ int launch(GemmArgs g, const void* A, const void* B, cudaStream_t st) {
 }
 
 }  // namespace
+
+// Splits of K of an FP32 product.  Weight gradients have few output tiles and a long K (the batch): about two CTAs per
+// SM, at least 4 K-steps each.
+int gemm_splits(int M, int N, int K) {
+  const int bn = N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64;
+  const int tiles = (N / bn) * (M / BM), KT = K / BK;
+  return tiles < 2 * num_sms() ? std::max(1, std::min(KT / 4, 2 * num_sms() / tiles)) : 1;
+}
 
 // D = A Bᵀ (AᵀB of [K][M] and [K][N] operands with rows_k) with the fused epilogue of g; M % 128 == 0, N % 64 == 0, K % 64 == 0, A and B 16-byte
 // aligned (TMA).  The widest tile that divides N is used.

@@ -7,7 +7,8 @@
 // TMA (128-byte swizzle); warp 1 lane 0 issues tcgen05.mma (kind::f16, M = 128, N = BN, K = 16) into a TMEM
 // accumulator and releases ring slots with tcgen05.commit; the epilogue warps read the accumulator with
 // tcgen05.ld (warp w owns TMEM lanes 32(w mod 4).. = tile rows) and apply the fused epilogue:
-//   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add by TMA, or with atomics)
+//   EPI_F32   out_f32 = D (+ out_f32 when accumulate; split-K CTAs add with atomics), or split-K partial tiles
+//             stored side by side for an ordered sum
 //   EPI_ACT   z = D + bias; out = bf16(act(z)); optional z_out = bf16(z)    forward layers
 //   EPI_DACT  out = bf16(D · act'(z_in))                                   backward layers
 // Two kernels: gemm_act_kernel (whole tiles of the activation epilogues) is persistent, and its epilogue runs
@@ -40,11 +41,12 @@ struct GemmArgs {
   int ldo;                      // output row stride (elements)
   int n_valid;                  // columns < n_valid are stored
   int accumulate;               // EPI_F32: add to the output
+  float* part;                  // EPI_F32: if not null, split z stores its tile at rows z M .. of [splits M][N] instead
+  int max_splits;               // EPI_F32 without part: most splits of K (0: as many as gemm_splits gives)
   __nv_bfloat16* z_out;         // EPI_ACT: pre-activation (ldo stride), may be null
   const __nv_bfloat16* z_in;    // EPI_DACT: pre-activation of this layer (ldo stride)
   int rows_k;                   // operands are [K][M] and [K][N] (EPI_F32)
-  int tma_add;                  // EPI_F32: the tile is added to the output by TMA
-  float* colsum;                // EPI_DACT: colsum[col] += Σ_rows out (as stored, bf16-rounded; 8-byte aligned); may be null
+  float* colpart;               // EPI_DACT: [M / 32][N] sums of out over 32 rows (as stored, bf16-rounded; 8-byte aligned); may be null
   unsigned* err;                // set to 1 by a CTA whose pipeline wait ran out
 };
 
@@ -155,12 +157,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* tm, int x, int y
                "r"(x), "r"(y), "r"(smem_u32(src))
                : "memory");
 }
-__device__ __forceinline__ void tma_add_2d(const CUtensorMap* tm, int x, int y, const void* src) {
-  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
-                   reinterpret_cast<uint64_t>(tm)),
-               "r"(x), "r"(y), "r"(smem_u32(src))
-               : "memory");
-}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -194,6 +190,19 @@ template <int BN>
 constexpr size_t gemm_act_smem_bytes() {
   return 1024 /* alignment slack */ + (size_t)act_stages<BN>() * (BM + BN) * BK * 2 + kActWarps * kStage +
          (2 * act_stages<BN>() + 4 + kActWarps) * 8 + 16;
+}
+
+// Σ over rows r, r + D, r + 2D, .. < 32 of the bf16 pairs at(row), as a tree (a row with the one 16 below it first):
+// five roundings deep, where a chain has 31.
+template <int D, class At>
+__device__ __forceinline__ float2 row_tree(const At& at, int r) {
+  if constexpr (D == 32) {
+    const unsigned u = at(r);
+    return make_float2(bf16_lo(u), bf16_hi(u));
+  } else {
+    const float2 a = row_tree<2 * D>(at, r), b = row_tree<2 * D>(at, r + D);
+    return make_float2(a.x + b.x, a.y + b.y);
+  }
 }
 
 template <int BN>
@@ -340,16 +349,9 @@ __global__ void __launch_bounds__(kActThreads, 1) gemm_act_kernel(const __grid_c
           tma_store_commit();
         }
       }
-      if (dact && g.colsum) {  // columns col + 2 lane, + 1 (the store above only reads the tile)
-        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-          const unsigned u = *reinterpret_cast<const unsigned*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
-          float2& a = (r & 1) ? s1 : s0;
-          a.x += bf16_lo(u);
-          a.y += bf16_hi(u);
-        }
-        atomicAdd(reinterpret_cast<float2*>(g.colsum + col) + lane, make_float2(s0.x + s1.x, s0.y + s1.y));
+      if (dact && g.colpart) {  // columns col + 2 lane, + 1 (the store above only reads the tile)
+        auto at = [&](int r) { return *reinterpret_cast<const unsigned*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4); };
+        reinterpret_cast<float2*>(g.colpart + (size_t)(row0 / 32) * g.N + col)[lane] = row_tree<1>(at, 0);
       }
       if (dact && t + step < ntiles) {  // the next tile's pre-activations, once this tile is read
         __syncwarp();
@@ -444,10 +446,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   tc_fence_after();
   const int quarter = warp & 3, half = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
-  if (ok && g.tma_add) {
+  if (ok && g.part) {
     // split K: 32 x 32 tiles staged in the operand ring (12 KB per warp, three buffers; rows of 128 bytes,
-    // 128-byte swizzle) and added by TMA.  16-byte atomics straight from the lanes' rows touched half a sector
-    // each: a 512 x 512 gradient of 65,536 rows takes 33 µs, 39 with them
+    // 128-byte swizzle) and stored by TMA, each split in its own rows; whoever reads them adds them in the splits'
+    // order.  Added here (by TMA or atomics, in the order of arrival) a gradient differed in its last bits from run
+    // to run, which BF16 weights and Adam's quotient grew to 1e-5 of the weights in 16 steps
     unsigned char* buf = base + warp * 12288;
     int q = 0;
 #pragma unroll 1
@@ -463,7 +466,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       for (int p = 0; p < 8; ++p) *reinterpret_cast<uint4*>(b + lane * 128 + ((p ^ (lane & 7)) << 4)) = make_uint4(v[4 * p], v[4 * p + 1], v[4 * p + 2], v[4 * p + 3]);
       proxy_fence();
       __syncwarp();
-      if (lane == 0) { tma_add_2d(&tmD, n0 + c0, m0 + quarter * 32, b); tma_store_commit(); }
+      if (lane == 0) { tma_store_2d(&tmD, n0 + c0, blockIdx.z * g.M + m0 + quarter * 32, b); tma_store_commit(); }
     }
     if (lane == 0) tma_store_wait_read();
     __syncwarp();

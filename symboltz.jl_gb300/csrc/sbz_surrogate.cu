@@ -12,7 +12,9 @@
 //   loss      Y = X_L W_Lᵀ + b_L (FP32), dY = 2 (Y - T) / (batch · nout), db_L = Σ_batch dY
 //   backward  dZ_{l-1} = (dZ_l W_l) ⊙ SiLU'(Z_{l-1})  (EPI_DACT, db_{l-1} = Σ_batch dZ_{l-1})
 //             dW_l = dZ_lᵀ X_{l-1} (EPI_F32 with rows along K, split K)
-//   Adam      one launch over every parameter: FP32 update, BF16 W and Wt refreshed.
+//   Adam      one launch over every parameter: gradient summed, FP32 update, BF16 W and Wt refreshed.
+// Sums over the batch leave the kernels as partial sums (a split of K, 32 or 256 rows) that the Adam launch adds
+// in their order, so equal trainings give equal bits.
 // The step (about 20 launches) is captured once in a CUDA graph and replayed; the step counter
 // and the learning rate live in device memory so the replayed graph needs no new parameters.
 #include <cuda_bf16.h>
@@ -29,6 +31,7 @@ namespace sbz {
 int capi_fail(int code, const char* msg);
 namespace mlp {
 int gemm(const GemmArgs& g, const void* A, const void* B, cudaStream_t st);
+int gemm_splits(int M, int N, int K);
 }
 }  // namespace sbz
 
@@ -41,9 +44,11 @@ constexpr int kPadIn = 64, kPadOut = 64;
 struct Layer {
   int kin, nrow;      // padded sizes (GEMM K and N)
   int nin, nout;      // logical sizes
-  float *W, *b, *mW, *vW, *mb, *vb, *gW, *gb;  // FP32 [nrow][kin], [nrow]
+  float *W, *b, *mW, *vW, *mb, *vb;  // FP32 [nrow][kin], [nrow]
+  float *gW, *gb;     // gradients of sbz_surrogate_gradients, same shapes
+  float *pW, *pb;     // partial sums of the gradients: [splits][nrow][kin], [row blocks][nrow]
   bf16 *Wh, *Wt;      // BF16 [nrow][kin], [kin][nrow]
-  bool gT;            // gW holds the gradient transposed ([kin][nrow])
+  bool gT;            // a partial sum in pW is transposed ([kin][nrow])
 };
 
 template <class T>
@@ -59,9 +64,8 @@ struct sbz_surrogate {
   float* Yf = nullptr;        // [batch][64] last-layer product (before bias)
   bf16* dY = nullptr;
   float* T = nullptr;         // [batch][nout] targets of the step
-  double* loss = nullptr;     // first entry of grads
-  unsigned char* grads = nullptr;  // loss and every layer's gW and gb: one memset per step
-  size_t grads_bytes = 0;
+  double *loss = nullptr, *ploss = nullptr;  // loss and its partial sums (row blocks)
+  unsigned char* grads = nullptr;  // loss, every layer's gW and gb, then the partial sums
   unsigned* err = nullptr;
   float *dataX = nullptr, *dataY = nullptr;
   long long ndata = 0;
@@ -70,7 +74,7 @@ struct sbz_surrogate {
   cudaStream_t stream = nullptr;
   long long* dstep = nullptr;  // device step counter (incremented at the start of each step)
   float* dlr = nullptr;        // device learning rate
-  void* segs = nullptr;        // device table of Adam segments
+  void* segs = nullptr;        // device tables of Adam segments: of the training batch, and of the last gradients call
   int nseg = 0;
   int nadam = 0;               // blocks of the Adam launch
   cudaGraph_t graph = nullptr;
@@ -127,12 +131,12 @@ __global__ void __launch_bounds__(128) gather_batch(int batch, int nin, int nout
 __global__ void set_value(float* dst, float v) { *dst = v; }
 
 // loss and output gradient: y = Yf + b (FP32), r = y - t, dY = 2 r / (batch · nout) (BF16; padding columns
-// stay zero) and the bias gradient gb[j] += Σ_rows dY[.][j] (as rounded).
+// stay zero), and a block's part of the loss and of the bias gradient Σ_rows dY[.][j] (as rounded; [block][kPadOut]).
 // 256 threads per block.  Advances the device step counter (if not null; nothing else here reads it).
 constexpr int kLossThreads = 256;
 __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, const float* __restrict__ Yf, const float* __restrict__ b,
-                                                           const float* __restrict__ T, bf16* __restrict__ dY, float* __restrict__ gb,
-                                                           double* __restrict__ loss, long long* __restrict__ dstep) {
+                                                           const float* __restrict__ T, bf16* __restrict__ dY, float* __restrict__ pb,
+                                                           double* __restrict__ ploss, long long* __restrict__ dstep) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   __shared__ float cs[kLossThreads / 32][kPadOut];
   double l = 0;
@@ -157,69 +161,134 @@ __global__ void __launch_bounds__(kLossThreads) loss_grad(int batch, int nout, c
   if (threadIdx.x == 0) {
     double s = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-    atomicAdd(loss, s / ((double)batch * nout));
+    ploss[blockIdx.x] = s / ((double)batch * nout);
     if (dstep && blockIdx.x == 0) ++*dstep;
   }
   if (threadIdx.x < nout) {
     float s = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += cs[w][threadIdx.x];
-    atomicAdd(gb + threadIdx.x, s);
+    pb[(size_t)blockIdx.x * kPadOut + threadIdx.x] = s;
   }
 }
 
-// Adam over every parameter in one launch, one 32 x 32 tile of a layer's weights (with BF16 copies
-// [nrow][kin] and [kin][nrow], the second written through shared memory along its rows; the gradient possibly
-// transposed) or 1,024 biases per block.  `start` is the segment's first block.  The bias corrections use
-// the device step counter.
-struct AdamSeg {
-  float *p, *m, *v;
-  const float* g;
-  bf16 *ph, *pt;
-  int start, n, gT, nrow, kin;
+// Sum in the order of the additions, compensated (their rounding errors are summed beside): the result is the terms'
+// sum but for about one rounding.
+struct Sum {
+  float s = 0.0f, c = 0.0f;
+  __device__ void add(float x) {
+    const float t = s + x, y = t - s;
+    c += (s - (t - y)) + (x - y);
+    s = t;
+  }
+  __device__ float value() const { return isfinite(c) ? s + c : s; }  // an infinite term makes c NaN
 };
 
-__global__ void __launch_bounds__(256) adam_all(const AdamSeg* __restrict__ segs, int nseg, const long long* __restrict__ step,
-                                                const float* __restrict__ lr, float b1, float b2, float eps) {
-  __shared__ float tile[32][33];
-  int q = 0;
-  while (q + 1 < nseg && segs[q + 1].start <= (int)blockIdx.x) ++q;
-  const AdamSeg S = segs[q];
-  const int blk = blockIdx.x - S.start, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const float t = (float)*step, rate = *lr;
-  const float c1 = 1.0f / (1.0f - exp2f(t * log2f(b1))), c2 = 1.0f / (1.0f - exp2f(t * log2f(b2)));
-  auto update = [&](size_t i, float gi) {
-    const float mi = b1 * S.m[i] + (1 - b1) * gi, vi = b2 * S.v[i] + (1 - b2) * gi * gi;
-    S.m[i] = mi; S.v[i] = vi;
-    const float pi = S.p[i] - rate * (mi * c1) / (sqrtf(vi * c2) + eps);
-    S.p[i] = pi;
-    return pi;
-  };
-  if (!S.ph) {
-    for (int i = blk * 1024 + threadIdx.x; i < min(S.n, (blk + 1) * 1024); i += 256) update(i, S.g[i]);
+// The gradients from their partial sums, and with ADAM the update of every parameter, in one launch: 1,024 weights of
+// a layer (with BF16 copies [nrow][kin] and [kin][nrow]) or 32 biases per block, the last block the loss.  `start` is
+// the segment's first block; the biases come first (up to 2,048 parts behind each other, weights at most 76).  The bias
+// corrections use the device step counter.  Bound: reading the parts from HBM (151 MB for 4 x 512 wide layers and 65,536
+// rows: 40 µs).  A warp reads 512 (input and output layer: 256) consecutive bytes of eight parts at a time (83 µs by
+// 32 x 32 tiles, 128 bytes).
+struct Seg {
+  float *p, *m, *v, *g;
+  const float* part;
+  long long stride;  // between partial sums
+  bf16 *ph, *pt;
+  int parts, start, gT, nrow, kin;
+};
+
+template <bool ADAM>
+__global__ void __launch_bounds__(256, 3) apply_grads(const Seg* __restrict__ segs, int nseg, const double* __restrict__ ploss, int nloss,
+                                                      double* __restrict__ loss, const long long* __restrict__ step,
+                                                      const float* __restrict__ lr, float b1, float b2, float eps) {
+  __shared__ float tile[16 * 68];
+  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  if (blockIdx.x == gridDim.x - 1) {  // the loss: lane sums of every 32nd part, then a butterfly
+    if (ty > 0) return;
+    double l = 0;
+    for (int i = tx; i < nloss; i += 32) l += ploss[i];
+    for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (tx == 0) *loss = l;
     return;
   }
-  const int kt = S.kin / 32, r0 = blk / kt * 32, k0 = blk % kt * 32;
-  if (S.gT) {
+  int q = 0;
+  while (q + 1 < nseg && segs[q + 1].start <= (int)blockIdx.x) ++q;
+  const Seg S = segs[q];
+  const int blk = blockIdx.x - S.start;
+  const float t = ADAM ? (float)*step : 0.0f, rate = ADAM ? *lr : 0.0f;
+  const float c1 = 1.0f / (1.0f - exp2f(t * log2f(b1))), c2 = 1.0f / (1.0f - exp2f(t * log2f(b2)));
+  auto adam = [&](float& p, float& m, float& v, float g) {
+    m = b1 * m + (1 - b1) * g;
+    v = b2 * v + (1 - b2) * g * g;
+    p = p - rate * (m * c1) / (sqrtf(v * c2) + eps);
+  };
+  auto update = [&](size_t i, float g) {
+    if (!ADAM) { S.g[i] = g; return 0.0f; }
+    float p = S.p[i], m = S.m[i], v = S.v[i];
+    adam(p, m, v, g);
+    S.p[i] = p; S.m[i] = m; S.v[i] = v;
+    return p;
+  };
+  if (!S.ph) {  // 32 biases: an eighth of the parts per warp, then the eighths
+    const int i = blk * 32 + tx, q0 = (int)((long long)S.parts * ty / 8), q1 = (int)((long long)S.parts * (ty + 1) / 8);
+    Sum a;
+    for (int r = q0; r < q1; r += 32) {
+      float x[32];
 #pragma unroll
-    for (int y = 0; y < 4; ++y) tile[tx][ty + 8 * y] = S.g[(size_t)(k0 + ty + 8 * y) * S.nrow + r0 + tx];  // [r][k]
+      for (int u = 0; u < 32; ++u) x[u] = r + u < q1 ? __ldg(S.part + (r + u) * S.stride + i) : 0.0f;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) a.add(x[u]);
+    }
+    tile[ty * 32 + tx] = a.s;
+    tile[256 + ty * 32 + tx] = a.c;
     __syncthreads();
+    if (ty > 0) return;
+    Sum b;
+    for (int w = 0; w < 8; ++w) { b.add(tile[w * 32 + tx]); b.c += tile[256 + w * 32 + tx]; }
+    update(i, b.value());
+    return;
   }
-  float p[4];
+  // 8 x 128 or 16 x 64 values of a part (its columns are the outputs when transposed), four in a row per thread
+  const int pc = S.gT ? S.nrow : S.kin, tc = pc % 128 == 0 ? 128 : 64, tr = 1024 / tc, l4 = tc / 4;
+  const int row0 = blk / (pc / tc) * tr, col0 = blk % (pc / tc) * tc, x4 = tid % l4 * 4, y = tid / l4;
+  const size_t at = (size_t)(row0 + y) * pc + col0 + x4;
+  Sum a[4];
+  for (int r = 0; r < S.parts; r += 8) {
+    float4 x[8];
 #pragma unroll
-  for (int y = 0; y < 4; ++y) {
-    const int r = ty + 8 * y;
-    const size_t i = (size_t)(r0 + r) * S.kin + k0 + tx;
-    p[y] = update(i, S.gT ? tile[r][tx] : S.g[i]);
-    S.ph[i] = __float2bfloat16(p[y]);
+    for (int u = 0; u < 8; ++u)
+      x[u] = r + u < S.parts ? __ldg(reinterpret_cast<const float4*>(S.part + (r + u) * S.stride + at)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) { a[0].add(x[u].x); a[1].add(x[u].y); a[2].add(x[u].z); a[3].add(x[u].w); }
   }
-  __syncthreads();
+  const float4 g = make_float4(a[0].value(), a[1].value(), a[2].value(), a[3].value());
+  if (S.gT) {  // one column of the part (an output) per 16 threads
+    *reinterpret_cast<float4*>(tile + y * 68 + x4) = g;
+    __syncthreads();
+    const int k = tid % 16;
 #pragma unroll
-  for (int y = 0; y < 4; ++y) tile[ty + 8 * y][tx] = p[y];
+    for (int j = 0; j < 4; ++j) {
+      const int r = tid / 16 + 16 * j;
+      const size_t i = (size_t)(col0 + r) * S.kin + row0 + k;
+      const float p = update(i, tile[k * 68 + r]);
+      if (ADAM) { S.ph[i] = __float2bfloat16(p); S.pt[(size_t)(row0 + k) * S.nrow + col0 + r] = __float2bfloat16(p); }
+    }
+    return;
+  }
+  if (!ADAM) { *reinterpret_cast<float4*>(S.g + at) = g; return; }
+  float4 p = *reinterpret_cast<const float4*>(S.p + at), m = *reinterpret_cast<const float4*>(S.m + at), v = *reinterpret_cast<const float4*>(S.v + at);
+  adam(p.x, m.x, v.x, g.x); adam(p.y, m.y, v.y, g.y); adam(p.z, m.z, v.z, g.z); adam(p.w, m.w, v.w, g.w);
+  *reinterpret_cast<float4*>(S.p + at) = p; *reinterpret_cast<float4*>(S.m + at) = m; *reinterpret_cast<float4*>(S.v + at) = v;
+  *reinterpret_cast<uint2*>(S.ph + at) = make_uint2(sbz::mlp::pack_bf16(p.x, p.y), sbz::mlp::pack_bf16(p.z, p.w));
+  *reinterpret_cast<float4*>(tile + y * tc + x4) = p;
   __syncthreads();
+  // a column's 8 rows are 16 bytes of the transposed copy
+  if (tid < tc * tr / 8) {
+    const int k = tid % tc, r = tid / tc * 8;
+    unsigned w[4];
 #pragma unroll
-  for (int y = 0; y < 4; ++y) {
-    const int k = ty + 8 * y;
-    S.pt[(size_t)(k0 + k) * S.nrow + r0 + tx] = __float2bfloat16(tile[tx][k]);
+    for (int j = 0; j < 4; ++j) w[j] = sbz::mlp::pack_bf16(tile[(r + 2 * j) * tc + k], tile[(r + 2 * j + 1) * tc + k]);
+    *reinterpret_cast<uint4*>(S.pt + (size_t)(col0 + k) * S.nrow + row0 + r) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -276,67 +345,93 @@ int refresh_bf16(sbz_surrogate* s) {
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : F(SBZ_ERR_CUDA, "surrogate: weight copy");
 }
 
-int gemm(sbz_surrogate* s, int M, int N, int K, const bf16* A, const bf16* B, int epi, int act, const float* bias, void* out, int ldo,
-         int n_valid, int acc, bf16* z_out, const bf16* z_in, float* colsum = nullptr, int rows_k = 0) {
-  using namespace sbz::mlp;
-  GemmArgs g{};
-  g.M = M; g.N = N; g.K = K; g.epi = epi; g.act = act; g.bias = bias;
-  g.out_bf16 = static_cast<bf16*>(out); g.out_f32 = static_cast<float*>(out); g.ldo = ldo; g.n_valid = n_valid; g.accumulate = acc;
-  g.z_out = z_out; g.z_in = z_in; g.err = s->err;
-  g.colsum = colsum; g.rows_k = rows_k;
+int gemm(sbz_surrogate* s, sbz::mlp::GemmArgs g, const bf16* A, const bf16* B) {
+  g.err = s->err;
   const int r = sbz::mlp::gemm(g, A, B, s->stream);
   return r == SBZ_OK ? SBZ_OK : F(r, "surrogate: GEMM launch");
+}
+
+// out = act(A Bᵀ + bias) or, with z_in, (A Bᵀ) ⊙ act'(z_in) of an N-wide layer
+int layer(sbz_surrogate* s, int M, int N, int K, const bf16* A, const bf16* B, const float* bias, bf16* out, bf16* z_out, const bf16* z_in,
+          float* colpart) {
+  sbz::mlp::GemmArgs g{};
+  g.M = M; g.N = N; g.K = K; g.epi = z_in ? sbz::mlp::EPI_DACT : sbz::mlp::EPI_ACT; g.act = sbz::mlp::ACT_SILU; g.bias = bias;
+  g.out_bf16 = out; g.ldo = N; g.n_valid = N; g.z_out = z_out; g.z_in = z_in; g.colpart = colpart;
+  return gemm(s, g, A, B);
+}
+
+// partial sums of AᵀB over the batch, A [batch][M] and B [batch][N]
+int weight_gradient(sbz_surrogate* s, int M, int N, const bf16* A, const bf16* B, float* part) {
+  sbz::mlp::GemmArgs g{};
+  g.M = M; g.N = N; g.K = s->batch; g.epi = sbz::mlp::EPI_F32; g.ldo = N; g.n_valid = N; g.part = part; g.rows_k = 1;
+  return gemm(s, g, A, B);
 }
 
 // forward pass of `rows` (multiple of 128, ≤ batch) rows already in X[0]; result in Yf.  With
 // `train`, the pre-activations are written for the backward pass.
 int forward(sbz_surrogate* s, int rows, bool train) {
-  using namespace sbz::mlp;
   const int nl = (int)s->L.size();
   for (int l = 0; l < nl - 1; ++l) {
     const Layer& y = s->L[l];
-    int r = gemm(s, rows, y.nrow, y.kin, s->X[l], y.Wh, EPI_ACT, ACT_SILU, y.b, s->X[l + 1], y.nrow, y.nrow, 0,
-                 train ? s->Z[l + 1] : nullptr, nullptr);
+    const int r = layer(s, rows, y.nrow, y.kin, s->X[l], y.Wh, y.b, s->X[l + 1], train ? s->Z[l + 1] : nullptr, nullptr, nullptr);
     if (r) return r;
   }
   const Layer& o = s->L[nl - 1];
-  return gemm(s, rows, o.nrow, o.kin, s->X[nl - 1], o.Wh, EPI_F32, ACT_NONE, nullptr, s->Yf, kPadOut, s->nout, 0, nullptr, nullptr);
+  sbz::mlp::GemmArgs g{};
+  g.M = rows; g.N = o.nrow; g.K = o.kin; g.epi = sbz::mlp::EPI_F32; g.out_f32 = s->Yf; g.ldo = kPadOut; g.n_valid = s->nout;
+  g.max_splits = 2;  // two parts added to zero give the same bits in either order
+  return gemm(s, g, s->X[nl - 1], o.Wh);
 }
 
-// backward pass after forward(train) + loss_grad (dY and the output layer's gb set): weight
-// gradients added into gW, bias gradients into gb by the EPI_DACT epilogues (both zeroed before)
+// backward pass after forward(train) + loss_grad (dY and the output layer's pb set): partial sums of the weight
+// gradients into pW, of the bias gradients into pb by the EPI_DACT epilogues
 int backward(sbz_surrogate* s) {
-  using namespace sbz::mlp;
   const int B = s->batch, nl = (int)s->L.size();
   // output layer: dW_Lᵀ = X_{L-1}ᵀ dY ([kin][64]); dZ_{L-1} = (dY W_L) ⊙ SiLU'(Z_{L-1})
-  Layer& o = s->L[nl - 1];
-  int r = gemm(s, o.kin, kPadOut, B, s->X[nl - 1], s->dY, EPI_F32, ACT_NONE, nullptr, o.gW, kPadOut, kPadOut, 1, nullptr, nullptr, nullptr, 1);
+  const Layer& o = s->L[nl - 1];
+  int r = weight_gradient(s, o.kin, kPadOut, s->X[nl - 1], s->dY, o.pW);
   if (r) return r;
-  r = gemm(s, B, o.kin, kPadOut, s->dY, o.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[nl - 1], o.kin, o.kin, 0, nullptr, s->Z[nl - 1],
-           s->L[nl - 2].gb);
+  r = layer(s, B, o.kin, kPadOut, s->dY, o.Wt, nullptr, s->dZ[nl - 1], nullptr, s->Z[nl - 1], s->L[nl - 2].pb);
   if (r) return r;
   // hidden layers l = nl-2 .. 0: input X[l], output gradient dZ[l+1]
   for (int l = nl - 2; l >= 0; --l) {
-    Layer& y = s->L[l];
-    r = gemm(s, y.nrow, y.kin, B, s->dZ[l + 1], s->X[l], EPI_F32, ACT_NONE, nullptr, y.gW, y.kin, y.kin, 1, nullptr, nullptr, nullptr, 1);
+    const Layer& y = s->L[l];
+    r = weight_gradient(s, y.nrow, y.kin, s->dZ[l + 1], s->X[l], y.pW);
     if (r) return r;
     if (l > 0) {
-      r = gemm(s, B, y.kin, y.nrow, s->dZ[l + 1], y.Wt, EPI_DACT, ACT_SILU, nullptr, s->dZ[l], y.kin, y.kin, 0, nullptr, s->Z[l],
-               s->L[l - 1].gb);
+      r = layer(s, B, y.kin, y.nrow, s->dZ[l + 1], y.Wt, nullptr, s->dZ[l], nullptr, s->Z[l], s->L[l - 1].pb);
       if (r) return r;
     }
   }
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : F(SBZ_ERR_CUDA, "surrogate: backward");
 }
 
-// forward + loss + backward of the `rows` rows in X[0] (and X[0]ᵀ) with targets T; advances dstep (if given)
+int loss_blocks(int rows) { return (rows + kLossThreads - 1) / kLossThreads; }
+
+// forward + loss + backward of the `rows` rows in X[0] with targets T; advances dstep (if given)
 int forward_backward(sbz_surrogate* s, int rows, long long* dstep) {
-  SCU(cudaMemsetAsync(s->grads, 0, s->grads_bytes, s->stream));
   int r = forward(s, rows, true);
   if (r) return r;
-  loss_grad<<<(rows + kLossThreads - 1) / kLossThreads, kLossThreads, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, s->T, s->dY, s->L.back().gb,
-                                                                                  s->loss, dstep);
+  loss_grad<<<loss_blocks(rows), kLossThreads, 0, s->stream>>>(rows, s->nout, s->Yf, s->L.back().b, s->T, s->dY, s->L.back().pb, s->ploss, dstep);
   return backward(s);
+}
+
+// splits of the batch in a layer's weight gradient, and row blocks in its bias gradient
+int weight_parts(const Layer& y, int rows) { return y.gT ? sbz::mlp::gemm_splits(y.kin, y.nrow, rows) : sbz::mlp::gemm_splits(y.nrow, y.kin, rows); }
+int bias_parts(const Layer& y, int rows) { return y.gT ? loss_blocks(rows) : rows / 32; }
+
+std::vector<Seg> make_segs(const sbz_surrogate* s, int rows, int& blocks) {
+  std::vector<Seg> segs;
+  blocks = 0;
+  for (auto& l : s->L) {
+    segs.push_back(Seg{l.b, l.mb, l.vb, l.gb, l.pb, l.nrow, nullptr, nullptr, bias_parts(l, rows), blocks, 0, l.nrow, 1});
+    blocks += l.nrow / 32;
+  }
+  for (auto& l : s->L) {
+    segs.push_back(Seg{l.W, l.mW, l.vW, l.gW, l.pW, (long long)l.nrow * l.kin, l.Wh, l.Wt, weight_parts(l, rows), blocks, l.gT ? 1 : 0, l.nrow, l.kin});
+    blocks += l.nrow * l.kin / 1024;
+  }
+  return segs;
 }
 
 // one training step on the stream (captured into the step graph)
@@ -345,7 +440,8 @@ int train_step(sbz_surrogate* s) {
   gather_batch<<<(B + 127) / 128, 128, 0, s->stream>>>(B, s->nin, s->nout, s->dataX, s->dataY, s->ndata, s->dstep, s->seed, 1, s->X[0], s->T);
   int r = forward_backward(s, B, s->dstep);
   if (r) return r;
-  adam_all<<<s->nadam, 256, 0, s->stream>>>(static_cast<const AdamSeg*>(s->segs), s->nseg, s->dstep, s->dlr, 0.9f, 0.999f, 1e-8f);
+  apply_grads<true><<<s->nadam + 1, 256, 0, s->stream>>>(static_cast<const Seg*>(s->segs), s->nseg, s->ploss, loss_blocks(B), s->loss, s->dstep, s->dlr,
+                                                         0.9f, 0.999f, 1e-8f);
   return cudaGetLastError() == cudaSuccess ? SBZ_OK : F(SBZ_ERR_CUDA, "surrogate: training step");
 }
 
@@ -401,18 +497,21 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
     for (float* p : {y.mb, y.vb}) cudaMemset(p, 0, sizeof(float) * y.nrow);
   }
   {
-    size_t off = 256;  // the loss, then gW and gb per layer on 256-byte boundaries
-    auto take = [&](size_t n) { const size_t o = off; off += (sizeof(float) * n + 255) & ~size_t(255); return o; };
-    std::vector<size_t> ow, ob;
-    for (auto& y : s->L) { ow.push_back(take((size_t)y.nrow * y.kin)); ob.push_back(take(y.nrow)); }
-    if (dalloc(&s->grads, off)) return bail("surrogate: gradient allocation");
-    s->grads_bytes = off;
-    cudaMemset(s->grads, 0, off);
-    s->loss = reinterpret_cast<double*>(s->grads);
-    for (int l = 0; l < nl; ++l) {
-      s->L[l].gW = reinterpret_cast<float*>(s->grads + ow[l]);
-      s->L[l].gb = reinterpret_cast<float*>(s->grads + ob[l]);
+    size_t off = 256;  // the loss, then gW and gb per layer and the partial sums, on 256-byte boundaries
+    auto take = [&](size_t bytes) { const size_t o = off; off += (bytes + 255) & ~size_t(255); return o; };
+    std::vector<size_t> o;
+    for (auto& y : s->L) {
+      const size_t nw = sizeof(float) * (size_t)y.nrow * y.kin, nb = sizeof(float) * (size_t)y.nrow;
+      for (size_t n : {nw, nb, nb * bias_parts(y, batch), nw * weight_parts(y, batch)}) o.push_back(take(n));
     }
+    const size_t ol = take(sizeof(double) * loss_blocks(batch));
+    if (dalloc(&s->grads, off)) return bail("surrogate: gradient allocation");
+    s->loss = reinterpret_cast<double*>(s->grads);
+    s->ploss = reinterpret_cast<double*>(s->grads + ol);
+    auto at = [&](int i) { return reinterpret_cast<float*>(s->grads + o[i]); };
+    for (int l = 0; l < nl; ++l) { s->L[l].gW = at(4 * l); s->L[l].gb = at(4 * l + 1); s->L[l].pb = at(4 * l + 2); s->L[l].pW = at(4 * l + 3); }
+    cudaMemset(s->loss, 0, sizeof(double));
+    cudaMemset(s->L[nl - 1].pb, 0, sizeof(float) * kPadOut * loss_blocks(batch));  // padding columns that no kernel writes
   }
   s->X.assign(nl, nullptr); s->Z.assign(nl, nullptr); s->dZ.assign(nl, nullptr);
   for (int l = 0; l < nl; ++l) {
@@ -428,19 +527,11 @@ int sbz_surrogate_create(int nin, int width, int nhidden, int nout, int batch, u
   // padding columns that no kernel writes
   cudaMemset(s->dY, 0, sizeof(bf16) * (size_t)batch * kPadOut);
   {
-    std::vector<AdamSeg> segs;
-    int start = 0;
-    for (auto& l : s->L) {
-      segs.push_back(AdamSeg{l.W, l.mW, l.vW, l.gW, l.Wh, l.Wt, start, l.nrow * l.kin, l.gT ? 1 : 0, l.nrow, l.kin});
-      start += l.nrow / 32 * (l.kin / 32);
-      segs.push_back(AdamSeg{l.b, l.mb, l.vb, l.gb, nullptr, nullptr, start, l.nrow, 0, l.nrow, 1});
-      start += (l.nrow + 1023) / 1024;
-    }
+    const std::vector<Seg> segs = make_segs(s, batch, s->nadam);
     s->nseg = (int)segs.size();
-    s->nadam = start;
-    if (dalloc(&s->dstep, 1) || dalloc(&s->dlr, 1) || cudaMalloc(&s->segs, sizeof(AdamSeg) * segs.size()) != cudaSuccess)
+    if (dalloc(&s->dstep, 1) || dalloc(&s->dlr, 1) || cudaMalloc(&s->segs, 2 * sizeof(Seg) * segs.size()) != cudaSuccess)
       return bail("surrogate: buffer allocation");
-    cudaMemcpy(s->segs, segs.data(), sizeof(AdamSeg) * segs.size(), cudaMemcpyHostToDevice);
+    cudaMemcpy(s->segs, segs.data(), sizeof(Seg) * segs.size(), cudaMemcpyHostToDevice);
     cudaMemset(s->dstep, 0, sizeof(long long));
   }
   if (refresh_bf16(s) != SBZ_OK) { free_all(s); delete s; return SBZ_ERR_CUDA; }
@@ -547,6 +638,13 @@ int sbz_surrogate_gradients(sbz_surrogate* s, int n, const float* X, const float
   gather_batch<<<(n + 127) / 128, 128, 0, s->stream>>>(n, s->nin, s->nout, dx, dy, n, nullptr, 0, 0, s->X[0], s->T);
   int r = forward_backward(s, n, nullptr);
   s->batch = keepB;
+  if (!r) {
+    int blocks = 0;
+    const std::vector<Seg> segs = make_segs(s, n, blocks);
+    Seg* d = static_cast<Seg*>(s->segs) + s->nseg;
+    if (cudaMemcpyAsync(d, segs.data(), sizeof(Seg) * segs.size(), cudaMemcpyHostToDevice, s->stream) != cudaSuccess) r = F(SBZ_ERR_CUDA, "surrogate: gradients");
+    else apply_grads<false><<<blocks + 1, 256, 0, s->stream>>>(d, s->nseg, s->ploss, loss_blocks(n), s->loss, nullptr, nullptr, 0.9f, 0.999f, 1e-8f);
+  }
   cudaFree(dx); cudaFree(dy);
   if (r) return r;
   if ((r = check_err(s))) return r;
@@ -558,7 +656,7 @@ int sbz_surrogate_gradients(sbz_surrogate* s, int n, const float* X, const float
       SCU(cudaMemcpy(g.data(), l.gW, sizeof(float) * g.size(), cudaMemcpyDeviceToHost));
       SCU(cudaMemcpy(b.data(), l.gb, sizeof(float) * b.size(), cudaMemcpyDeviceToHost));
       for (int rr = 0; rr < l.nout; ++rr)
-        for (int k = 0; k < l.nin; ++k) grads[o++] = l.gT ? g[(size_t)k * l.nrow + rr] : g[(size_t)rr * l.kin + k];
+        for (int k = 0; k < l.nin; ++k) grads[o++] = g[(size_t)rr * l.kin + k];
       for (int rr = 0; rr < l.nout; ++rr) grads[o++] = b[rr];
     }
   }
