@@ -183,6 +183,15 @@ int sbz_problem_set_stream(sbz_problem* pb, void* stream);
  * line of sight, C_l, D2H, total, (reserved). */
 int sbz_problem_timings(const sbz_problem* pb, double* ms8);
 
+/* No counterpart in the reference.  Which kernel a perturbation launch of these modes takes on a device of num_sms
+ * SMs with the problem's options (no device needed), in shape[4]: SBZ_PT_GENERIC, SBZ_PT_LATENCY (one mode per SM) or
+ * SBZ_PT_THROUGHPUT; warps per mode in whose order its norms are summed (what mixed-precision results depend on); modes
+ * per SM (generic kernel: 0); warps that run a mode.  ks NULL: wavenumbers not known on the host (sbz_solve_pt_device). */
+#define SBZ_PT_GENERIC 0
+#define SBZ_PT_LATENCY 1
+#define SBZ_PT_THROUGHPUT 2
+int sbz_pt_launch_shape(const sbz_problem* pb, int nk, const double* ks, int ntau, int num_sms, int* shape);
+
 /* No counterpart in the reference (its solvept threads over k on the CPU).  Autotuner for the
  * perturbation kernel's launch shape: times the candidates (warps per mode, blocks per SM) =
  * (1,0) (2,0) (2,2) (4,1) (4,2) (4,3) (8,1) on a k-stratified sample of the given modes (an eighth of

@@ -518,6 +518,17 @@ int sbz_solve_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks, co
   return SBZ_OK;
 }
 
+int sbz_pt_launch_shape(const sbz_problem* pb, int nk, const double* ks, int ntau, int num_sms, int* shape) {
+  if (!pb || nk < 1 || ntau < 0 || num_sms < 1 || !shape) return fail(SBZ_ERR_ARG, "sbz_pt_launch_shape: bad arguments");
+  sbz::PtArgs A{};
+  pt_model_args(pb, A);
+  A.nitems = nk;
+  A.load = ks ? pt_load(pb, ks, nk, ntau) : 0.0;
+  const sbz::PtShape s = sbz::pt_shape(A, pb->opts.precision, pb->opts.warps_per_mode, pb->opts.blocks_per_sm, num_sms);
+  shape[0] = s.kernel; shape[1] = s.nw; shape[2] = s.modes; shape[3] = s.warps;
+  return SBZ_OK;
+}
+
 int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks, const double* tau_ini, int ntau,
                     const double* taus, int output, int* best, double* ms) {
   if (!check_pt_args(pb, nk, ntau, output)) return SBZ_ERR_ARG;

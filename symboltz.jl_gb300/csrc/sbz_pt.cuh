@@ -35,6 +35,11 @@ struct PtArgs {
   unsigned int* counter;      // device work-queue counter, zero before launch
 };
 
+// Kernel that runs a launch: warps per mode in whose order the norms are summed (nw) and that run it (warps), modes that
+// share an SM (generic kernel: 0) and blocks per SM (generic kernel; 0: as many as fit).
+enum { PT_GENERIC = 0, PT_LATENCY = 1, PT_THROUGHPUT = 2 };
+struct PtShape { int kernel, nw, warps, modes, blocks; };
+PtShape pt_shape(const PtArgs& A, int precision, int warps_per_mode, int blocks_per_sm, int num_sms);
 int pt_launch(const PtArgs& A, int precision, int warps_per_block, int warps_per_mode, int blocks_per_sm, int num_sms,
               cudaStream_t stream);
 int rhs_launch(const PtArgs& A, const double* y, const double* tau, double* f, double* ft, cudaStream_t st);

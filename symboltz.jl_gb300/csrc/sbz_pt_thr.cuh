@@ -853,6 +853,14 @@ __device__ void thr_body(const PtArgs& A, const ModelDesc& M, const CompDesc* __
   }
 }
 
+// Shared memory of a block of `modes` modes.
+template <typename ST>
+__host__ inline size_t thr_block_bytes(int n, int modes) { return ((sizeof(ModelDesc) + 15) & ~size_t(15)) + modes * thr_mode_bytes<ST>(n); }
+// Modes of two warps that an SM holds (two blocks of four, or one: 228 KB of shared memory, 1 KB of it per block for the
+// driver).  Two to four modes of four warps fit at every size.
+template <typename ST>
+__host__ inline int thr2_resident(int n) { return 2 * (thr_block_bytes<ST>(n, 4) + 1024) <= 228 * 1024 ? 8 : 4; }
+
 // NT threads per block (NT / (32 G) modes), MINB blocks per SM: 128 x 3 keeps 168 registers per thread (no
 // spills), 256 x 2 runs 16 warps per SM on 128.
 template <int G, int NT, int MINB, int NSL, typename ST>
@@ -900,7 +908,7 @@ __global__ void __launch_bounds__(NT, MINB) pt_thr_kernel(PtArgs A) {
 template <int G, int NT, int MINB, int NSL, typename ST>
 int launch_thr(const PtArgs& A, int max_blocks, int num_sms, cudaStream_t stream) {
   constexpr int modes = NT / (32 * G);
-  const size_t smem = ((sizeof(ModelDesc) + 15) & ~size_t(15)) + modes * thr_mode_bytes<ST>(A.model_n);
+  const size_t smem = thr_block_bytes<ST>(A.model_n, modes);
   auto kern = pt_thr_kernel<G, NT, MINB, NSL, ST>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return SBZ_ERR_CUDA;
   int per_sm = 0;

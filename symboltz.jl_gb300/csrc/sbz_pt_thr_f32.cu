@@ -5,9 +5,11 @@ namespace sbz {
 
 int pt_launch_thr2_f32(const PtArgs& A, int num_sms, cudaStream_t stream);
 
-int pt_launch_thr_f32(const PtArgs& A, int modes_per_sm, int num_sms, cudaStream_t stream) {
+int pt_thr2_resident_f32(int n) { return ptk::thr2_resident<float>(n); }
+
+int pt_launch_thr_f32(const PtArgs& A, int warps, int modes_per_sm, int num_sms, cudaStream_t stream) {
   using namespace ptk;
-  if (modes_per_sm > 4) return pt_launch_thr2_f32(A, num_sms, stream);
+  if (warps == 2) return pt_launch_thr2_f32(A, num_sms, stream);
   const int slots = (A.model_n + 127) / 128;
   if (slots < 1 || slots > 2) return SBZ_ERR_ARG;
   if (modes_per_sm > 3)
