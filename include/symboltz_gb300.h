@@ -193,14 +193,16 @@ int sbz_problem_timings(const sbz_problem* pb, double* ms8);
 int sbz_pt_launch_shape(const sbz_problem* pb, int nk, const double* ks, int ntau, int num_sms, int* shape);
 
 /* No counterpart in the reference (its solvept threads over k on the CPU).  Autotuner for the
- * perturbation kernel's launch shape: times the candidates (warps per mode, blocks per SM) =
- * (1,0) (2,0) (2,2) (4,1) (4,2) (4,3) (8,1) on a k-stratified sample of the given modes (an eighth of
- * them above 2048 modes, all of them otherwise), stores the fastest in the problem's options and
- * returns it in best[2]; ms[SBZ_TUNE_CANDIDATES] receives the candidates' kernel times (may be
- * NULL).  Arguments as sbz_solve_pt. */
+ * perturbation kernel's launch shape: times the open shapes (0,0) (the default) and (4,0), then the candidates (warps per
+ * mode, blocks per SM) = (1,0) (2,0) (2,2) (4,1) (4,2) (4,3) (8,1) on a k-stratified sample of the given modes (down to an
+ * eighth of them where that still fills the device, all of them otherwise), stores the fastest in the problem's
+ * options (the default unless another is 2 % faster) and returns it in best[2]; ms[SBZ_TUNE_CANDIDATES]
+ * receives the candidates' kernel times (may be NULL), sbz_autotune_open_ms those of the two open shapes in the last call.
+ * Arguments as sbz_solve_pt. */
 #define SBZ_TUNE_CANDIDATES 7
 int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks, const double* tau_ini, int ntau,
                     const double* taus, int output, int* best, double* ms);
+int sbz_autotune_open_ms(const sbz_problem* pb, double* ms2);
 
 /* No counterpart in the reference: the source surrogate's dense-layer GEMM (BF16 tcgen05 tensor
  * cores, FP32 accumulation), exposed for testing.  D = A·Bᵀ with A [M][K] and B [N][K] bf16

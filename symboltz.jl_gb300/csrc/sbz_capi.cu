@@ -134,6 +134,7 @@ struct sbz_problem {
   bool own_stream = true;
   cudaEvent_t ev[12] = {};
   double timings[8] = {};
+  double open_ms[2] = {};  // open shapes in the last sbz_autotune_pt
 };
 
 namespace {
@@ -412,9 +413,10 @@ static double pt_load(const sbz_problem* pb, const double* ks, int nk, int ntau)
 }
 
 static int pt_run(sbz_problem* pb, int nk, double load, const int* d_cosmo, const double* d_ks, const double* d_ti, const int* d_order,
-                  int ntau, const double* d_taus, int output, double* d_out, int* d_status, int64_t* d_steps) {
+                  int ntau, const double* d_taus, int output, double* d_out, int* d_status, int64_t* d_steps, int plan = 0) {
   sbz::PtArgs A{};
   pt_model_args(pb, A);
+  A.plan = plan;
   A.item_cosmo = d_cosmo; A.item_k = d_ks; A.item_tau_ini = d_ti; A.order = d_order; A.nitems = nk; A.load = load;
   A.taus = ntau > 0 ? d_taus : nullptr; A.ntau = ntau;
   A.output = output; A.out = d_out; A.status = d_status; A.steps = d_steps;
@@ -533,13 +535,15 @@ int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks,
                     const double* taus, int output, int* best, double* ms) {
   if (!check_pt_args(pb, nk, ntau, output)) return SBZ_ERR_ARG;
   if (nk <= 0 || !ks || !tau_ini) return fail(SBZ_ERR_ARG, "sbz_autotune_pt: bad arguments");
-  // stratified sample in k (every m-th mode of the k-sorted list): large batches are timed on an
-  // eighth of their modes, small ones in full, so the sample stays in the same regime (tail-bound
-  // or throughput-bound) as the workload
+  // stratified sample in k (every m-th mode of the k-sorted list): down to an eighth of the modes, while it keeps 20
+  // longest modes' work per SM, so that it is bound like the workload (by its work, not by its longest modes; an eighth of
+  // 2,400 modes of n = 133 is one round of longest modes: one mode per SM wins on it, and takes 164 ms on all of them where
+  // four take 105); a sample's launch takes the kernel that all the modes would
   std::vector<int> byk(nk);
   std::iota(byk.begin(), byk.end(), 0);
   std::stable_sort(byk.begin(), byk.end(), [&](int a, int b) { return ks[a] > ks[b]; });
-  const int m = nk > 2048 ? 8 : 1;
+  const double load = pt_load(pb, ks, nk, ntau);
+  const int m = (int)std::min(8.0, std::max(1.0, std::floor(load / (20.0 * pb->num_sms))));
   std::vector<int> sc, order;
   std::vector<double> sk, st;
   for (int i = 0; i < nk; i += m) {
@@ -568,27 +572,39 @@ int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks,
   if (ntau > 0) SBZ_CUDA(cudaMemcpyAsync(pb->d_taus.p, taus, sizeof(double) * ntau * pb->ncosmo, cudaMemcpyHostToDevice, s));
   int r;
   if ((r = ensure_events(pb)) != SBZ_OK) return r;
-  const int cand[SBZ_TUNE_CANDIDATES][2] = {{1, 0}, {2, 0}, {2, 2}, {4, 1}, {4, 2}, {4, 3}, {8, 1}};
+  // the default first (any width), then four-warp sums with open blocks: another shape has to be 2 % faster
+  const int cand[2 + SBZ_TUNE_CANDIDATES][2] = {{0, 0}, {4, 0}, {1, 0}, {2, 0}, {2, 2}, {4, 1}, {4, 2}, {4, 3}, {8, 1}};
   const int keep_nw = pb->opts.warps_per_mode, keep_bps = pb->opts.blocks_per_sm;
   double best_ms = 1e300;
   int bi = 0;
-  for (int c = 0; c < SBZ_TUNE_CANDIDATES; ++c) {
+  for (int c = 0; c < 2 + SBZ_TUNE_CANDIDATES; ++c) {
     pb->opts.warps_per_mode = cand[c][0];
     pb->opts.blocks_per_sm = cand[c][1];
+    // the shortest mode untimed: a kernel's first launch loads it
+    r = pt_run(pb, 1, load, pb->d_cosmo.as<int>() + ns - 1, pb->d_k.as<double>() + ns - 1, pb->d_ti.as<double>() + ns - 1, nullptr, ntau,
+               pb->d_taus.as<double>(), output, pb->d_out.as<double>(), pb->d_status.as<int>(), pb->d_steps.as<int64_t>(), nk);
+    if (r != SBZ_OK) { pb->opts.warps_per_mode = keep_nw; pb->opts.blocks_per_sm = keep_bps; return r; }
     SBZ_CUDA(cudaEventRecord(pb->ev[8], s));
-    r = pt_run(pb, ns, pt_load(pb, sk.data(), ns, ntau), pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
-               pb->d_taus.as<double>(), output, pb->d_out.as<double>(), pb->d_status.as<int>(), pb->d_steps.as<int64_t>());
+    r = pt_run(pb, ns, load, pb->d_cosmo.as<int>(), pb->d_k.as<double>(), pb->d_ti.as<double>(), pb->d_order.as<int>(), ntau,
+               pb->d_taus.as<double>(), output, pb->d_out.as<double>(), pb->d_status.as<int>(), pb->d_steps.as<int64_t>(), nk);
     if (r != SBZ_OK) { pb->opts.warps_per_mode = keep_nw; pb->opts.blocks_per_sm = keep_bps; return r; }
     SBZ_CUDA(cudaEventRecord(pb->ev[9], s));
     SBZ_CUDA(cudaEventSynchronize(pb->ev[9]));
     float t = 0;
     cudaEventElapsedTime(&t, pb->ev[8], pb->ev[9]);
-    if (ms) ms[c] = t;
-    if (t < best_ms) { best_ms = t; bi = c; }
+    if (c < 2) pb->open_ms[c] = t;
+    else if (ms) ms[c - 2] = t;
+    if (t < 0.98 * best_ms) { best_ms = t; bi = c; }
   }
   pb->opts.warps_per_mode = cand[bi][0];
   pb->opts.blocks_per_sm = cand[bi][1];
   if (best) { best[0] = cand[bi][0]; best[1] = cand[bi][1]; }
+  return SBZ_OK;
+}
+
+int sbz_autotune_open_ms(const sbz_problem* pb, double* ms2) {
+  if (!pb || !ms2) return fail(SBZ_ERR_ARG, "null argument");
+  ms2[0] = pb->open_ms[0]; ms2[1] = pb->open_ms[1];
   return SBZ_OK;
 }
 

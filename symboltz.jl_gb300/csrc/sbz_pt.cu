@@ -34,6 +34,7 @@ static int auto_warps_per_mode(int nitems, int num_sms) { return nitems <= 32 * 
 // for mixed n > 128 at r = 1.7 (one mode per SM chosen, two 13 to 16 % faster).  Lines on the mode count alone gave up to
 // 40 % away where the modes' lengths are close.
 struct Sharing { int modes, warps; };
+static int plan_items(const PtArgs& A) { return A.plan > 0 ? A.plan : A.nitems; }
 static Sharing modes_per_sm(const PtArgs& A, int precision, int num_sms) {
   const bool mixed = precision == SBZ_MIXED;
   static const float mixed_slow[3][4] = {{1.45f, 1.56f, 1.87f, 2.8f}, {1.46f, 1.65f, 2.07f, 3.7f}, {1.75f, 1.97f, 2.33f, 3.75f}};
@@ -42,7 +43,7 @@ static Sharing modes_per_sm(const PtArgs& A, int precision, int num_sms) {
   const float* slow = mixed ? mixed_slow[n <= 64 ? 0 : n <= 128 ? 1 : 2] : fp64_slow[n <= 64 ? 0 : 1];
   const int two = mixed ? pt_thr2_resident_f32(n) : pt_thr2_resident_f64(n);  // modes of two warps
   const Sharing shape[4] = {{2, 4}, {3, 4}, {4, 4}, {two, 2}};
-  const double r = (A.load > 0 ? A.load : 0.25 * A.nitems) / num_sms;  // modes on the device only: as of a geometric grid up to 0.2 h/Mpc
+  const double r = (A.load > 0 ? A.load : 0.25 * plan_items(A)) / num_sms;  // modes on the device only: as of a geometric grid up to 0.2 h/Mpc
   Sharing best{1, 4};
   double tb = r > 1 ? r : 1;
   for (int i = 0; i < 4; ++i) {
@@ -54,17 +55,18 @@ static Sharing modes_per_sm(const PtArgs& A, int precision, int num_sms) {
 }
 
 PtShape pt_shape(const PtArgs& A, int precision, int warps_per_mode, int blocks_per_sm, int num_sms) {
-  const int nw = warps_per_mode > 0 ? warps_per_mode : auto_warps_per_mode(A.nitems, num_sms);
+  const int items = plan_items(A);
+  const int nw = warps_per_mode > 0 ? warps_per_mode : auto_warps_per_mode(items, num_sms);
   const bool lat_fits = A.nchain <= 8 && A.chain_rows <= 32;  // four solver warps hold every chain (nx <= 5)
   Sharing sh = modes_per_sm(A, precision, num_sms);
   // one-warp norms, and many modes of models that do not fit the latency kernel, need the throughput kernel
-  if (sh.modes == 1 && (nw == 1 || (!lat_fits && A.nitems > 7 * num_sms))) sh.modes = 2;
+  if (sh.modes == 1 && (nw == 1 || (!lat_fits && items > 7 * num_sms))) sh.modes = 2;
   // throughput kernel: blocks left open, chains that fit a warp; one-warp modes only where the width was
   // left open too (asked for, they keep their own kernel)
   // (two-warp modes asked for: 5,000 of n = 133 take 134 ms in their own kernel and 105 here, of n = 188 119 and 128)
   if (blocks_per_sm <= 0 && sh.modes > 1 && A.chain_rows <= 32 && (warps_per_mode <= 0 || (nw == 2 && A.model_n <= 160) || nw == 4))
     return PtShape{PT_THROUGHPUT, nw, sh.warps, sh.modes, 0};
-  if (blocks_per_sm <= 0 && nw == 4) blocks_per_sm = A.nitems <= 8 * num_sms || (sh.modes == 1 && lat_fits) ? 1 : 2;
+  if (blocks_per_sm <= 0 && nw == 4) blocks_per_sm = items <= 8 * num_sms || (sh.modes == 1 && lat_fits) ? 1 : 2;
   if (nw == 8) blocks_per_sm = 1;  // eight-warp groups: one mode per SM
   if (nw == 4 && blocks_per_sm == 1 && lat_fits) return PtShape{PT_LATENCY, nw, nw, 1, 1};  // one mode per SM
   return PtShape{PT_GENERIC, nw, nw, 0, blocks_per_sm};

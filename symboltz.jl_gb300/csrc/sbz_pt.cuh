@@ -20,6 +20,7 @@ struct PtArgs {
   const double* item_tau_ini; // device
   const int* order;           // device, processing order (nullptr = identity)
   int nitems;
+  int plan;                   // modes that the launch shape is chosen for (0: nitems; the tuner times samples)
   const double* taus;         // device, [c * ntau + j] (nullptr when ntau == 0)
   int ntau;
   int output;
@@ -30,7 +31,7 @@ struct PtArgs {
   int64_t maxiters;
   int refine;
   float refine_skip;          // skip stages 2-6 refinement below this stage-1 correction (0: never; < 0: by launch shape)
-  double load;                // Σ over the modes of their expected steps / those of the longest (0: not known)
+  double load;                // Σ over the modes of their expected steps / those of the longest (0: not known), of the modes in plan
   int norm_warps;             // throughput kernel: warps per mode whose summation order the norms follow (4, 2 or 1)
   unsigned int* counter;      // device work-queue counter, zero before launch
 };

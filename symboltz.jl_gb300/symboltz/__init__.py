@@ -223,8 +223,8 @@ _OUT = {"sources": L.SBZ_OUT_SOURCES, "delta_m": L.SBZ_OUT_DELTA_M, "state": L.S
 
 def autotune(prob: CosmologyProblem, ks, ptivini=-np.inf, *, saveat=None, output="sources", cosmo=None):
     """Pick the perturbation kernel's launch shape (warps per mode, blocks per SM) for this workload
-    by timing the candidates on a k-stratified sample of it (``sbz_autotune_pt``); the choice is
-    stored in the problem and used by later solves.  Returns {"warps_per_mode", "blocks_per_sm",
+    by timing the candidates on a k-stratified sample of it (``sbz_autotune_pt``; (0, 0) is the library's own
+    choice); the choice is stored in the problem and used by later solves.  Returns {"warps_per_mode", "blocks_per_sm",
     "candidates_ms": {(nw, bps): ms}}."""
     prob.solvebg()
     ks = L.f64(np.atleast_1d(ks))
@@ -243,9 +243,11 @@ def autotune(prob: CosmologyProblem, ks, ptivini=-np.inf, *, saveat=None, output
     ms = L.f64(np.zeros(7))
     L.check(L.lib().sbz_autotune_pt(prob._h, nk, L.iptr(cos), L.dptr(ks), L.dptr(ti), taus.shape[1], L.dptr(taus), kind,
                                     L.iptr(best), L.dptr(ms)), "autotune")
-    cands = [(1, 0), (2, 0), (2, 2), (4, 1), (4, 2), (4, 3), (8, 1)]
+    open_ms = L.f64(np.zeros(2))
+    L.check(L.lib().sbz_autotune_open_ms(prob._h, L.dptr(open_ms)), "autotune")
+    cands = [(1, 0), (2, 0), (2, 2), (4, 1), (4, 2), (4, 3), (8, 1), (0, 0), (4, 0)]
     prob.opts.warps_per_mode, prob.opts.blocks_per_sm = int(best[0]), int(best[1])
-    return {"warps_per_mode": int(best[0]), "blocks_per_sm": int(best[1]), "candidates_ms": {c: float(m) for c, m in zip(cands, ms)}}
+    return {"warps_per_mode": int(best[0]), "blocks_per_sm": int(best[1]), "candidates_ms": {c: float(m) for c, m in zip(cands, [*ms, *open_ms])}}
 
 
 def solvept(prob: CosmologyProblem, ks, ptivini=-np.inf, *, saveat=None, output="state", cosmo=None):

@@ -20,7 +20,7 @@ EXPORTS = (
     "sbz_default_opts", "sbz_last_error", "sbz_momentum_quadrature", "sbz_problem_create", "sbz_problem_destroy", "sbz_problem_set_params",
     "sbz_problem_nstate", "sbz_solve_bg", "sbz_bg_knots", "sbz_bg_eval", "sbz_bg_coefficients", "sbz_solve_pt", "sbz_solve_pt_device", "sbz_pt_rhs",
     "sbz_spectrum_matter", "sbz_spectrum_primordial", "sbz_bessel_create", "sbz_bessel_destroy", "sbz_bessel_eval",
-    "sbz_los_integrate", "sbz_los_integrate_device", "sbz_cl_integrate", "sbz_cl_integrate_noalloc", "sbz_autotune_pt", "sbz_pt_launch_shape", "sbz_mlp_gemm", "sbz_surrogate_create", "sbz_surrogate_destroy", "sbz_surrogate_nparams",
+    "sbz_los_integrate", "sbz_los_integrate_device", "sbz_cl_integrate", "sbz_cl_integrate_noalloc", "sbz_autotune_pt", "sbz_autotune_open_ms", "sbz_pt_launch_shape", "sbz_mlp_gemm", "sbz_surrogate_create", "sbz_surrogate_destroy", "sbz_surrogate_nparams",
     "sbz_surrogate_get_params", "sbz_surrogate_set_params", "sbz_surrogate_set_data", "sbz_surrogate_train",
     "sbz_surrogate_gradients", "sbz_surrogate_infer", "sbz_surrogate_save", "sbz_surrogate_load", "sbz_trainset_append", "sbz_trainset_info", "sbz_trainset_read", "sbz_spectrum_cmb", "sbz_spectrum_cmb_sources", "sbz_problem_set_stream",
     "sbz_problem_timings",
@@ -75,6 +75,7 @@ def lib():
     L.sbz_bg_eval.argtypes = [vp, C.c_int, C.c_int, dp, dp]
     L.sbz_bg_coefficients.argtypes = [vp, C.c_int, C.c_int, dp, dp]
     L.sbz_solve_pt.argtypes = [vp, C.c_int, ip, dp, dp, C.c_int, dp, C.c_int, dp, ip, i64p]
+    L.sbz_autotune_open_ms.argtypes = [vp, dp]
     L.sbz_pt_launch_shape.argtypes = [vp, C.c_int, dp, C.c_int, C.c_int, ip]
     L.sbz_autotune_pt.argtypes = [vp, C.c_int, ip, dp, dp, C.c_int, dp, C.c_int, ip, dp]
     fp = C.POINTER(C.c_float)
