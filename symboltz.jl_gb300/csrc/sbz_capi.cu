@@ -67,28 +67,32 @@ cudaError_t up(DevBuf& b, const T* h, size_t n, cudaStream_t st) {
 
 // Weights w with ∫ S = Σ_i w_i y_i for the natural cubic spline S through (X_i, y_i): the integral
 // aᵀy - cᵀz of the spline (z = second derivatives, T z = R y) is (a - Rᵀ T⁻¹ c)ᵀ y, so one
-// tridiagonal solve with the symmetric T gives the weights for every integrand on this grid.
+// tridiagonal solve with the symmetric T gives the weights for every integrand on this grid.  The same integral by intervals: ∫ S = Σ_i h_i/2 (y_i + y_{i+1}) - e_i (y_{i+1} - y_i), e_i = 6 (v_i - v_{i+1}) / h_i
+// with T v = c (v = 0 at the ends).
+std::vector<double> spline_integral_solve(const std::vector<double>& X) {
+  const int n = (int)X.size(), m = n - 2;  // interior second derivatives z_1..z_{n-2}
+  std::vector<double> v(n, 0.0), cp(n, 0.0);
+  for (int i = 1; i <= m; ++i) {  // Thomas on T v = c, T_ii = 2(h_{i-1}+h_i), T_i,i+1 = h_i
+    const double h0 = X[i] - X[i - 1], h1 = X[i + 1] - X[i];
+    const double c = (h0 * h0 * h0 + h1 * h1 * h1) / 24.0;
+    const double den = 2.0 * (h0 + h1) - (i > 1 ? h0 * cp[i - 1] : 0.0);
+    cp[i] = h1 / den;
+    v[i] = (c - (i > 1 ? h0 * v[i - 1] : 0.0)) / den;
+  }
+  for (int i = m - 1; i >= 1; --i) v[i] -= cp[i] * v[i + 1];
+  return v;
+}
+
 void spline_integral_weights(const std::vector<double>& X, std::vector<double>& w) {
   const int n = (int)X.size();
   w.assign(n, 0.0);
   std::vector<double> h(n - 1);
   for (int i = 0; i + 1 < n; ++i) { h[i] = X[i + 1] - X[i]; w[i] += 0.5 * h[i]; w[i + 1] += 0.5 * h[i]; }
-  const int m = n - 2;  // interior second derivatives z_1..z_{n-2}
-  if (m < 1) return;
-  std::vector<double> cp(m), v(m);
-  for (int j = 0; j < m; ++j) {  // Thomas on T v = c, T_jj = 2(h_{i-1}+h_i), T_j,j+1 = h_i (i = j+1)
-    const int i = j + 1;
-    const double c = (h[i - 1] * h[i - 1] * h[i - 1] + h[i] * h[i] * h[i]) / 24.0;
-    const double den = 2.0 * (h[i - 1] + h[i]) - (j > 0 ? h[i - 1] * cp[j - 1] : 0.0);
-    cp[j] = h[i] / den;
-    v[j] = (c - (j > 0 ? h[i - 1] * v[j - 1] : 0.0)) / den;
-  }
-  for (int j = m - 2; j >= 0; --j) v[j] -= cp[j] * v[j + 1];
-  for (int j = 0; j < m; ++j) {  // w -= Rᵀ v,  R y = 6 ((y_{i+1}-y_i)/h_i - (y_i-y_{i-1})/h_{i-1})
-    const int i = j + 1;
-    w[i - 1] -= 6.0 / h[i - 1] * v[j];
-    w[i] += 6.0 * (1.0 / h[i - 1] + 1.0 / h[i]) * v[j];
-    w[i + 1] -= 6.0 / h[i] * v[j];
+  const std::vector<double> v = spline_integral_solve(X);
+  for (int i = 1; i <= n - 2; ++i) {  // w -= Rᵀ v,  R y = 6 ((y_{i+1}-y_i)/h_i - (y_i-y_{i-1})/h_{i-1})
+    w[i - 1] -= 6.0 / h[i - 1] * v[i];
+    w[i] += 6.0 * (1.0 / h[i - 1] + 1.0 / h[i]) * v[i];
+    w[i + 1] -= 6.0 / h[i] * v[i];
   }
 }
 
@@ -953,23 +957,28 @@ int sbz_los_integrate_device(const sbz_bessel* c, int nsrc, const double* S, int
 
 int sbz_cl_integrate(int nk, const double* ks, const double* P0, int nl, const double* ThA, const double* ThB, double* Cl) {
   if (nk < 2 || nl < 1 || !ks || !P0 || !ThA || !ThB || !Cl) return fail(SBZ_ERR_ARG, "sbz_cl_integrate: bad arguments");
-  std::vector<double> X(nk + 1), wk, g(nk);
+  std::vector<double> X(nk + 1), head(3 * (size_t)nk);  // head: (a, e) per interval, then g per point (cl_pair_launch)
   X[0] = 0;
   for (int i = 0; i < nk; ++i) X[i + 1] = ks[i];
   for (int i = 1; i <= nk; ++i) if (!(X[i] > X[i - 1])) return fail(SBZ_ERR_ARG, "ks must be positive and increasing");
-  // the natural-spline integral of 2/π k² P0 Θ_A Θ_B as a weighted sum over k
-  spline_integral_weights(X, wk);
-  for (int i = 0; i < nk; ++i) g[i] = wk[i + 1] * (2.0 / M_PI) * ks[i] * ks[i] * P0[i];
+  // the natural-spline integral of 2/π k² P0 Θ_A Θ_B
+  const std::vector<double> v = spline_integral_solve(X);
+  for (int i = 0; i < nk; ++i) {
+    const double h = X[i + 1] - X[i];
+    head[2 * (size_t)i] = 0.5 * h; head[2 * (size_t)i + 1] = 6.0 * (v[i] - v[i + 1]) / h;
+    head[2 * (size_t)nk + i] = (2.0 / M_PI) * ks[i] * ks[i] * P0[i];
+  }
   struct Owned : DevBuf {  // released on every return path
     ~Owned() { release(); }
   } buf;
   const size_t th = (size_t)nk * nl;
-  SBZ_CUDA(buf.ensure(sizeof(double) * (nk + 2 * th + nl)));
-  double *d_g = buf.as<double>(), *d_A = d_g + nk, *d_B = d_A + th, *d_Cl = d_B + th;
-  SBZ_CUDA(cudaMemcpy(d_g, g.data(), sizeof(double) * nk, cudaMemcpyHostToDevice));
+  SBZ_CUDA(buf.ensure(sizeof(double) * (3 * (size_t)nk + 2 * th + nl)));
+  double2* d_ae = buf.as<double2>();
+  double *d_g = reinterpret_cast<double*>(d_ae + nk), *d_A = d_g + nk, *d_B = d_A + th, *d_Cl = d_B + th;
+  SBZ_CUDA(cudaMemcpy(d_ae, head.data(), sizeof(double) * head.size(), cudaMemcpyHostToDevice));
   SBZ_CUDA(cudaMemcpy(d_A, ThA, sizeof(double) * th, cudaMemcpyHostToDevice));
   SBZ_CUDA(cudaMemcpy(d_B, ThB, sizeof(double) * th, cudaMemcpyHostToDevice));
-  const int r = sbz::cl_pair_launch(nk, d_g, nl, d_A, d_B, d_Cl, 0);
+  const int r = sbz::cl_pair_launch(nk, d_g, d_ae, nl, d_A, d_B, d_Cl, 0);
   if (r == 0) SBZ_CUDA(cudaMemcpy(Cl, d_Cl, sizeof(double) * nl, cudaMemcpyDeviceToHost));
   return r == 0 ? SBZ_OK : fail(SBZ_ERR_CUDA, "C_l kernel");
 }

@@ -281,20 +281,33 @@ __global__ void __launch_bounds__(256) los_f32_kernel(const float2* __restrict__
   }
 }
 
-// C_l = Σ_k g_k A(k, l) B(k, l): 32 l by 8 k-lanes per block, one coalesced row piece of A and B per k.
-__global__ void __launch_bounds__(256) cl_pair_kernel(int nk, const double* __restrict__ g, int nl, const double* __restrict__ A,
-                                                      const double* __restrict__ B, double* __restrict__ Cl) {
-  __shared__ double red[8][33];
-  const int lx = threadIdx.x & 31, ky = threadIdx.x >> 5, il = blockIdx.x * 32 + lx;
+// C_l = Σ_i a_i (Y_i + Y_{i+1}) - e_i (Y_{i+1} - Y_i) over the intervals between the points (0, 0) and
+// (k, Y = g A B), ae: (a_i, e_i): trapezoid and the spline's correction on the differences (one weight per point,
+// trapezoid and corrections of both sides added up, would cancel between close points: 1e-8 of C_l where two are 1e-9
+// apart).  8 l by 32 runs of intervals per block: an FP64 instruction costs the same for any number of lanes, so a warp
+// takes four runs.
+__global__ void __launch_bounds__(256) cl_pair_kernel(int nk, const double* __restrict__ g, const double2* __restrict__ ae, int nl,
+                                                      const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ Cl) {
+  __shared__ double red[32][9];
+  const int lx = threadIdx.x & 7, run = threadIdx.x >> 3, il = blockIdx.x * 8 + lx;
+  const int i0 = (int)((long long)nk * run / 32), i1 = (int)((long long)nk * (run + 1) / 32);
+  auto Y = [&](int i) { return g[i] * A[(size_t)i * nl + il] * B[(size_t)i * nl + il]; };
   double sum = 0;
-  if (il < nl)
+  if (il < nl) {
+    double y0 = i0 > 0 && i0 < i1 ? Y(i0 - 1) : 0.0;
 #pragma unroll 4
-    for (int i = ky; i < nk; i += 8) sum = fma(g[i] * A[(size_t)i * nl + il], B[(size_t)i * nl + il], sum);
-  red[ky][lx] = sum;
+    for (int i = i0; i < i1; ++i) {
+      const double y1 = Y(i);
+      const double2 w = ae[i];
+      sum = fma(w.x, y0 + y1, fma(-w.y, y1 - y0, sum));
+      y0 = y1;
+    }
+  }
+  red[run][lx] = sum;
   __syncthreads();
-  if (ky == 0 && il < nl) {
+  if (run == 0 && il < nl) {
     double t = 0;
-    for (int q = 0; q < 8; ++q) t += red[q][lx];
+    for (int q = 0; q < 32; ++q) t += red[q][lx];
     Cl[il] = t;
   }
 }
@@ -620,8 +633,8 @@ int los_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S,
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int cl_pair_launch(int nk, const double* d_g, int nl, const double* d_A, const double* d_B, double* d_Cl, cudaStream_t st) {
-  cl_pair_kernel<<<(nl + 31) / 32, 256, 0, st>>>(nk, d_g, nl, d_A, d_B, d_Cl);
+int cl_pair_launch(int nk, const double* d_g, const double2* d_ae, int nl, const double* d_A, const double* d_B, double* d_Cl, cudaStream_t st) {
+  cl_pair_kernel<<<(nl + 7) / 8, 256, 0, st>>>(nk, d_g, d_ae, nl, d_A, d_B, d_Cl);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

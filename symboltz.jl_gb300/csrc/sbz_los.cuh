@@ -26,8 +26,8 @@ int bessel_eval(const BesselDev& J, int il, int n, const double* d_x, double* d_
 int los_launch(const BesselDev& J, const int* d_ls, int nsrc, const double* d_S, long long st_t, long long st_k, const double* d_taus,
                const double* d_chi, const double* d_w, int ntau, int nk, const double* d_ks, int il_limber,
                double* d_out, cudaStream_t st);
-// C_l = Σ_k g_k A(k,l) B(k,l) for two [nk][nl] arrays
-int cl_pair_launch(int nk, const double* d_g, int nl, const double* d_A, const double* d_B, double* d_Cl, cudaStream_t st);
+// C_l = Σ_i ae_i.x (Y_i + Y_{i+1}) - ae_i.y (Y_{i+1} - Y_i), Y_0 = 0, Y_{i+1} = g_i A(k_i,l) B(k_i,l) for two [nk][nl] arrays
+int cl_pair_launch(int nk, const double* d_g, const double2* d_ae, int nl, const double* d_A, const double* d_B, double* d_Cl, cudaStream_t st);
 int cl_launch(int nk, const double* d_ks, const double* d_P0, int nl, const double* d_ThA, const double* d_ThB,
               const double* d_cprime, const double* d_invden, double* d_zbuf, double* d_Cl, cudaStream_t st);
 
