@@ -446,6 +446,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
   tc_fence_after();
   const int quarter = warp & 3, half = warp >> 2;
   const int row = m0 + quarter * 32 + lane;
+  // 16-byte accesses along the rows of whatever the epilogue touches
+  const uintptr_t bases = g.epi == EPI_F32 ? (uintptr_t)g.out_f32 : (uintptr_t)g.out_bf16 | (uintptr_t)(g.epi == EPI_ACT ? g.z_out : g.z_in);
+  const bool vec_rows = g.ldo % 8 == 0 && (bases & 15) == 0;
   if (ok && g.part) {
     // split K: 32 x 32 tiles staged in the operand ring (12 KB per warp, three buffers; rows of 128 bytes,
     // 128-byte swizzle) and stored by TMA, each split in its own rows; whoever reads them adds them in the splits'
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_tn_kernel(const __grid_const
       const bool live = row < g.M;
       const size_t o = (size_t)row * g.ldo + col;
       const int nv = min(32, g.n_valid - col);
-      const bool vec = nv == 32 && (g.ldo % 8) == 0;
+      const bool vec = nv == 32 && vec_rows;
       if (g.epi == EPI_F32) {
         if (!live) continue;
         float* out = g.out_f32 + o;
