@@ -539,7 +539,7 @@ int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks,
                     const double* taus, int output, int* best, double* ms) {
   if (!check_pt_args(pb, nk, ntau, output)) return SBZ_ERR_ARG;
   if (nk <= 0 || !ks || !tau_ini) return fail(SBZ_ERR_ARG, "sbz_autotune_pt: bad arguments");
-  // stratified sample in k (every m-th mode of the k-sorted list): down to an eighth of the modes, while it keeps 20
+  // stratified sample in k (every m-th mode of the k-sorted list): down to an eighth of the modes, while it keeps 10
   // longest modes' work per SM, so that it is bound like the workload (by its work, not by its longest modes; an eighth of
   // 2,400 modes of n = 133 is one round of longest modes: one mode per SM wins on it, and takes 164 ms on all of them where
   // four take 105); a sample's launch takes the kernel that all the modes would
@@ -547,7 +547,7 @@ int sbz_autotune_pt(sbz_problem* pb, int nk, const int* cosmo, const double* ks,
   std::iota(byk.begin(), byk.end(), 0);
   std::stable_sort(byk.begin(), byk.end(), [&](int a, int b) { return ks[a] > ks[b]; });
   const double load = pt_load(pb, ks, nk, ntau);
-  const int m = (int)std::min(8.0, std::max(1.0, std::floor(load / (20.0 * pb->num_sms))));
+  const int m = (int)std::min(8.0, std::max(1.0, std::floor(load / (10.0 * pb->num_sms))));
   std::vector<int> sc, order;
   std::vector<double> sk, st;
   for (int i = 0; i < nk; i += m) {
