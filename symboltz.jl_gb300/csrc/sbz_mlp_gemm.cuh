@@ -176,9 +176,10 @@ __device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&v)[32]) {
 
 // Activation layers (EPI_ACT, EPI_DACT) of whole 128 x BN tiles: one CTA per SM takes every gridDim-th tile, and
 // the accumulator is double-buffered in TMEM, so the epilogue of a tile (about 25 µs per 65,536 x 512 layer, bound
-// by instruction issue) runs beside the loads and the product of the next one (402 MB from
-// L2, the bound at 512 inputs: 45 µs with three ring slots of 48 KB, 55 with two).  Warp 0 loads, warp 1 issues the products, 16 epilogue warps take
-// 32 rows x 64 columns each (BN = 128: eight of them per tile, in turn).  A warp stages its tiles in 8 KB of
+// by instruction issue) runs beside the loads and the product of the next one: 45 µs at 512 inputs with three ring slots
+// of 48 KB, 55 with two.  HBM takes 30 of them at the copy rate (67 MB read, 134 written); the 402 MB from L2 are not the
+// bound (a third less of them, weight tiles shared by two CTAs, took as long).  Warp 0 loads, warp 1 issues the products,
+// 16 epilogue warps take 32 rows x 64 columns each (BN = 128: eight of them per tile, in turn).  A warp stages its tiles in 4 KB of
 // shared memory and one lane stores them with TMA: every global sector is written whole, where 16-byte stores
 // from 32 rows at a stride of 1 KB wrote halves.  128-byte rows, 128-byte swizzle (16-byte piece p of row r at
 // p ^ (r mod 8): conflict-free by rows and by columns).  EPI_DACT loads its pre-activations by TMA one tile ahead

@@ -15,7 +15,8 @@ int pt_thr2_resident_f32(int n);
 int pt_thr2_resident_f64(int n);
 
 // Warps per mode when the caller leaves it open.  The results of a mode depend on it (order of the norms'
-// sums, refinement default), not on the kernel that runs it.
+// sums, refinement default).  In mixed precision they do not depend on the kernel that runs it; in all-FP64 the
+// latency and throughput kernels form reciprocals of pivots (lat_rcp) where the generic kernel divides.
 static int auto_warps_per_mode(int nitems, int num_sms) { return nitems <= 32 * num_sms ? 4 : 1; }
 
 // Modes that share an SM when the caller leaves it open, 1: the latency kernel; warps that run each.  With few modes per

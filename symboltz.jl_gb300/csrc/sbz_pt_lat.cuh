@@ -67,7 +67,7 @@ struct LatMem {
   ST dd[NM], sup[NM], sub[NM], dinv[NM], mfw[NM], bP[NM];
   ST Z1[NM + 1], Z2[NM + 1];
   ST H[64], Hinv[64];
-  ST hs[2], hmul[2], hcorr[2];   // couplings of the photon tails to the head
+  ST hmul[2], hcorr[2];   // couplings of the photon tails to the head
   ST wS[kWF], fS[4];
   CSet cs[kNSets];
   double B[kMaxT][B_COUNT], dB[kMaxT][B_COUNT];  // base scalars of the companions' times

@@ -861,8 +861,9 @@ __host__ inline size_t thr_block_bytes(int n, int modes) { return ((sizeof(Model
 template <typename ST>
 __host__ inline int thr2_resident(int n) { return 2 * (thr_block_bytes<ST>(n, 4) + 1024) <= 228 * 1024 ? 8 : 4; }
 
-// NT threads per block (NT / (32 G) modes), MINB blocks per SM: 128 x 3 keeps 168 registers per thread (no
-// spills), 256 x 2 runs 16 warps per SM on 128.
+// NT threads per block (NT / (32 G) modes), MINB blocks per SM: 128 x 3 keeps 168 registers per thread (no spills but
+// 16 bytes in FP64), 256 x 2 runs 16 warps per SM on 128 (spills of 124 to 140 bytes with one row per lane, 378 (FP64
+// 724) with two, 1,052 with three: two-warp modes above 128 equations).
 template <int G, int NT, int MINB, int NSL, typename ST>
 __global__ void __launch_bounds__(NT, MINB) pt_thr_kernel(PtArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
