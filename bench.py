@@ -49,8 +49,8 @@ REFINE_SKIP_CL = 1e-2
 # within 1.3e-5 for atol 3e-8 (oracle, Rodas5P, against rtol = atol = 1e-9).
 PT_RTOL, PT_ATOL = 1e-6, 3e-8
 # DRAM bytes (read + write) of the spectrum's perturbation launch: one ncu pass of
-# dram__bytes_read.sum + dram__bytes_write.sum on `bench.py --profile-case los` (4.15 MB + 2.53 MB)
-PT_LAUNCH_DRAM_BYTES = 6.68e6
+# dram__bytes_read.sum + dram__bytes_write.sum on `bench.py --profile-case los` (4.01 MB + 1.60 MB)
+PT_LAUNCH_DRAM_BYTES = 5.61e6
 
 
 def workload_grids(S, prob):
@@ -248,11 +248,11 @@ def run_ours(args):
         "phases_ms": {k: round(float(np.mean([p[k] for p in phases])), 3) for k in phases[0]},
         "roofline": {"bound": "fp64", "achieved": round(achieved, 5), "peak": round(fp64_peak, 3), "unit": "TFLOP/s",
                      "frac": round(achieved / fp64_peak, 5),
-                     # dram__bytes_read.sum + dram__bytes_write.sum of one full pt_kernel launch of this
-                     # workload (ncu, profiles/launches_bench_lcdm_massive_nu.md): 1.98 MB + 2.66 MB; the
-                     # coefficient tables stay in L1/L2, the kernel is FP64-latency bound
+                     # dram__bytes_read.sum + dram__bytes_write.sum of one full launch of this workload
+                     # (ncu, profiles/launches_bench_lcdm_massive_nu.md); the coefficient tables stay in
+                     # L1/L2, the kernel is FP64-latency bound
                      "traffic": PT_LAUNCH_DRAM_BYTES,
-                     "kernel": "pt_kernel (perturbation modes)", "flops_per_step": fl, "steps_per_launch": steps_total,
+                     "kernel": "pt_lat_kernel (perturbation modes, one per SM)", "flops_per_step": fl, "steps_per_launch": steps_total,
                      "peak_source": "cuBLAS DGEMM 4096^3 measured in this run (no FP64 entry in MEASURED_PEAKS.json)",
                      # the same launch against the HBM roofline: measured traffic over its CUDA-event time
                      "hbm": {"achieved_gbs": round(PT_LAUNCH_DRAM_BYTES / pt_avg / 1e9, 6), "peak_gbs": peaks.get("hbm_gbs"),
@@ -386,7 +386,8 @@ def mlp_step_bytes(batch=65536, nin_pad=64, width=512, nhidden=4, nout_pad=64, n
     per kernel that touches it): forward layers read X_{l-1} and write X_l and Z_l (BF16), the
     output layer writes FP32 Y; the loss reads Y and writes dY; each backward dX GEMM reads its
     output gradient and Z and writes dZ; each weight-gradient GEMM reads dZ and X; Adam reads
-    and writes p, m, v and reads the gradient (FP32) and writes two BF16 copies of the weights."""
+    and writes p, m, v and reads the gradient (FP32) and writes two BF16 copies of the weights.  The
+    partial sums of the gradients (151 MB, written and read) are not counted."""
     a, w = 2 * batch, width
     fwd = a * nin_pad + 2 * a * w + (nhidden - 1) * (a * w + 2 * a * w) + a * w + 4 * batch * nout_pad
     loss = 4 * batch * nout_pad + a * nout_pad
