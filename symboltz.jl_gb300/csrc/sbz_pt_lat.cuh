@@ -244,7 +244,8 @@ __device__ __forceinline__ Fun lat_matvec(const LGrp& g, LatMem<NSL, ST>& W, con
 
 // Reciprocal of a pivot.  FP32: the hardware approximation (pivots are far from the subnormals that the
 // non-ftz form would handle).  FP64: its 20-bit seed and two Newton steps r += r (1 - v r), each squaring
-// the error: about one unit in the last place for a fifth of a division's FP64 instructions.
+// the error: a unit in the last place at most (the division's bits in 2e9 random values) for a fifth of a division's
+// FP64 instructions.
 template <typename ST>
 __device__ __forceinline__ ST lat_rcp(ST v);
 template <>
